@@ -100,7 +100,12 @@ struct tl_ctx {
   cudaGraphExec_t cg_prof_exec = nullptr;
   LoopArgs cg_prof_key{};
   long long cg_prof_nk = 0;
-  int pgrid = -1;  // co-resident CTAs of the persistent CG kernel (-1: not yet queried)
+  // persistent CG kernel: -1 not yet planned, 0 the mesh does not fit, 1 pplan holds; the boxes
+  // its CTAs exchange partial sums and rims in, and the number of the next sum
+  int pstate = -1;
+  PersistPlan pplan{};
+  void* pbox = nullptr;
+  unsigned pepoch = 0;
   // host transfers: an upload and a download stream (tl_stage_state, tl_fetch_field) and
   // XFER_FIELDS staging fields -- two staged (density, energy1) pairs, the fetch snapshot, and
   // two for the synchronous uploads / downloads.  A host array moves as one contiguous copy
@@ -331,12 +336,9 @@ bool writes_setup_input(int field) {
          field == TL_FIELD_MI;
 }
 
-// The persistent CG kernel replaces the batched kernels up to this many cells (plain or
-// jac_diag preconditioner): per iteration it measured 13.8 / 16.9 / 27.6 / 49.5 us at 128^2 /
-// 256^2 / 512^2 / 1024^2 against 25.6 / 26.2 / 32.3 / 47.6 us for the batched kernels (CUDA
-// graphs), so it stops paying near 800^2.  TL_CG_PERSISTENT=0 / 1 forces it off / on.
-constexpr long long PERSIST_MAX_CELLS = 640LL * 1024;
-constexpr int PERSIST_RUN = 256;  // iterations per launch at most (the host reads the status between)
+// The persistent CG kernel takes every plain or jac_diag CG whose mesh fits on chip (about a
+// million cells).  TL_CG_PERSISTENT=0 forces it off.
+constexpr int PERSIST_RUN = 1024;  // iterations per launch at most (the host reads the status between)
 
 // TL_CHEBY_SWEEP=0: the FP64 Chebyshev iterations as the two one-step kernels instead of one
 // staged sweep (same bits)
@@ -355,11 +357,30 @@ bool use_ppcg_inner_sweep() {
 bool use_persistent(tl_ctx* c) {
   if (c->prof || c->g.precond == TL_PREC_JAC_BLOCK) return false;
   const char* e = getenv("TL_CG_PERSISTENT");
-  const bool forced_on = e && e[0] == '1', forced_off = e && e[0] == '0';
-  if (forced_off) return false;
-  if (!forced_on && (long long)c->L.nx * c->L.ny > PERSIST_MAX_CELLS) return false;
-  if (c->pgrid < 0) c->pgrid = persistent_cg_grid();
-  return c->pgrid > 0;
+  if (e && e[0] == '0') return false;
+  if (c->pstate < 0) {
+    c->pstate = 0;
+    if (persist_prepare(c->L.nx, c->L.ny, c->g.precond, &c->pplan) &&
+        cudaMalloc(&c->pbox, persist_box_bytes(c->pplan)) == cudaSuccess) {
+      c->pstate = 1;
+      c->pepoch = 0;
+    }
+    cudaGetLastError();
+  }
+  return c->pstate == 1;
+}
+
+int run_persistent(tl_ctx* c, const LoopArgs& la) {
+  if (c->pepoch == 0 || c->pepoch > 0xf0000000u) {  // the numbers start (again): no box holds one
+    CK(cudaMemsetAsync(c->pbox, 0, persist_box_bytes(c->pplan), c->stream));
+    c->pepoch = 1;
+  }
+  // TL_CG_BARRIER_EXTRA=1: the grid sums wait for one partial that never comes, so every wait runs
+  // out (about a second) and the solve reports TL_ERR_TIMEOUT -- the test of the bounded wait
+  const char* ex = getenv("TL_CG_BARRIER_EXTRA");
+  CK(launch_persistent_cg(la, c->pplan, PERSIST_RUN, c->pepoch, c->pbox, c->stream, ex && ex[0] == '1' ? 1 : 0));
+  c->pepoch += 2 * PERSIST_RUN;
+  return TL_OK;
 }
 
 int run_cg_batch(tl_ctx* c, const LoopArgs& la) {
@@ -652,6 +673,7 @@ int tl_destroy(tl_ctx* c) {
   if (c->fe_done) cudaEventDestroy(c->fe_done);
   if (c->up) cudaStreamDestroy(c->up);
   if (c->down) cudaStreamDestroy(c->down);
+  cudaFree(c->pbox);
   if (c->cg_exec) cudaGraphExecDestroy(c->cg_exec);
   if (c->cg_prof_exec) cudaGraphExecDestroy(c->cg_prof_exec);
   if (c->mix_exec) cudaGraphExecDestroy(c->mix_exec);
@@ -696,7 +718,7 @@ int tl_device_bytes(const tl_ctx* c, unsigned long long* bytes) {
   if (!c || !bytes) return fail(TL_ERR_ARG, "tl_device_bytes: null argument");
   *bytes = c->slab_bytes + sizeof(double) * 4 * MAX_REDUCE_BLOCKS + 256 + sizeof(LoopState) +
            sizeof(double) * 2 * ((size_t)c->hist_cap + c->ch_cap) + c->mix_bytes + (c->tape ? c->tape_bytes : 0) +
-           (c->xfer ? (size_t)tl_ctx::XFER_FIELDS * c->field_stride : 0);
+           (c->xfer ? (size_t)tl_ctx::XFER_FIELDS * c->field_stride : 0) + (c->pbox ? persist_box_bytes(c->pplan) : 0);
   return TL_OK;
 }
 
@@ -1765,14 +1787,8 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
       const int n_before = n;
       bool sampled = false;  // the timed graph form: only iteration TIMED_ITER of the batch is timed
       if (use_persistent(c)) {
-        launch_flush_u(la, c->stream);  // a pending update of the batched kernels (none normally)
-        unsigned* bar = c->counter + 4;  // barrier counter, generation, error word
-        CK(cudaMemsetAsync(bar, 0, 3 * sizeof(unsigned), c->stream));
-        // TL_CG_BARRIER_EXTRA=1: the barriers wait for one arrival that never comes, so every
-        // wait runs out (about a second) and the solve reports TL_ERR_TIMEOUT -- the test of the
-        // bounded wait
-        const char* ex = getenv("TL_CG_BARRIER_EXTRA");
-        CK(launch_persistent_cg(la, PERSIST_RUN, bar, c->pgrid, c->stream, ex && ex[0] == '1' ? 1 : 0));
+        if (H.u_pending) launch_flush_u(la, c->stream);  // of the batched kernels (none normally)
+        if ((rc = run_persistent(c, la))) return rc;
       } else if (!c->prof && use_graphs()) {
         if ((rc = run_cg_batch(c, la))) return rc;
       } else if (use_graphs()) {

@@ -104,6 +104,36 @@ struct LoopState {
   double u_alpha;
 };
 
+// End of an iteration of the device-resident loops: error = sqrt|err_raw|, the EXIT test, n = n + 1
+// and, while a switch to Chebyshev / PPCG is possible, its rule.
+__device__ __forceinline__ void loop_finish_iteration(LoopState* st, double err_raw) {
+  const double err = sqrt(fabs(err_raw));
+  st->error = err;
+  if (!isfinite(err)) {
+    st->status = EXIT_BREAKDOWN;
+    st->n_exit = st->n;
+    return;
+  }
+  if (fabs(err) < st->eps * st->initial_residual) {
+    st->status = EXIT_CONVERGED;
+    st->n_exit = st->n;
+    return;
+  }
+  st->old_error = err;
+  st->n += 1;
+  if (st->n > st->max_iters) {
+    st->status = EXIT_MAX_ITERS;
+    st->n_exit = st->n;
+    return;
+  }
+  if (st->check_switch) {
+    // tea_solve.f90:160-174 evaluated for the next iteration (cheby_calc_steps == 0 here)
+    const bool sw = (!st->first && st->use_ppcg && st->n > 1) ||
+                    (fabs(st->old_error) <= st->epslim && st->n >= st->presteps);
+    if (sw) st->status = STOP_SWITCH;
+  }
+}
+
 // Word of the context's counter buffer that a blocked FP32 sweep of the precision form sets
 // when a bounded wait for a staged row expired (1) or its shared memory was misaligned (2):
 // MixFields::err points here, and the PPCG loop's epilogue turns it into EXIT_TIMEOUT.

@@ -12,8 +12,7 @@
 // FP64 PPCG outer iteration (tea_solve.f90:289-331): k_fused_cg_w<PPCG> (p = z + beta p,
 // w = A p, p.w, r_store = r, z.r, alpha), k_fused_cg_ur in a PPCG mode (u, r updates, init_sd),
 // the inner sweeps, then k_fused_ppcg_rrn (z = utemp, (r - r_store).z, beta, the EXIT test).
-// Also here: the persistent cooperative CG kernel for small meshes and the device-resident
-// Jacobi sweep.
+// Also here: the device-resident Jacobi sweep.
 //
 // The matvec kernel marches up a strip of 2*FT columns, one row per step: each thread owns
 // two adjacent columns (16-byte loads), keeps p of rows k-1, k, k+1 in registers and swaps
@@ -30,34 +29,6 @@ namespace {
 
 constexpr int FT = 128;      // threads per CTA
 constexpr int SW = 2 * FT;   // strip width (columns)
-
-__device__ __forceinline__ void finish_iteration(LoopState* st, double err_raw) {
-  const double err = sqrt(fabs(err_raw));
-  st->error = err;
-  if (!isfinite(err)) {
-    st->status = EXIT_BREAKDOWN;
-    st->n_exit = st->n;
-    return;
-  }
-  if (fabs(err) < st->eps * st->initial_residual) {
-    st->status = EXIT_CONVERGED;
-    st->n_exit = st->n;
-    return;
-  }
-  st->old_error = err;
-  st->n += 1;
-  if (st->n > st->max_iters) {
-    st->status = EXIT_MAX_ITERS;
-    st->n_exit = st->n;
-    return;
-  }
-  if (st->check_switch) {
-    // tea_solve.f90:160-174 evaluated for the next iteration (cheby_calc_steps == 0 here)
-    const bool sw = (!st->first && st->use_ppcg && st->n > 1) ||
-                    (fabs(st->old_error) <= st->epslim && st->n >= st->presteps);
-    if (sw) st->status = STOP_SWITCH;
-  }
-}
 
 // the matvec sweep's sums: p.w (CG), and z.r (PPCG)
 template <bool PPCG>
@@ -94,7 +65,7 @@ struct EpiCgUr {
     st->u_psel = st->n & 1;
     st->rro = rrn;
     st->cg_calc_steps += 1;
-    finish_iteration(st, rrn);
+    loop_finish_iteration(st, rrn);
   }
 };
 
@@ -690,167 +661,6 @@ __global__ void __launch_bounds__(FT, 7) k_cheby_iter_ws(Fields f, Layout L, con
   cp_wait<0>();
 }
 
-// ---- persistent cooperative CG (small meshes) ----------------------------------------------
-// One cooperative launch runs up to `max_run` iterations of the CG loop (tea_solve.f90:341-369)
-// with grid barriers instead of kernel boundaries; the launch and reduction latency of two
-// kernels per iteration dominates below about a million cells.  Per iteration:
-//   phase A  p_n = src + beta p_{n-1} (neighbours' p_n recomputed in place), w = A p_n, p.w;
-//   barrier; every CTA sums the per-CTA partials in the same fixed order -> alpha;
-//   phase B  u += alpha p_n, r -= alpha w (z = Mi r for jac_diag), r.z;
-//   barrier; every CTA sums -> beta, error, the EXIT / switch tests of finish_iteration.
-// Each CTA runs the epilogues on its own shared-memory copy of the loop state (the sums are
-// identical, so are the decisions); CTA 0 writes the alpha/beta history and, at the end, the
-// state.  u is updated in phase B, so no update is left pending.
-// The grid barrier is an arrival counter and a generation word; a wait gives up after
-// PB_SPIN_LIMIT polls (about a second), sets the error word, and every CTA returns with
-// status EXIT_TIMEOUT instead of waiting longer.
-constexpr int PB_T = 256;
-constexpr unsigned long long PB_SPIN_LIMIT = 1ull << 22;  // polls of >= 64 ns plus two L2 atomics each
-
-__device__ __forceinline__ bool pb_barrier(unsigned* arrive, unsigned* gen, unsigned* err, unsigned nblocks) {
-  __shared__ int failed;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    failed = 0;
-    const unsigned g = atomicAdd(gen, 0u);
-    __threadfence();
-    if (atomicAdd(arrive, 1u) == nblocks - 1) {
-      atomicExch(arrive, 0u);
-      __threadfence();
-      atomicAdd(gen, 1u);
-    } else {
-      unsigned long long spins = 0;
-      while (atomicAdd(gen, 0u) == g) {
-        if (atomicAdd(err, 0u) != 0u || ++spins > PB_SPIN_LIMIT) {
-          atomicExch(err, 1u);
-          failed = 1;
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return failed == 0;
-}
-
-// sum of partials[0 .. nb) in a fixed order; the same bits in every CTA
-__device__ __forceinline__ double pb_total(const double* partials, int nb, double* scratch, double* bcast) {
-  double v[1] = {0.0};
-  for (int b = threadIdx.x; b < nb; b += PB_T) v[0] += __ldcg(partials + b);
-  block_sum<1>(v, scratch);
-  if (threadIdx.x == 0) *bcast = v[0];
-  __syncthreads();
-  return *bcast;
-}
-
-// extra_arrivals: arrivals the barriers wait for beyond the grid's CTAs -- 0, except in the test
-// of the bounded wait (an arrival that never comes)
-__global__ void __launch_bounds__(PB_T) k_persistent_cg(LoopArgs a, int max_run, unsigned* bar, int extra_arrivals) {
-  __shared__ LoopState S;
-  __shared__ double scratch[MAX_REDUCE_THREADS];
-  __shared__ double bcast;
-  const Layout L = a.L;
-  const unsigned nb = gridDim.x;
-  const unsigned nwait = nb + (unsigned)extra_arrivals;
-  unsigned* arrive = bar;
-  unsigned* gen = bar + 1;
-  unsigned* err = bar + 2;
-  if (threadIdx.x == 0) S = *a.rd.st;
-  __syncthreads();
-  const bool use_z = a.precond != 1;
-  const double* __restrict__ src = use_z ? a.f.z : a.f.r;
-  const long long ncell = (long long)L.nx * L.ny;
-  const long long stride = (long long)nb * PB_T;
-  double* partA = a.rd.partials;
-  double* partB = a.rd.partials + nb;
-  int done = 0;
-  bool ok = true;
-  while (S.status == RUN && done < max_run) {
-    const int n = S.n;
-    const double* __restrict__ pold = (n & 1) ? a.f.p : a.f.p2;
-    double* __restrict__ pout = (n & 1) ? a.f.p2 : a.f.p;
-    const bool upd = S.p_pending != 0;
-    const double beta = S.beta;
-    auto pn = [&](long long c) { return upd ? fma(beta, pold[c], src[c]) : pold[c]; };
-    // ---- phase A: p_n, w = A p_n, p.w ----
-    double acc[1] = {0.0};
-    for (long long i = (long long)blockIdx.x * PB_T + threadIdx.x; i < ncell; i += stride) {
-      const int j = (int)(i % L.nx) + 1, k = (int)(i / L.nx) + 1;
-      const long long c = L.at(j, k);
-      const double pc = pn(c);
-      // off the domain the neighbour is the mirror value (tl_fused.cu's matvec)
-      const double pt = k < L.ny ? pn(c + L.ld) : pc, pb = k > 1 ? pn(c - L.ld) : pc;
-      const double pr = j < L.nx ? pn(c + 1) : pc, pl = j > 1 ? pn(c - 1) : pc;
-      double wv = a.f.di[c] * pc;
-      wv = fma(-a.f.cy[c + L.ld], pt, wv);
-      wv = fma(-a.f.cy[c], pb, wv);
-      wv = fma(-a.f.cx[c + 1], pr, wv);
-      wv = fma(-a.f.cx[c], pl, wv);
-      a.f.w[c] = wv;
-      pout[c] = pc;
-      acc[0] = fma(wv, pc, acc[0]);
-    }
-    block_sum<1>(acc, scratch);
-    if (threadIdx.x == 0) partA[blockIdx.x] = acc[0];
-    __threadfence();
-    if (!(ok = pb_barrier(arrive, gen, err, nwait))) break;
-    const double pw = pb_total(partA, nb, scratch, &bcast);
-    // EpiCgW
-    const double alpha = S.rro / pw;
-    if (threadIdx.x == 0) {
-      S.u_pending = 0;
-      S.pw = pw;
-      S.alpha = alpha;
-      if (blockIdx.x == 0) a.rd.hist_a[n] = alpha;
-      if (!isfinite(alpha)) {
-        S.status = EXIT_BREAKDOWN;
-        S.n_exit = n;
-      }
-    }
-    __syncthreads();
-    if (S.status != RUN) break;
-    // ---- phase B: u += alpha p_n, r -= alpha w, r.z ----
-    acc[0] = 0.0;
-    for (long long i = (long long)blockIdx.x * PB_T + threadIdx.x; i < ncell; i += stride) {
-      const int j = (int)(i % L.nx) + 1, k = (int)(i / L.nx) + 1;
-      const long long c = L.at(j, k);
-      a.f.u[c] = fma(alpha, pout[c], a.f.u[c]);
-      const double rv = fma(-alpha, a.f.w[c], a.f.r[c]);
-      a.f.r[c] = rv;
-      double zv = rv;
-      if (use_z) {
-        zv = a.f.mi[c] * rv;
-        a.f.z[c] = zv;
-      }
-      acc[0] = fma(rv, zv, acc[0]);
-    }
-    block_sum<1>(acc, scratch);
-    if (threadIdx.x == 0) partB[blockIdx.x] = acc[0];
-    __threadfence();
-    if (!(ok = pb_barrier(arrive, gen, err, nwait))) break;
-    const double rrn = pb_total(partB, nb, scratch, &bcast);
-    // EpiCgUr (u already updated)
-    if (threadIdx.x == 0) {
-      S.rrn = rrn;
-      const double b = rrn / S.rro;
-      S.beta = b;
-      if (blockIdx.x == 0) a.rd.hist_b[n] = b;
-      S.p_pending = 1;
-      S.rro = rrn;
-      S.cg_calc_steps += 1;
-      finish_iteration(&S, rrn);
-    }
-    __syncthreads();
-    ++done;
-  }
-  if (!ok && threadIdx.x == 0) S.status = EXIT_TIMEOUT;
-  __syncthreads();
-  // every CTA's copy is the same; CTA 0 publishes it (after all CTAs read the state at entry)
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.rd.st = S;
-}
-
 // Applies a pending deferred u update (LoopState::u_pending) when the CG loop stops.
 __global__ void __launch_bounds__(FT) k_flush_u(LoopArgs a) {
   const LoopState* st = a.rd.st;
@@ -985,7 +795,7 @@ struct EpiPpcgRrn {
     st->beta = rrn / st->rro;
     st->p_pending = 1;
     st->rro = rrn;
-    finish_iteration(st, rrn);
+    loop_finish_iteration(st, rrn);
     // a blocked FP32 inner sweep of this iteration gave up waiting for a staged row: stop here
     if (rd.counter[MIX_ERR_WORD] != 0u) {
       st->status = EXIT_TIMEOUT;
@@ -1097,26 +907,6 @@ void launch_fused_cg_w(const LoopArgs& a, bool ppcg, cudaStream_t s) {
   cudaLaunchKernel(k, grid, dim3(FT), args, cg_w_smem(mode), s);
 }
 
-int persistent_cg_grid() {
-  int dev = 0, sms = 0, per_sm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persistent_cg, PB_T, 0) != cudaSuccess) return 0;
-  return sms * per_sm;
-}
-
-cudaError_t launch_persistent_cg(const LoopArgs& a, int max_run, unsigned* bar, int grid, cudaStream_t s,
-                                 int extra_arrivals) {
-  const long long ncell = (long long)a.L.nx * a.L.ny;
-  long long need = (ncell + PB_T - 1) / PB_T;
-  int g = (int)(need < grid ? need : grid);
-  if (g < 1) g = 1;
-  LoopArgs aa = a;
-  void* args[] = {&aa, &max_run, &bar, &extra_arrivals};
-  ++launch_counter();
-  return cudaLaunchCooperativeKernel((const void*)k_persistent_cg, dim3(g), dim3(PB_T), args, 0, s);
-}
-
 // Update sweeps: 12 CTAs of 128 threads per SM (1824 on 152 SMs), each striding over rows.
 // At 8192^2 the r -= alpha w, r.r sweep took 0.2514 ms with 1824 CTAs, against 0.2645 with
 // 1696 (11 per SM, rounded to whole strips), 0.2640 with 1984, 0.259 with 2048, 0.266 with
@@ -1177,7 +967,7 @@ namespace {
 
 struct EpiJacobi {
   LoopState* st;
-  __device__ void operator()(double (&acc)[1]) const { finish_iteration(st, acc[0]); }
+  __device__ void operator()(double (&acc)[1]) const { loop_finish_iteration(st, acc[0]); }
 };
 
 // Jacobi iteration n (tea_leaf_jacobi_solve_kernel, jacobi_kernel.f90:26-77) with un and u in

@@ -114,12 +114,19 @@ void launch_fused_ppcg_ur(const LoopArgs& a, bool init_sd, cudaStream_t s);
 void launch_fused_ppcg_rrn(const LoopArgs& a, bool copy_z, cudaStream_t s);
 // u += alpha p of the last CG iteration when it is still pending (end of a CG phase)
 void launch_flush_u(const LoopArgs& a, cudaStream_t s);
-// persistent cooperative CG (no preconditioner or jac_diag): up to max_run iterations in one
-// launch; bar = three zeroed words (barrier counter, generation, error); grid = the co-resident
-// CTA count from persistent_cg_grid() (0 if it cannot be determined)
-int persistent_cg_grid();
-cudaError_t launch_persistent_cg(const LoopArgs& a, int max_run, unsigned* bar, int grid, cudaStream_t s,
-                                 int extra_arrivals = 0);
+// persistent cooperative CG on chip (no preconditioner or jac_diag; tl_persist.cu): the mesh in
+// tiles of tw x th cells, one per CTA, clusters of cs CTAs, a thread owning one column and every
+// ry-th row of its tile
+struct PersistPlan {
+  int gx, gy, tw, th, ry, variant, cs;
+};
+// the plan of a mesh on the current device; false if it does not fit on chip
+bool persist_prepare(int nx, int ny, int precond, PersistPlan* out);
+size_t persist_box_bytes(const PersistPlan& p);  // its grid sums' inboxes and the tiles' halo boxes
+// up to max_run iterations in one launch; epoch .. epoch + 2 max_run - 1 number its grid sums, and
+// no earlier launch on these boxes (zeroed once) has used them or higher ones
+cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch,
+                                 void* box, cudaStream_t s, int extra = 0);
 // one Jacobi iteration from un into u_out (the two swap every iteration), error and the loop's
 // test in the epilogue
 void launch_fused_jacobi(const LoopArgs& a, const double* un, double* u_out, cudaStream_t s);

@@ -1,0 +1,688 @@
+// tl_persist.cu -- the persistent CG kernel of meshes that fit on chip: one cooperative launch
+// runs many iterations of the CG loop (tea_solve.f90:341-369) with the whole problem held in
+// shared memory and registers.
+//
+// Each CTA (one per SM) owns a tile of the mesh.  p with its one-cell halo, the scaled face
+// coefficients and Di live in shared memory, r, w (and u, when the registers allow) in the
+// registers of the thread that owns the cell: a thread owns one column and every ry-th row of its
+// tile.  Per iteration:
+//   phase A  p_n = src + beta p_{n-1} on the tile and its halo (from the neighbours' src at the
+//            tile's rim), w = A p_n, p.w; grid sum -> alpha;
+//   phase B  u += alpha p_n, r -= alpha w (z = Mi r with jac_diag), r.z, the rim's src sent to the
+//            neighbour tiles; grid sum -> beta, error, the EXIT / switch tests.
+// HBM and L2 see the rims and the partial sums only; the fields are read when a launch starts and
+// written when it ends.
+//
+// What bounds it: below about 300^2 cells the latency of the two grid sums and of the FP64
+// operations in a row (61 cycles each for one warp), above that the FP64 pipe.  So
+// - a grid sum is one hop: the first warp stores the CTA's partial, tagged with the sum's number,
+//   into every CTA's inbox, and five warps poll the CTA's own inbox, a word a lane, until all
+//   partials have come (3300 cycles on 152 CTAs; 4400 when one warp polls five words a lane).  One
+//   table of partials that all CTAs poll takes 7000 cycles, since every store then waits behind the
+//   polls of its line; an arrival counter with a generation word is two dependent atomics and a
+//   second read.  Summing in clusters of 4 first (2600 cycles by itself) loses by its second
+//   conversion: the loop's scalar code runs on one warp, at the rate its instructions are fetched.
+//   A mesh of a few thousand cells takes one cluster of up to 16 CTAs, which exchange through
+//   shared memory (600 cycles), one of a few hundred a single CTA;
+// - the rim goes the same way: its owner stores each value with the sum's number into the
+//   neighbour tile's box, and the neighbour's threads poll for it while the first warp waits for
+//   the sum.  Publishing it through the field needs a fence (1900 cycles) before the sum;
+// - sums across threads are integers relative to the largest exponent, not FP64 additions: an FP64
+//   instruction holds a sub-partition's pipe for 64 cycles however few lanes need it.
+//
+// Time per CG iteration, the solve's set-up included, against the form before it (up to 640K cells
+// one persistent kernel with the fields in memory and two barriers an iteration, above the batched
+// sweeps of tl_fused.cu in CUDA graphs): 64^2 3.9 against 12 us, 128^2 5.9 / 13.8, 256^2 7.2 / 14.5,
+// 512^2 10.4 / 27.6, 777 x 1013 with jac_diag 24.2 / 43.9, 1000^2 27.4 / 47, 1024^2 27.2 / 42.4.
+// Every mesh that fits runs here: the largest, 1100^2, is where it gains least.  The FP64 pipe's
+// share is 1.1 us at 256^2 and 17 us at 1000^2.
+#include "tl_kernels.cuh"
+
+namespace tl {
+
+namespace {
+
+constexpr int PTHREADS = 512;  // threads per CTA
+constexpr int PT = PTHREADS - 32;  // those that own cells: all but the first warp, which exchanges the sums
+constexpr int PW = PT / 32;    // their warps
+constexpr int PH = 2;          // halo cells per thread at most
+constexpr int POLLW = 5;       // warps that poll the inbox at most
+constexpr int SLOTS = 32 * POLLW;            // words of an inbox
+constexpr int PERSIST_MAX_CTAS = SLOTS - 1;  // one is left for the test of the bounded wait
+constexpr int MAX_CLUSTER = 16;                  // CTAs of a cluster
+constexpr size_t PERSIST_SMEM_MAX = 225 * 1024;
+// polls before a wait gives up (about a second: a poll takes an L2 round trip; one of shared
+// memory some 50 cycles)
+constexpr unsigned PERSIST_POLL_LIMIT = 1u << 21;
+constexpr unsigned PERSIST_POLL_LIMIT_SM = 1u << 25;
+
+struct PersistArgs {
+  LoopArgs a;
+  PersistPlan pl;
+  int max_run;
+  unsigned epoch;   // number of the launch's first grid sum
+  ulonglong2* box;  // by parity of the sum's number, an inbox per CTA; then the tiles' halo boxes
+  int extra;        // partials waited for beyond the grid's (the test of the bounded wait)
+};
+
+// Sums across lanes: a value as an integer multiple of 2^(e - 1075 - FSH), e the largest biased
+// exponent among the values, rounded to nearest; the integers are added exactly, so the result does
+// not depend on an order.  A value's rounding error is at most 2^-55 of the largest, where an FP64
+// tree makes one of 2^-53 at each level.
+constexpr int FSH = 1;  // 53 + FSH bits for the largest value: 512 of them fit 63 bits
+struct Fix {
+  long long q;
+  unsigned e;  // 0x7ff: an infinity or NaN among the values
+};
+__device__ __forceinline__ unsigned expo(double v) { return (unsigned)(emu::bits(v) >> 52) & 0x7ffu; }
+// the sum over the warp of q (|q| < 2^58), as limbs of 21 bits through redux.sync
+__device__ __forceinline__ long long warp_add(long long q) {
+  const int l0 = __reduce_add_sync(0xffffffffu, (int)(q & 0x1fffff));
+  const int l1 = __reduce_add_sync(0xffffffffu, (int)((q >> 21) & 0x1fffff));
+  const int l2 = __reduce_add_sync(0xffffffffu, (int)(q >> 42));
+  return (long long)l0 + ((long long)l1 << 21) + ((long long)l2 << 42);
+}
+__device__ __forceinline__ Fix warp_fix(double v) {
+  const uint64_t b = emu::bits(v);
+  const unsigned ev = max((unsigned)(b >> 52) & 0x7ffu, 1u);
+  const unsigned e = __reduce_max_sync(0xffffffffu, ev);
+  const uint64_t m = (b & emu::FRAC) | ((b << 1 >> 53) ? emu::HIDDEN : 0ull);
+  const long long i = (long long)((((m << (FSH + 1)) >> min(e - ev, 63u)) + 1ull) >> 1);
+  return Fix{warp_add((b & emu::SIGN) ? -i : i), e};
+}
+// the sum over the warp of sums, one a lane, of at most 16 lanes or of single values
+__device__ __forceinline__ Fix warp_fix(const Fix& f) {
+  const unsigned e = __reduce_max_sync(0xffffffffu, f.e);
+  const unsigned d = min(e - f.e, 63u);
+  return Fix{warp_add((f.q + (d ? 1ll << (d - 1) : 0ll)) >> d), e};
+}
+__device__ __noinline__ double scale_slowly(double t, int k) { return ldexp(t, k); }
+__device__ __forceinline__ double fix_value(const Fix& f) {
+  if (f.e == 0x7ffu) return emu::from_bits(emu::QNAN);
+  const double t = (double)f.q;
+  const int k = (int)f.e - 1075 - FSH, et = (int)expo(t);
+  if (et == 0) return t;  // zero
+  if (et + k >= 1 && et + k < 0x7ff) return emu::from_bits(emu::bits(t) + ((uint64_t)(long long)k << 52));
+  return scale_slowly(t, k);
+}
+
+// A value in a box: its halves, each beside the sum's number, so that either word shows by itself
+// that it belongs to this sum.
+__device__ __forceinline__ void box_put(ulonglong2* s, double v, unsigned epoch) {
+  const unsigned long long b = emu::bits(v);
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(s), "l"((b & 0xffffffff00000000ull) | epoch),
+               "l"((b << 32) | epoch)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 box_get(const ulonglong2* s) {
+  ulonglong2 w;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w.x), "=l"(w.y) : "l"(s) : "memory");
+  return w;
+}
+__device__ __forceinline__ bool box_is(const ulonglong2& w, unsigned epoch) {
+  return (unsigned)w.x == epoch && (unsigned)w.y == epoch;
+}
+__device__ __forceinline__ double box_value(const ulonglong2& w) {
+  return emu::from_bits((w.x & 0xffffffff00000000ull) | (w.y >> 32));
+}
+// the same in the shared memory of a CTA of the cluster
+__device__ __forceinline__ void cbox_put(const ulonglong2* s, unsigned rank, double v, unsigned epoch) {
+  const unsigned long long b = emu::bits(v);
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(s)), "r"(rank));
+  asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(a),
+               "l"((b & 0xffffffff00000000ull) | epoch), "l"((b << 32) | epoch)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 cbox_get(const ulonglong2* s) {
+  ulonglong2 w;
+  asm volatile("ld.relaxed.cluster.shared::cta.v2.u64 {%0, %1}, [%2];"
+               : "=l"(w.x), "=l"(w.y)
+               : "r"((unsigned)__cvta_generic_to_shared(s))
+               : "memory");
+  return w;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\n barrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool finite_bits(double v) { return expo(v) != 0x7ffu; }
+template <int ID, int N>
+__device__ __forceinline__ void bar_sync() {
+  asm volatile("barrier.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+template <int ID, int N>
+__device__ __forceinline__ void bar_arrive() {
+  asm volatile("barrier.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+  asm volatile("barrier.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// x, in a way that keeps the compiler from computing what follows from it once for all iterations:
+// the addresses of a thread's cells would take as many registers as the cells themselves
+__device__ __forceinline__ int fresh(int x) {
+  asm volatile("" : "+r"(x));
+  return x;
+}
+
+// What the exchange of a sum needs, in shared memory.
+struct Exchange {
+  Fix part[PW];        // the owning warps' sums
+  Fix inbox[POLLW];    // the polling warps' sums
+  ulonglong2 cbox[2][MAX_CLUSTER + 1];  // one cluster: its CTAs' partials, by parity of the sum's number
+  int fail;            // a wait ran out
+};
+
+// First warp: the owning warps' sums added up over the grid; meanwhile() runs while the partials
+// are on their way.  in: the inboxes of this parity.  Not inlined, so that both sums of an
+// iteration run the same instructions.
+__device__ __noinline__ double exchange_sum(Exchange* x, ulonglong2* in, unsigned epoch, int ctas, int cs, int extra,
+                                            double rro, double* inv_rro) {
+  const int lane = threadIdx.x & 31;
+  bar_sync<1, PTHREADS>();
+  Fix p{0, 1u};
+  if (lane < PW) p = x->part[lane];
+  double total = fix_value(warp_fix(p));
+  if (ctas > cs) {
+#pragma unroll
+    for (int q = 0; q < POLLW; ++q)
+      if (lane + 32 * q < ctas) box_put(in + (size_t)(lane + 32 * q) * SLOTS + blockIdx.x, total, epoch);
+    if (inv_rro) *inv_rro = 1.0 / rro;  // while the partials are on their way
+    const int nq = (ctas + extra + 31) / 32;
+    bar_sync(3, 32 * (nq + 1));
+    p = Fix{0, 1u};
+    if (lane < nq) p = x->inbox[lane];
+    total = fix_value(warp_fix(p));
+  } else {
+    const int mine = cs + extra;
+    if (mine > 1) {
+      const ulonglong2* box = x->cbox[epoch & 1u];
+      if (lane < cs) cbox_put(box + blockIdx.x, lane, total, epoch);
+      if (inv_rro) *inv_rro = 1.0 / rro;
+      ulonglong2 w = make_ulonglong2(0ull, 0ull);
+      bool here = lane >= mine;
+      for (unsigned tries = 0; !here && tries < PERSIST_POLL_LIMIT_SM; ++tries) {
+        w = cbox_get(box + lane);
+        here = box_is(w, epoch);
+      }
+      if (!here) x->fail = 1;
+      __syncwarp();
+      total = fix_value(warp_fix(lane < mine ? box_value(w) : 0.0));
+    } else if (inv_rro) {
+      *inv_rro = 1.0 / rro;
+    }
+  }
+  return total;
+}
+
+// The threads but the first warp's own the cells.  The first warp exchanges the sums and runs the
+// loop's scalar steps, so that in the wait for beta the owners update u and fetch the halo.  The
+// warps meet at
+//   1  the owning warps' sums are in shared memory (owners arrive, the first warp waits);
+//   2  owners only: p is complete in shared memory;
+//   3  the words of the inbox are added up (the polling warps arrive, the first warp waits);
+//   0  the sum's outcome is in shared memory (all).
+// M: cells a thread may own.  From sizes up on a tile's share grows past the registers and the
+// shared memory: p of the owned cells stays in registers too up to 4, u and Mi up to 6 (they are in
+// the fields otherwise, u updated in the wait for beta), and Di is read from the field above 14.
+template <int M, bool DIAG>
+__global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
+  constexpr bool PREG = M <= 4, UREG = M <= 6, DISM = M <= 14;
+  __shared__ LoopState S;
+  __shared__ Exchange X;
+  __shared__ double sh_alpha, sh_beta;
+  __shared__ int sh_status;
+  extern __shared__ __align__(16) double psm[];
+  const Layout L = g.a.L;
+  const Fields& f = g.a.f;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const bool owner = wid != 0;
+  const int to = t - 32;  // number of the owner
+  const int cs = g.pl.cs, ctas = gridDim.x;
+  if (t < 2 * (MAX_CLUSTER + 1)) X.cbox[t / (MAX_CLUSTER + 1)][t % (MAX_CLUSTER + 1)] = make_ulonglong2(0ull, 0ull);
+  if (t == 0) {
+    S = *g.a.rd.st;
+    sh_status = S.status;
+    sh_beta = S.beta;
+    X.fail = 0;
+  }
+  if (cs > 1)
+    cluster_sync();  // every CTA's box is empty before a peer writes into it
+  else
+    __syncthreads();
+  if (sh_status != RUN) return;  // in every CTA
+
+  const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
+  const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;  // first cell of the tile, from 0
+  const bool tile = owner && by < g.pl.gy;  // one cluster: the last CTAs may have no tile
+  const int tw = tile ? min(g.pl.tw, L.nx - j0) : 0, th = tile ? min(g.pl.th, L.ny - k0) : 0;
+  const int P = g.pl.tw + 2, ry = g.pl.ry;
+  const int asz = (g.pl.th + 2) * P;
+  double* const sp = psm;
+  double* const scx = psm + asz;
+  double* const scy = psm + 2 * asz;
+  double* const sdi = psm + 3 * asz;
+
+  // the thread's column and first row; cells i = 0 .. mine-1 at rows ty + i ry
+  const int tx = owner ? to % g.pl.tw : 0, ty = owner ? to / g.pl.tw : 0;
+  const int mine = (tx < tw && ty < ry && ty < th) ? (th - 1 - ty) / ry + 1 : 0;
+  const int o0 = (ty + 1) * P + tx + 1;
+  const int c0 = (int)L.at(j0 + tx + 1, k0 + ty + 1);
+  const int ostep = ry * P, cstep = ry * L.ld;
+  const int i_first = ty == 0 ? 0 : -1, i_last = (mine > 0 && (th - 1 - ty) % ry == 0) ? mine - 1 : -1;
+  const bool at_l = tx == 0 && j0 == 0, at_r = tx == tw - 1 && j0 + tw == L.nx;  // at the domain's side
+  const int i_b = k0 == 0 ? i_first : -1, i_t = k0 + th == L.ny ? i_last : -1;
+
+  // A tile's halo box: its left column, right column (th each), bottom row, top row (tw each).
+  const int hbox = 2 * (g.pl.th + g.pl.tw);
+  ulonglong2* const halo = g.box + (size_t)2 * gridDim.x * SLOTS;
+  // halo cells this thread fetches (those beside other tiles): p there, and the next source
+  int ho[PH], hh[PH];
+  double hp[PH], hs[PH];
+  double* const src = DIAG ? f.z : f.r;
+  int n = S.n;
+  const double* const pold = (n & 1) ? f.p : f.p2;
+  bool upd = S.p_pending != 0;
+#pragma unroll
+  for (int q = 0; q < PH; ++q) {
+    const int h = to + q * PT;
+    ho[q] = -1;
+    hh[q] = 0;
+    hp[q] = hs[q] = 0.0;
+    int x = -1, y = h;
+    bool is = j0 > 0 && y < th;
+    if (h >= g.pl.th) x = tw, y = h - g.pl.th, is = j0 + tw < L.nx && y < th;
+    if (h >= 2 * g.pl.th) x = h - 2 * g.pl.th, y = -1, is = k0 > 0 && x < tw;
+    if (h >= 2 * g.pl.th + g.pl.tw) x = h - 2 * g.pl.th - g.pl.tw, y = th, is = k0 + th < L.ny && x < tw;
+    if (is && tile && h < hbox) {
+      ho[q] = (y + 1) * P + x + 1;
+      hh[q] = (int)blockIdx.x * hbox + h;
+      const int c = (int)L.at(j0 + x + 1, k0 + y + 1);
+      hp[q] = pold[c];
+      if (upd) hs[q] = src[c];
+    }
+  }
+  // where the thread's rim cells go: the neighbour tiles' boxes (-1: no such neighbour)
+  const int to_l = (tx == 0 && j0 > 0) ? ((int)blockIdx.x - 1) * hbox + g.pl.th + ty : -1;
+  const int to_r = (tx == tw - 1 && j0 + tw < L.nx) ? ((int)blockIdx.x + 1) * hbox + ty : -1;
+  const int rim_b = k0 > 0 ? i_first : -1, rim_t = k0 + th < L.ny ? i_last : -1;
+  const int to_b = ((int)blockIdx.x - g.pl.gx) * hbox + 2 * g.pl.th + g.pl.tw + tx;
+  const int to_t = ((int)blockIdx.x + g.pl.gx) * hbox + 2 * g.pl.th + tx;
+
+  double r[M], w[M], u[UREG ? M : 1], mi[UREG && DIAG ? M : 1], pr[PREG ? M : 1];
+  // (w holds the source z of the next p between phases B and A with DIAG)
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const int o = o0 + i * ostep, c = c0 + i * cstep;
+    r[i] = w[i] = 0.0;
+    if (UREG) u[i] = 0.0;
+    if (UREG && DIAG) mi[i] = 0.0;
+    if (PREG) pr[i] = 0.0;
+    if (i < mine) {
+      r[i] = f.r[c];
+      if (DIAG) w[i] = f.z[c];
+      if (UREG) u[i] = f.u[c];
+      if (UREG && DIAG) mi[i] = f.mi[c];
+      if (PREG)
+        pr[i] = pold[c];
+      else
+        sp[o] = pold[c];
+      if (DISM) sdi[o] = f.di[c];
+      scx[o] = f.cx[c];
+      scy[o] = f.cy[c];
+      if (tx == tw - 1) scx[o + 1] = f.cx[c + 1];
+      if (i == i_last) scy[o + P] = f.cy[c + L.ld];
+    }
+  }
+
+  // scalars of the loop, in the first warp
+  const double goal = S.eps * S.initial_residual;
+  const uint64_t goal2 = emu::bits(goal > 1e-140 ? goal * goal * (1.0 + 1e-12) : INFINITY);
+  double rro = S.rro, inv_rro = 0.0, pw = S.pw, alpha_ = S.alpha, beta_ = S.beta, rrn = S.rrn;
+  const bool check_switch = S.check_switch != 0;
+  const int max_iters = S.max_iters;
+  bool error_due = false;
+  unsigned epoch = g.epoch;
+  __syncthreads();
+
+  // owners: the warp's sum of v; then the polling warps' share of the grid's
+  auto give = [&](double v) {
+    const Fix s = warp_fix(v);
+    if (lane == 0) X.part[wid - 1] = s;
+    bar_arrive<1, PTHREADS>();
+  };
+  const int nwait = ctas > cs ? ctas + g.extra : 0, nq = (nwait + 31) / 32;
+  auto poll = [&] {
+    if (wid > nq) return;
+    const int slot = (wid - 1) * 32 + lane;
+    const ulonglong2* in = g.box + ((size_t)(epoch & 1u) * ctas + blockIdx.x) * SLOTS + slot;
+    ulonglong2 x = make_ulonglong2(0ull, 0ull);
+    bool here = slot >= nwait;
+    for (unsigned tries = 0; !here && tries < PERSIST_POLL_LIMIT; ++tries) {
+      x = box_get(in);
+      here = box_is(x, epoch);
+    }
+    if (!here) X.fail = 1;
+    __syncwarp();
+    const Fix q = warp_fix(slot < nwait ? box_value(x) : 0.0);
+    if (lane == 0) X.inbox[wid - 1] = q;
+    bar_arrive(3, 32 * (nq + 1));
+  };
+  auto inboxes = [&] { return g.box + (size_t)(epoch & 1u) * ctas * SLOTS; };
+
+  int done = 0;
+  bool updated = false;  // phase B of the last iteration ran
+  for (; done < g.max_run; ++done) {
+    // ---- phase A: p_n on the tile and its halo (off the domain the mirror value), w = A p_n, p.w ----
+    updated = false;
+    if (owner) {
+      const double beta = sh_beta;
+      // the even iterations' p is what the loop leaves in the field p
+      double* const pf = (n & 1) ? nullptr : f.p;
+      int o = fresh(o0), c = fresh(c0);
+#pragma unroll
+      for (int i = 0; i < M; ++i, o += ostep, c += cstep) {
+        if (i < mine) {
+          double p = PREG ? pr[i] : sp[o];
+          if (upd) p = fma(beta, p, DIAG ? w[i] : r[i]);
+          if (PREG) pr[i] = p;
+          sp[o] = p;
+          if (pf) pf[c] = p;
+          if (at_l) sp[o - 1] = p;
+          if (at_r) sp[o + 1] = p;
+          if (i == i_b) sp[o - P] = p;
+          if (i == i_t) sp[o + P] = p;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < PH; ++q)
+        if (ho[q] >= 0) {
+          if (upd) hp[q] = fma(beta, hp[q], hs[q]);
+          sp[ho[q]] = hp[q];
+        }
+      bar_sync<2, PT>();
+      double acc = 0.0;
+      o = fresh(o0);
+      c = fresh(c0);
+#pragma unroll
+      for (int i = 0; i < M; ++i, o += ostep, c += cstep) {
+        if (i < mine) {
+          const double pc = PREG ? pr[i] : sp[o];
+          double wv = (DISM ? sdi[o] : __ldg(f.di + c)) * pc;
+          wv = fma(-scy[o + P], sp[o + P], wv);
+          wv = fma(-scy[o], sp[o - P], wv);
+          wv = fma(-scx[o + 1], sp[o + 1], wv);
+          wv = fma(-scx[o], sp[o - 1], wv);
+          w[i] = wv;
+          acc = fma(wv, pc, acc);
+        }
+      }
+      give(acc);
+      poll();
+    } else {
+      pw = exchange_sum(&X, inboxes(), epoch, ctas, cs, g.extra, rro, &inv_rro);
+      alpha_ = rro / pw;
+      if (lane == 0) {
+        sh_alpha = alpha_;
+        if (!finite_bits(alpha_)) {
+          S.status = EXIT_BREAKDOWN;
+          S.n_exit = n;
+          sh_status = EXIT_BREAKDOWN;
+        }
+        if (blockIdx.x == 0) g.a.rd.hist_a[n] = alpha_;
+      }
+    }
+    ++epoch;
+    __syncthreads();
+    if (X.fail || sh_status != RUN) break;
+    // ---- phase B: r -= alpha w, z = Mi r, r.z; the rim to the neighbours; u += alpha p_n ----
+    if (owner) {
+      const double alpha = sh_alpha;
+      double acc = 0.0;
+      int c = fresh(c0), l = fresh(to_l), e = fresh(to_r);
+#pragma unroll
+      for (int i = 0; i < M; ++i, c += cstep, l += ry, e += ry) {
+        if (i < mine) {
+          const double rv = fma(-alpha, w[i], r[i]);
+          r[i] = rv;
+          double zv = rv;
+          if (DIAG) {
+            zv = (UREG ? mi[i] : __ldg(f.mi + c)) * rv;
+            w[i] = zv;
+          }
+          if (to_l >= 0) box_put(halo + l, zv, epoch);
+          if (to_r >= 0) box_put(halo + e, zv, epoch);
+          if (i == rim_b) box_put(halo + to_b, zv, epoch);
+          if (i == rim_t) box_put(halo + to_t, zv, epoch);
+          acc = fma(rv, zv, acc);
+        }
+      }
+      give(acc);
+      poll();
+      int o = fresh(o0);
+      c = fresh(c0);
+#pragma unroll
+      for (int i = 0; i < M; ++i, o += ostep, c += cstep) {
+        if (i < mine) {
+          const double pc = PREG ? pr[i] : sp[o];
+          if (UREG)
+            u[i] = fma(alpha, pc, u[i]);
+          else
+            f.u[c] = fma(alpha, pc, f.u[c]);
+        }
+      }
+      bool got = false;
+      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+        got = true;
+#pragma unroll
+        for (int q = 0; q < PH; ++q)
+          if (ho[q] >= 0) {
+            const ulonglong2 x = box_get(halo + hh[q]);
+            got = got && box_is(x, epoch);
+            hs[q] = box_value(x);
+          }
+      }
+      if (!got) X.fail = 1;
+    } else {
+      rrn = exchange_sum(&X, inboxes(), epoch, ctas, cs, g.extra, rro, nullptr);
+      // rrn / rro from the reciprocal of rro: one correction gives the correctly rounded quotient
+      // in the normal range (P. Markstein, IBM J. Res. Dev. 34(1), 1990); else the division
+      double b = rrn * inv_rro;
+      b = fma(fma(-b, rro, rrn), inv_rro, b);
+      const unsigned eb = expo(b), eo = expo(rro);
+      if (eb < 300u || eb > 1700u || eo < 300u || eo > 1700u) b = rrn / rro;
+      beta_ = b;
+      // without the square root when the outcome is plain: the error is far enough above the goal
+      // (goal2: its square with a margin; non-negative doubles order as their bits) and nothing
+      // else can stop the loop.  The error itself is then left to the launch's end.
+      error_due = !check_switch && n < max_iters && (emu::bits(rrn) & ~emu::SIGN) > goal2 && expo(rrn) < 2000u;
+      if (lane == 0) {
+        sh_beta = b;
+        if (!error_due) {
+          S.n = n;
+          loop_finish_iteration(&S, rrn);
+          sh_status = S.status;
+        }
+        if (blockIdx.x == 0) g.a.rd.hist_b[n] = b;
+      }
+      rro = rrn;
+    }
+    ++epoch;
+    updated = true;
+    upd = true;
+    ++n;
+    __syncthreads();
+    if (X.fail || sh_status != RUN) {
+      ++done;
+      break;
+    }
+  }
+  if (cs > 1) cluster_sync();  // no CTA leaves while a peer may still write into its shared memory
+  if (X.fail) {
+    if (t == 0) g.a.rd.st->status = EXIT_TIMEOUT;
+    return;
+  }
+  // ---- the fields and the state as the loop's kernels leave them (w = A p_n formed again) ----
+  const int last = updated ? n - 1 : n;  // the iteration whose p is in shared memory
+  double* const pout = (last & 1) ? f.p2 : f.p;
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const int o = o0 + i * ostep, c = c0 + i * cstep;
+    if (i < mine) {
+      const double pc = sp[o];
+      double wv = (DISM ? sdi[o] : f.di[c]) * pc;
+      wv = fma(-scy[o + P], sp[o + P], wv);
+      wv = fma(-scy[o], sp[o - P], wv);
+      wv = fma(-scx[o + 1], sp[o + 1], wv);
+      wv = fma(-scx[o], sp[o - 1], wv);
+      f.w[c] = wv;
+      pout[c] = pc;
+      f.r[c] = r[i];
+      if (UREG) f.u[c] = u[i];
+      if (DIAG && updated) f.z[c] = w[i];
+    }
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    S.u_pending = 0;
+    S.pw = pw;
+    S.alpha = alpha_;
+    S.cg_calc_steps += done;
+    if (done > 0) {
+      S.rrn = rrn;
+      S.beta = beta_;
+      S.rro = rro;
+      S.p_pending = 1;
+      if (error_due) {
+        S.n = n;
+        S.error = S.old_error = sqrt(fabs(rrn));
+      }
+    }
+    *g.a.rd.st = S;
+  }
+}
+
+using PersistKernel = void (*)(PersistArgs);
+struct PersistVariant {
+  int m;
+  PersistKernel k[2];  // without / with jac_diag
+};
+#define PERSIST_VARIANT(M) {M, {k_persistent_cg<M, false>, k_persistent_cg<M, true>}}
+const PersistVariant kVariants[] = {PERSIST_VARIANT(1), PERSIST_VARIANT(2),  PERSIST_VARIANT(4),  PERSIST_VARIANT(6),
+                                    PERSIST_VARIANT(8), PERSIST_VARIANT(11), PERSIST_VARIANT(14), PERSIST_VARIANT(18)};
+
+// p, cx, cy and, up to 14 cells a thread, Di
+size_t plan_smem(const PersistPlan& p) {
+  return (size_t)(kVariants[p.variant].m <= 14 ? 4 : 3) * (p.th + 2) * (p.tw + 2) * sizeof(double);
+}
+
+// A launch of a plan: cooperative (its CTAs wait for one another), in clusters.
+struct PersistLaunch {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[2];
+  PersistLaunch(int ctas, int cs, size_t smem, cudaStream_t s) {
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(PTHREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeCooperative;
+    at[1].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+  }
+};
+
+// Clusters of cs CTAs of kernel k that are co-resident (0: none).  Sets the attributes a launch
+// needs, the same for every plan: contexts share them.
+int persist_clusters(const void* k, int cs, size_t smem) {
+  int n = 0;
+  PersistLaunch l(cs, cs, smem, nullptr);
+  l.cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, k, &l.cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+}  // namespace
+
+int persist_ctas(const PersistPlan& p) { return (p.gx * p.gy + p.cs - 1) / p.cs * p.cs; }
+
+size_t persist_box_bytes(const PersistPlan& p) {
+  return (size_t)persist_ctas(p) * (2 * SLOTS + 2 * (p.th + p.tw)) * sizeof(ulonglong2);
+}
+
+// The tiling of an nx x ny mesh with the least cycles an iteration: FP64 instructions of a warp on
+// the busiest SM (10 an iteration and cell, 17 cycles of the SM's four pipes each), the halo, and
+// the two grid sums' exchange (700 more cycles each in one cluster, 3200 across the grid).
+// clusters[i]: co-resident clusters of 2^i CTAs.
+bool persist_plan(int nx, int ny, const int (&clusters)[5], PersistPlan* out) {
+  double best = 0.0;
+  bool found = false;
+  // one CTA, one cluster of 2 .. 16, all SMs
+  const int kinds[6][2] = {{1, 1}, {2, 1}, {4, 1}, {8, 1}, {16, 1}, {1, PERSIST_MAX_CTAS}};
+  for (const auto& kind : kinds) {
+    const int cs = kind[0];
+    int have = 0;
+    for (int i = 0; i < 5; ++i)
+      if (cs == 1 << i) have = clusters[i];
+    const int ctas = cs * (have < kind[1] ? have : kind[1]);
+    for (int g0 = 1; g0 <= ctas && g0 <= nx; ++g0) {
+      const int tw = (nx + g0 - 1) / g0;
+      if (tw > PT) continue;
+      PersistPlan p;
+      p.cs = cs;
+      p.tw = tw;
+      p.gx = (nx + tw - 1) / tw;
+      int gy = ctas / p.gx;
+      if (gy > ny) gy = ny;
+      if (gy < 1) continue;
+      p.th = (ny + gy - 1) / gy;
+      p.gy = (ny + p.th - 1) / p.th;
+      p.ry = PT / tw < p.th ? PT / tw : p.th;
+      const int m = (p.th + p.ry - 1) / p.ry;
+      p.variant = -1;
+      for (int v = (int)(sizeof(kVariants) / sizeof(kVariants[0])) - 1; v >= 0; --v)
+        if (kVariants[v].m >= m) p.variant = v;
+      const int halo = 2 * (p.tw + p.th);
+      if (p.variant < 0 || halo > PH * PT || plan_smem(p) > PERSIST_SMEM_MAX) continue;
+      const double slabs = (double)((p.ry * tw + 31) / 32) * m;
+      const double sums = kind[1] > 1 ? 3200.0 : (cs > 1 ? 700.0 : 0.0);
+      const double cost = slabs * 170.0 + 0.5 * halo + 8.0 * p.th + 2.0 * sums;
+      if (!found || cost < best) {
+        best = cost;
+        *out = p;
+        found = true;
+      }
+    }
+  }
+  return found;
+}
+
+// Plans the mesh for the current device; false if it does not fit on chip.
+bool persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
+  int clusters[5];
+  const int diag = precond == 2 ? 1 : 0;
+  const void* k0 = (const void*)kVariants[0].k[diag];
+  for (int i = 0; i < 5; ++i) clusters[i] = persist_clusters(k0, 1 << i, PERSIST_SMEM_MAX);
+  if (!persist_plan(nx, ny, clusters, out)) return false;
+  const int n = persist_clusters((const void*)kVariants[out->variant].k[diag], out->cs, plan_smem(*out));
+  return n * out->cs >= persist_ctas(*out);
+}
+
+cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch, void* box,
+                                 cudaStream_t s, int extra) {
+  PersistArgs g{a, p, max_run, epoch, static_cast<ulonglong2*>(box), extra};
+  void* args[] = {&g};
+  PersistLaunch l(persist_ctas(p), p.cs, plan_smem(p), s);
+  ++launch_counter();
+  return cudaLaunchKernelExC(&l.cfg, (const void*)kVariants[p.variant].k[a.precond == 2 ? 1 : 0], args);
+}
+
+}  // namespace tl
