@@ -100,12 +100,13 @@ struct tl_ctx {
   cudaGraphExec_t cg_prof_exec = nullptr;
   LoopArgs cg_prof_key{};
   long long cg_prof_nk = 0;
-  // persistent CG kernel: -1 not yet planned, 0 the mesh does not fit, 1 pplan holds; the boxes
-  // its CTAs exchange partial sums and rims in, and the number of the next sum
-  int pstate = -1;
-  PersistPlan pplan{};
-  void* pbox = nullptr;
-  unsigned pepoch = 0;
+  // the persistent on-chip loops: FP64 CG, and the FP32 process of the precision form
+  struct Persist {
+    int state = -1;  // -1 not yet planned, 0 the mesh does not fit, 1 plan holds
+    PersistPlan plan{};
+    void* box = nullptr;  // what its CTAs exchange partial sums and rims in
+    unsigned epoch = 0;   // number of the next sum
+  } pcg, pmix;
   // host transfers: an upload and a download stream (tl_stage_state, tl_fetch_field) and
   // XFER_FIELDS staging fields -- two staged (density, energy1) pairs, the fetch snapshot, and
   // two for the synchronous uploads / downloads.  A host array moves as one contiguous copy
@@ -336,8 +337,8 @@ bool writes_setup_input(int field) {
          field == TL_FIELD_MI;
 }
 
-// The persistent CG kernel takes every plain or jac_diag CG whose mesh fits on chip (about a
-// million cells).  TL_CG_PERSISTENT=0 forces it off.
+// The persistent on-chip loops take every plain or jac_diag CG whose mesh fits: FP64 to about 1100^2
+// cells, the FP32 process of the precision form to about 2050^2.  TL_CG_PERSISTENT=0 forces them off.
 constexpr int PERSIST_RUN = 1024;  // iterations per launch at most (the host reads the status between)
 
 // TL_CHEBY_SWEEP=0: the FP64 Chebyshev iterations as the two one-step kernels instead of one
@@ -354,32 +355,50 @@ bool use_ppcg_inner_sweep() {
   return !(e && e[0] == '0');
 }
 
-bool use_persistent(tl_ctx* c) {
+template <typename F>
+bool use_persistent(tl_ctx* c, tl_ctx::Persist& p, F&& prepare) {
   if (c->prof || c->g.precond == TL_PREC_JAC_BLOCK) return false;
   const char* e = getenv("TL_CG_PERSISTENT");
   if (e && e[0] == '0') return false;
-  if (c->pstate < 0) {
-    c->pstate = 0;
-    if (persist_prepare(c->L.nx, c->L.ny, c->g.precond, &c->pplan) &&
-        cudaMalloc(&c->pbox, persist_box_bytes(c->pplan)) == cudaSuccess) {
-      c->pstate = 1;
-      c->pepoch = 0;
+  if (p.state < 0) {
+    p.state = 0;
+    if (prepare(c->L.nx, c->L.ny, c->g.precond, &p.plan) &&
+        cudaMalloc(&p.box, persist_box_bytes(p.plan)) == cudaSuccess) {
+      p.state = 1;
+      p.epoch = 0;
     }
     cudaGetLastError();
   }
-  return c->pstate == 1;
+  return p.state == 1;
+}
+
+// the numbers of the next launch's sums; when they start (again), no box holds one
+int next_epoch(tl_ctx* c, tl_ctx::Persist& p, unsigned* epoch) {
+  if (p.epoch == 0 || p.epoch > 0xf0000000u) {
+    CK(cudaMemsetAsync(p.box, 0, persist_box_bytes(p.plan), c->stream));
+    p.epoch = 1;
+  }
+  *epoch = p.epoch;
+  p.epoch += 2 * PERSIST_RUN;
+  return TL_OK;
 }
 
 int run_persistent(tl_ctx* c, const LoopArgs& la) {
-  if (c->pepoch == 0 || c->pepoch > 0xf0000000u) {  // the numbers start (again): no box holds one
-    CK(cudaMemsetAsync(c->pbox, 0, persist_box_bytes(c->pplan), c->stream));
-    c->pepoch = 1;
-  }
+  unsigned epoch;
+  int rc = next_epoch(c, c->pcg, &epoch);
+  if (rc) return rc;
   // TL_CG_BARRIER_EXTRA=1: the grid sums wait for one partial that never comes, so every wait runs
   // out (about a second) and the solve reports TL_ERR_TIMEOUT -- the test of the bounded wait
   const char* ex = getenv("TL_CG_BARRIER_EXTRA");
-  CK(launch_persistent_cg(la, c->pplan, PERSIST_RUN, c->pepoch, c->pbox, c->stream, ex && ex[0] == '1' ? 1 : 0));
-  c->pepoch += 2 * PERSIST_RUN;
+  CK(launch_persistent_cg(la, c->pcg.plan, PERSIST_RUN, epoch, c->pcg.box, c->stream, ex && ex[0] == '1' ? 1 : 0));
+  return TL_OK;
+}
+
+int run_persistent_mix(tl_ctx* c) {
+  unsigned epoch;
+  int rc = next_epoch(c, c->pmix, &epoch);
+  if (rc) return rc;
+  CK(launch_persistent_mix(c->mix, c->L, c->mst, c->pmix.plan, PERSIST_RUN, epoch, c->pmix.box, c->stream));
   return TL_OK;
 }
 
@@ -673,7 +692,8 @@ int tl_destroy(tl_ctx* c) {
   if (c->fe_done) cudaEventDestroy(c->fe_done);
   if (c->up) cudaStreamDestroy(c->up);
   if (c->down) cudaStreamDestroy(c->down);
-  cudaFree(c->pbox);
+  cudaFree(c->pcg.box);
+  cudaFree(c->pmix.box);
   if (c->cg_exec) cudaGraphExecDestroy(c->cg_exec);
   if (c->cg_prof_exec) cudaGraphExecDestroy(c->cg_prof_exec);
   if (c->mix_exec) cudaGraphExecDestroy(c->mix_exec);
@@ -718,7 +738,8 @@ int tl_device_bytes(const tl_ctx* c, unsigned long long* bytes) {
   if (!c || !bytes) return fail(TL_ERR_ARG, "tl_device_bytes: null argument");
   *bytes = c->slab_bytes + sizeof(double) * 4 * MAX_REDUCE_BLOCKS + 256 + sizeof(LoopState) +
            sizeof(double) * 2 * ((size_t)c->hist_cap + c->ch_cap) + c->mix_bytes + (c->tape ? c->tape_bytes : 0) +
-           (c->xfer ? (size_t)tl_ctx::XFER_FIELDS * c->field_stride : 0) + (c->pbox ? persist_box_bytes(c->pplan) : 0);
+           (c->xfer ? (size_t)tl_ctx::XFER_FIELDS * c->field_stride : 0) +
+           (c->pcg.box ? persist_box_bytes(c->pcg.plan) : 0) + (c->pmix.box ? persist_box_bytes(c->pmix.plan) : 0);
   return TL_OK;
 }
 
@@ -1338,7 +1359,9 @@ int mixed_cg(tl_ctx* c, const tl_solve_opts* o, tl_solve_info* info, long long l
     CK(cudaMemcpyAsync(c->mst, &H, sizeof(MixState), cudaMemcpyHostToDevice, c->stream));
     while (H.status == RUN) {
       const int n_before = H.n;
-      if (!c->prof && use_graphs()) {
+      if (use_persistent(c, c->pmix, mix_persist_prepare)) {
+        if ((rc = run_persistent_mix(c))) return rc;
+      } else if (!c->prof && use_graphs()) {
         if ((rc = run_mix_batch(c, rd))) return rc;
       } else {
         for (int i = 0; i < batch; ++i) {
@@ -1363,6 +1386,8 @@ int mixed_cg(tl_ctx* c, const tl_solve_opts* o, tl_solve_info* info, long long l
       }
     }
     if (H.status == EXIT_BREAKDOWN) return fail(TL_ERR_BREAKDOWN, "tl_tea_leaf: non-finite FP32 CG scalar");
+    if (H.status == EXIT_TIMEOUT)
+      return fail(TL_ERR_TIMEOUT, "tl_tea_leaf: a wait of the persistent FP32 CG kernel expired");
     const bool switching = pre && H.status == STOP_SWITCH;
     const bool capped = H.n > H.max_n;
     // trial replacement: true FP64 residual of u + d, u itself untouched
@@ -1786,7 +1811,7 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
       LoopArgs la = c->loop();
       const int n_before = n;
       bool sampled = false;  // the timed graph form: only iteration TIMED_ITER of the batch is timed
-      if (use_persistent(c)) {
+      if (use_persistent(c, c->pcg, persist_prepare)) {
         if (H.u_pending) launch_flush_u(la, c->stream);  // of the batched kernels (none normally)
         if ((rc = run_persistent(c, la))) return rc;
       } else if (!c->prof && use_graphs()) {

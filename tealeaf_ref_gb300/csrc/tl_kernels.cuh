@@ -119,6 +119,7 @@ void launch_flush_u(const LoopArgs& a, cudaStream_t s);
 // ry-th row of its tile
 struct PersistPlan {
   int gx, gy, tw, th, ry, variant, cs;
+  int rows;  // FP32 form: a thread owns this many consecutive rows
 };
 // the plan of a mesh on the current device; false if it does not fit on chip
 bool persist_prepare(int nx, int ny, int precond, PersistPlan* out);
@@ -175,6 +176,12 @@ void launch_mix_iteration(const MixFields& m, const Layout& L, const Reduce& rd,
                           cudaEvent_t between = nullptr);
 // accept the correction: u += d (FP64), d = 0
 void launch_mix_apply(const Fields& f, const MixFields& m, const Layout& L, cudaStream_t s);
+
+// The FP32 steps on chip (tl_persist.cu), for meshes that fit: up to max_run steps of the loop in
+// one launch, as launch_mix_iteration would run them
+bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out);
+cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState* ms, const PersistPlan& p, int max_run,
+                                  unsigned epoch, void* box, cudaStream_t s, int extra = 0);
 
 // ---- FP32 polynomial sweeps of the precision form of Chebyshev / PPCG (tl_mixed_poly.cu) ----
 // PPCG inner loop in FP32 from the FP64 r: inner_steps Chebyshev steps with ch_a/ch_b[1..],

@@ -30,7 +30,7 @@
 #include <cmath>
 #include <vector>
 
-#include "tl_kernels.cuh"
+#include "tl_mixed.cuh"
 
 namespace tl {
 
@@ -38,33 +38,6 @@ namespace {
 
 constexpr int MT = 128;      // threads per CTA
 constexpr int MSW = 4 * MT;  // strip width (four columns per thread)
-
-// ---- error-free transformations (Knuth's TwoSum; TwoProduct with FMA) ----
-struct Dot2 {
-  float s = 0.f, c = 0.f;  // running sum and accumulated error terms
-  __device__ __forceinline__ void add(float a, float b) {
-    const float p = a * b;
-    const float pe = fmaf(a, b, -p);  // a*b = p + pe exactly
-    const float t = s + p;
-    const float z = t - s;
-    const float se = (s - (t - z)) + (p - z);  // s + p = t + se exactly
-    s = t;
-    c += pe + se;
-  }
-  __device__ __forceinline__ double value() const { return (double)s + (double)c; }
-};
-
-__device__ __forceinline__ void mix_finish(MixState* ms) {
-  ms->n += 1;
-  if (ms->switch_rr > 0.0 && ms->n >= ms->presteps && ms->rr <= ms->switch_rr) {
-    ms->status = STOP_SWITCH;
-    return;
-  }
-  // hand over to the host for a residual replacement (the recursive residual fell by delta,
-  // or this phase used up its step budget), or stop at the overall cap
-  if (!(ms->rr > ms->delta2 * ms->rr_max) || ms->n > ms->max_n || ms->n >= ms->phase_end)
-    ms->status = EXIT_CONVERGED;
-}
 
 // Records the norms of a trial residual; the host decides whether to accept the correction.
 // The pending d update was flushed before the trial (k_mix_flush_d), so it is cleared here.

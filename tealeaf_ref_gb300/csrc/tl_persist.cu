@@ -33,10 +33,10 @@
 // Time per CG iteration, the solve's set-up included, against the form before it (up to 640K cells
 // one persistent kernel with the fields in memory and two barriers an iteration, above the batched
 // sweeps of tl_fused.cu in CUDA graphs): 64^2 3.9 against 12 us, 128^2 5.9 / 13.8, 256^2 7.2 / 14.5,
-// 512^2 10.4 / 27.6, 777 x 1013 with jac_diag 24.2 / 43.9, 1000^2 27.4 / 47, 1024^2 27.2 / 42.4.
+// 512^2 10.4 / 27.6, 777 x 1013 with jac_diag 23.7 / 43.9, 1000^2 24.5 / 47, 1024^2 26.0 / 42.4.
 // Every mesh that fits runs here: the largest, 1100^2, is where it gains least.  The FP64 pipe's
 // share is 1.1 us at 256^2 and 17 us at 1000^2.
-#include "tl_kernels.cuh"
+#include "tl_mixed.cuh"
 
 namespace tl {
 
@@ -229,6 +229,7 @@ __device__ __noinline__ double exchange_sum(Exchange* x, ulonglong2* in, unsigne
 template <int M, bool DIAG>
 __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
   constexpr bool PREG = M <= 4, UREG = M <= 6, DISM = M <= 14;
+  constexpr int MG = M < 6 ? M : 6;  // rows whose loads from the fields are in flight together
   __shared__ LoopState S;
   __shared__ Exchange X;
   __shared__ double sh_alpha, sh_beta;
@@ -406,16 +407,28 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       o = fresh(o0);
       c = fresh(c0);
 #pragma unroll
-      for (int i = 0; i < M; ++i, o += ostep, c += cstep) {
-        if (i < mine) {
-          const double pc = PREG ? pr[i] : sp[o];
-          double wv = (DISM ? sdi[o] : __ldg(f.di + c)) * pc;
-          wv = fma(-scy[o + P], sp[o + P], wv);
-          wv = fma(-scy[o], sp[o - P], wv);
-          wv = fma(-scx[o + 1], sp[o + 1], wv);
-          wv = fma(-scx[o], sp[o - 1], wv);
-          w[i] = wv;
-          acc = fma(wv, pc, acc);
+      for (int i0 = 0; i0 < M; i0 += MG) {
+        if (i0 >= mine) break;
+        double di[DISM ? 1 : MG];
+        if (!DISM) {
+#pragma unroll
+          for (int j = 0; j < MG; ++j)
+            if (i0 + j < mine) di[j] = __ldg(f.di + c + j * cstep);
+          c += MG * cstep;
+        }
+#pragma unroll
+        for (int j = 0; j < MG; ++j, o += ostep) {
+          const int i = i0 + j;
+          if (i < M && i < mine) {
+            const double pc = PREG ? pr[i] : sp[o];
+            double wv = (DISM ? sdi[o] : di[DISM ? 0 : j]) * pc;
+            wv = fma(-scy[o + P], sp[o + P], wv);
+            wv = fma(-scy[o], sp[o - P], wv);
+            wv = fma(-scx[o + 1], sp[o + 1], wv);
+            wv = fma(-scx[o], sp[o - 1], wv);
+            w[i] = wv;
+            acc = fma(wv, pc, acc);
+          }
         }
       }
       give(acc);
@@ -442,20 +455,32 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       double acc = 0.0;
       int c = fresh(c0), l = fresh(to_l), e = fresh(to_r);
 #pragma unroll
-      for (int i = 0; i < M; ++i, c += cstep, l += ry, e += ry) {
-        if (i < mine) {
-          const double rv = fma(-alpha, w[i], r[i]);
-          r[i] = rv;
-          double zv = rv;
-          if (DIAG) {
-            zv = (UREG ? mi[i] : __ldg(f.mi + c)) * rv;
-            w[i] = zv;
+      for (int i0 = 0; i0 < M; i0 += MG) {
+        if (i0 >= mine) break;
+        double mg[DIAG && !UREG ? MG : 1];
+        if (DIAG && !UREG) {
+#pragma unroll
+          for (int j = 0; j < MG; ++j)
+            if (i0 + j < mine) mg[j] = __ldg(f.mi + c + j * cstep);
+          c += MG * cstep;
+        }
+#pragma unroll
+        for (int j = 0; j < MG; ++j, l += ry, e += ry) {
+          const int i = i0 + j;
+          if (i < M && i < mine) {
+            const double rv = fma(-alpha, w[i], r[i]);
+            r[i] = rv;
+            double zv = rv;
+            if (DIAG) {
+              zv = (UREG ? mi[UREG ? i : 0] : mg[UREG ? 0 : j]) * rv;
+              w[i] = zv;
+            }
+            if (to_l >= 0) box_put(halo + l, zv, epoch);
+            if (to_r >= 0) box_put(halo + e, zv, epoch);
+            if (i == rim_b) box_put(halo + to_b, zv, epoch);
+            if (i == rim_t) box_put(halo + to_t, zv, epoch);
+            acc = fma(rv, zv, acc);
           }
-          if (to_l >= 0) box_put(halo + l, zv, epoch);
-          if (to_r >= 0) box_put(halo + e, zv, epoch);
-          if (i == rim_b) box_put(halo + to_b, zv, epoch);
-          if (i == rim_t) box_put(halo + to_t, zv, epoch);
-          acc = fma(rv, zv, acc);
         }
       }
       give(acc);
@@ -463,14 +488,26 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       int o = fresh(o0);
       c = fresh(c0);
 #pragma unroll
-      for (int i = 0; i < M; ++i, o += ostep, c += cstep) {
-        if (i < mine) {
-          const double pc = PREG ? pr[i] : sp[o];
-          if (UREG)
-            u[i] = fma(alpha, pc, u[i]);
-          else
-            f.u[c] = fma(alpha, pc, f.u[c]);
+      for (int i0 = 0; i0 < M; i0 += MG) {
+        if (i0 >= mine) break;
+        double ug[UREG ? 1 : MG];
+        if (!UREG) {
+#pragma unroll
+          for (int j = 0; j < MG; ++j)
+            if (i0 + j < mine) ug[j] = f.u[c + j * cstep];
         }
+#pragma unroll
+        for (int j = 0; j < MG; ++j, o += ostep) {
+          const int i = i0 + j;
+          if (i < M && i < mine) {
+            const double pc = PREG ? pr[i] : sp[o];
+            if (UREG)
+              u[UREG ? i : 0] = fma(alpha, pc, u[UREG ? i : 0]);
+            else
+              f.u[c + j * cstep] = fma(alpha, pc, ug[UREG ? 0 : j]);
+          }
+        }
+        c += MG * cstep;
       }
       bool got = false;
       for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
@@ -559,6 +596,451 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       }
     }
     *g.a.rd.st = S;
+  }
+}
+
+// ---- the FP32 process of the precision form (tl_mixed.cu) -------------------------------------
+// The same loop on FP32 vectors: k_mix_w and k_mix_ur with d += alpha p in the wait for beta.  p
+// with its halo and r live in shared memory, w and d in tensor memory (which no tensor core uses
+// here: 128 words a thread); the operator's coefficients stay in the fields, which the L2 cache
+// (and, for small tiles, the SM's own) holds.  8 bytes a cell in shared memory take meshes of up to
+// 4.3 million cells, 2048^2 among them.  A thread owns consecutive rows of a column, so a row's
+// upper face is the next row's lower one; the coefficients of the next group of rows are in flight
+// while one is used.  Time per iteration, the replacements included, against the sweeps' two
+// launches: 512^2 10.3 against 25.0 us, 1000^2 13.4 / 34.0, 1500 x 1999 24.5 / 48.0, 2048^2 32.4 /
+// 50.4, with jac_diag 37.1 / 55.5; with w in registers and d in its field 2048^2 took 46.7 us.  The
+// sums' exchange bounds it up to about 1000^2, the coefficients' way from L2 above.
+// The dot products are the sweeps': Dot2 per thread, then exact integers.
+struct MixPersistArgs {
+  MixFields m;
+  Layout L;
+  MixState* ms;
+  PersistPlan pl;
+  int max_run;
+  unsigned epoch;
+  ulonglong2* box;
+  int extra;
+};
+
+// a float beside the sum's number
+__device__ __forceinline__ void fbox_put(unsigned long long* s, float v, unsigned epoch) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(s), "l"(((unsigned long long)__float_as_uint(v) << 32) | epoch)
+               : "memory");
+}
+__device__ __forceinline__ unsigned long long fbox_get(const unsigned long long* s) {
+  unsigned long long w;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(s) : "memory");
+  return w;
+}
+
+// s + c of every lane, summed over the warp
+__device__ __forceinline__ Fix warp_fix(const Dot2& d) {
+  const unsigned bs = __float_as_uint(d.s), bc = __float_as_uint(d.c);
+  auto ex = [](unsigned b) {
+    const unsigned e = (b >> 23) & 0xffu;
+    return e == 0xffu ? 0x7ffu : max(e, 1u) + 896u;  // biased as a double's
+  };
+  auto fix = [](unsigned b, unsigned ev, unsigned e) {
+    const uint64_t m = (uint64_t)((b & 0x7fffffu) | ((b & 0x7f800000u) ? 0x800000u : 0u)) << 29;
+    const long long i = (long long)((((m << (FSH + 1)) >> min(e - ev, 63u)) + 1ull) >> 1);
+    return (b >> 31) ? -i : i;
+  };
+  const unsigned es = ex(bs), ec = ex(bc);
+  const unsigned e = __reduce_max_sync(0xffffffffu, max(es, ec)) ;
+  return Fix{warp_add((fix(bs, es, e) >> 1) + (fix(bc, ec, e) >> 1)), e == 0x7ffu ? e : e + 1u};
+}
+
+// Tensor memory as the threads' own storage: 512 columns of 128 lanes, of which a warp reaches the
+// 32 lanes of its number modulo 4; the four warps of a quarter take 128 columns each, 2 MROWS words a
+// thread.
+constexpr int MROWS = 64;  // rows a thread may own
+constexpr int MC = 8;      // rows handled together
+__device__ __forceinline__ void tmem_alloc(unsigned* at) {  // a whole warp
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(at))
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free(unsigned a) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(a) : "memory");
+}
+__device__ __forceinline__ void tmem_put(unsigned a, const float (&v)[8]) {
+  __syncwarp();
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(a), "f"(v[0]), "f"(v[1]),
+               "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+// before the words are read again
+__device__ __forceinline__ void tmem_put_done() {
+  __syncwarp();
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_get(unsigned a, float (&v)[8]) {
+  __syncwarp();
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "r"(a)
+               : "memory");
+}
+
+template <bool DIAG>
+__global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g) {
+  __shared__ MixState S;
+  __shared__ Exchange X;
+  __shared__ float sh_alpha, sh_beta;
+  __shared__ int sh_status;
+  __shared__ unsigned sh_tmem;
+  extern __shared__ __align__(16) float fsm[];
+  const Layout L = g.L;
+  const MixFields& f = g.m;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const bool owner = wid != 0;
+  const int to = t - 32;
+  const int ctas = gridDim.x;
+  if (t == 0) {
+    S = *g.ms;
+    sh_status = S.status;
+    sh_beta = (float)S.beta;
+    X.fail = 0;
+  }
+  __syncthreads();
+  if (sh_status != RUN) return;
+  if (wid == 0) tmem_alloc(&sh_tmem);
+
+  const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
+  const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;
+  const int tw = min(g.pl.tw, L.nx - j0), th = min(g.pl.th, L.ny - k0);
+  const int P = g.pl.tw + 2, rows = g.pl.rows;
+  float* const sp = fsm;
+  float* const sr = fsm + (g.pl.th + 2) * P;
+
+  // the thread's column and rows y0 .. y0+mine-1
+  const int tx = owner ? to % g.pl.tw : 0, seg = owner ? to / g.pl.tw : 0, y0 = seg * rows;
+  const int mine = (owner && tx < tw && seg < g.pl.ry) ? max(0, min(rows, th - y0)) : 0;
+  const int o0 = (y0 + 1) * P + tx + 1, r0 = y0 * g.pl.tw + tx;
+  const int c0 = (int)L.at(j0 + tx + 1, k0 + y0 + 1);
+  const int ld = L.ld, rst = g.pl.tw;
+  const bool at_l = tx == 0 && j0 == 0, at_r = tx == tw - 1 && j0 + tw == L.nx;
+  const int i_first = y0 == 0 ? 0 : -1, i_last = (mine > 0 && y0 + mine == th) ? mine - 1 : -1;
+  const int i_b = k0 == 0 ? i_first : -1, i_t = k0 + th == L.ny ? i_last : -1;
+
+  const int hbox = 2 * (g.pl.th + g.pl.tw);
+  unsigned long long* const halo = reinterpret_cast<unsigned long long*>(g.box + (size_t)2 * ctas * SLOTS);
+  int ho[PH], hh[PH];
+  float hp[PH], hs[PH];
+  float* const src = DIAG ? f.z : f.r;
+  int n = S.n;
+  const float* const pold = (n & 1) ? f.p : f.p2;
+  bool upd = S.p_pending != 0;
+#pragma unroll
+  for (int q = 0; q < PH; ++q) {
+    const int h = to + q * PT;
+    ho[q] = -1;
+    hh[q] = 0;
+    hp[q] = hs[q] = 0.f;
+    int x = -1, y = h;
+    bool is = j0 > 0 && y < th;
+    if (h >= g.pl.th) x = tw, y = h - g.pl.th, is = j0 + tw < L.nx && y < th;
+    if (h >= 2 * g.pl.th) x = h - 2 * g.pl.th, y = -1, is = k0 > 0 && x < tw;
+    if (h >= 2 * g.pl.th + g.pl.tw) x = h - 2 * g.pl.th - g.pl.tw, y = th, is = k0 + th < L.ny && x < tw;
+    if (is && owner && h < hbox) {
+      ho[q] = (y + 1) * P + x + 1;
+      hh[q] = (int)blockIdx.x * hbox + h;
+      const int c = (int)L.at(j0 + x + 1, k0 + y + 1);
+      hp[q] = pold[c];
+      if (upd) hs[q] = src[c];
+    }
+  }
+  const int to_l = (mine && tx == 0 && j0 > 0) ? ((int)blockIdx.x - 1) * hbox + g.pl.th + y0 : -1;
+  const int to_r = (mine && tx == tw - 1 && j0 + tw < L.nx) ? ((int)blockIdx.x + 1) * hbox + y0 : -1;
+  const int rim_b = k0 > 0 ? i_first : -1, rim_t = k0 + th < L.ny ? i_last : -1;
+  const int to_b = ((int)blockIdx.x - g.pl.gx) * hbox + 2 * g.pl.th + g.pl.tw + tx;
+  const int to_t = ((int)blockIdx.x + g.pl.gx) * hbox + 2 * g.pl.th + tx;
+
+  __syncthreads();
+  // this thread's words of tensor memory: w (z between phases B and A with DIAG), then d
+  const unsigned tw_ = sh_tmem + ((unsigned)(wid & 3) << 21) + (unsigned)(wid >> 2) * (2 * MROWS), td_ = tw_ + MROWS;
+  const int nch = owner ? (rows + MC - 1) / MC : 0;
+  {
+    int o = o0, rr = r0, c = c0;
+    // the deferred d += alpha p of an earlier step (its p is the one read here)
+    const bool upd_d = S.d_pending != 0;
+    const float da = (float)S.d_alpha;
+    for (int ch = 0; ch < nch; ++ch) {
+      float z[MC], d[MC];
+#pragma unroll
+      for (int j = 0; j < MC; ++j, o += P, rr += rst, c += ld) {
+        z[j] = d[j] = 0.f;
+        if (ch * MC + j < mine) {
+          const float p = pold[c];
+          sp[o] = p;
+          sr[rr] = f.r[c];
+          if (DIAG) z[j] = f.z[c];
+          d[j] = f.d[c];
+          if (upd_d) d[j] = fmaf(da, p, d[j]);
+        }
+      }
+      tmem_put(tw_ + ch * MC, z);
+      tmem_put(td_ + ch * MC, d);
+    }
+    tmem_put_done();
+  }
+
+  double rro = S.rro, rro_prev = S.rro_prev, pw = S.pw, alpha_ = S.alpha, beta_ = S.beta, rr_ = S.rr;
+  unsigned epoch = g.epoch;
+  __syncthreads();
+
+  auto give = [&](const Dot2& v) {
+    const Fix s = warp_fix(v);
+    if (lane == 0) X.part[wid - 1] = s;
+    bar_arrive<1, PTHREADS>();
+  };
+  const int nwait = ctas > 1 ? ctas + g.extra : 0, nq = (nwait + 31) / 32;
+  auto poll = [&] {
+    if (wid > nq) return;
+    const int slot = (wid - 1) * 32 + lane;
+    const ulonglong2* in = g.box + ((size_t)(epoch & 1u) * ctas + blockIdx.x) * SLOTS + slot;
+    ulonglong2 x = make_ulonglong2(0ull, 0ull);
+    bool here = slot >= nwait;
+    for (unsigned tries = 0; !here && tries < PERSIST_POLL_LIMIT; ++tries) {
+      x = box_get(in);
+      here = box_is(x, epoch);
+    }
+    if (!here) X.fail = 1;
+    __syncwarp();
+    const Fix q = warp_fix(slot < nwait ? box_value(x) : 0.0);
+    if (lane == 0) X.inbox[wid - 1] = q;
+    bar_arrive(3, 32 * (nq + 1));
+  };
+  auto inboxes = [&] { return g.box + (size_t)(epoch & 1u) * ctas * SLOTS; };
+  struct Coefs {
+    float di[MC], cl[MC], cr[MC], ct[MC];  // Di, the left, right and upper face of a group of rows
+  } ka, kb;
+  auto load_coefs = [&](int ch, Coefs& k) {
+    int c = c0 + ch * MC * ld;
+#pragma unroll
+    for (int j = 0; j < MC; ++j, c += ld) {
+      k.di[j] = k.cl[j] = k.cr[j] = k.ct[j] = 0.f;
+      if (ch * MC + j < mine) {
+        k.di[j] = __ldg(f.di + c);
+        k.cl[j] = __ldg(f.cx + c);
+        k.cr[j] = __ldg(f.cx + c + 1);
+        k.ct[j] = __ldg(f.cy + c + ld);
+      }
+    }
+  };
+  load_coefs(0, ka);
+
+  bool any = false;
+  for (int done = 0; done < g.max_run; ++done) {
+    // ---- phase A: p_n, w = A p_n, p.w ----
+    if (owner) {
+      const float beta = sh_beta;
+      {
+        int o = o0, rr = r0;
+        for (int ch = 0; ch < nch; ++ch) {
+          float z[MC];
+          if (DIAG) tmem_get(tw_ + ch * MC, z);
+#pragma unroll
+          for (int j = 0; j < MC; ++j, o += P, rr += rst) {
+            const int i = ch * MC + j;
+            if (i < mine) {
+              float p = sp[o];
+              if (upd) p = fmaf(beta, p, DIAG ? z[j] : sr[rr]);
+              sp[o] = p;
+              if (at_l) sp[o - 1] = p;
+              if (at_r) sp[o + 1] = p;
+              if (i == i_b) sp[o - P] = p;
+              if (i == i_t) sp[o + P] = p;
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < PH; ++q)
+        if (ho[q] >= 0) {
+          if (upd) hp[q] = fmaf(beta, hp[q], hs[q]);
+          sp[ho[q]] = hp[q];
+        }
+      bar_sync<2, PT>();
+      Dot2 dot;
+      {
+        int o = o0;
+        float pb = 0.f, pc = 0.f, cyb = 0.f;
+        if (mine > 0) pb = sp[o - P], pc = sp[o], cyb = __ldg(f.cy + c0);
+        auto rows_of = [&](int ch, const Coefs& k) {
+          float w[MC];
+#pragma unroll
+          for (int j = 0; j < MC; ++j, o += P) {
+            w[j] = 0.f;
+            if (ch * MC + j < mine) {
+              const float pt = sp[o + P];
+              float a = k.di[j] * pc;
+              a = fmaf(-k.ct[j], pt, a);
+              a = fmaf(-cyb, pb, a);
+              a = fmaf(-k.cr[j], sp[o + 1], a);
+              a = fmaf(-k.cl[j], sp[o - 1], a);
+              w[j] = a;
+              dot.add(a, pc);
+              pb = pc;
+              pc = pt;
+              cyb = k.ct[j];
+            }
+          }
+          tmem_put(tw_ + ch * MC, w);
+        };
+        // two groups of coefficients: the next one's loads are in flight while one is used
+        for (int ch = 0; ch < nch; ch += 2) {
+          if (ch + 1 < nch) load_coefs(ch + 1, kb);
+          rows_of(ch, ka);
+          if (ch + 1 < nch) {
+            if (ch + 2 < nch) load_coefs(ch + 2, ka);
+            rows_of(ch + 1, kb);
+          }
+        }
+        tmem_put_done();
+      }
+      give(dot);
+      poll();
+    } else {
+      pw = exchange_sum(&X, inboxes(), epoch, ctas, 1, g.extra, rro, nullptr);
+      alpha_ = rro / pw;
+      if (lane == 0) {
+        sh_alpha = (float)alpha_;
+        if (!finite_bits(alpha_)) sh_status = EXIT_BREAKDOWN;
+        if (blockIdx.x == 0 && S.hist_a) S.hist_a[n] = alpha_;
+      }
+    }
+    ++epoch;
+    __syncthreads();
+    if (X.fail || sh_status != RUN) break;
+    // ---- phase B: r -= alpha w, z = Mi r, r.z; the rim to the neighbours; d += alpha p_n ----
+    if (owner) {
+      const float alpha = sh_alpha;
+      Dot2 dot;
+      {
+        int rr = r0, c = c0;
+        for (int ch = 0; ch < nch; ++ch) {
+          float w[MC], mi[MC];
+          if (DIAG) {
+#pragma unroll
+            for (int j = 0; j < MC; ++j, c += ld)
+              mi[j] = ch * MC + j < mine ? __ldg(f.mi + c) : 0.f;
+          }
+          tmem_get(tw_ + ch * MC, w);
+#pragma unroll
+          for (int j = 0; j < MC; ++j, rr += rst) {
+            const int i = ch * MC + j;
+            if (i < mine) {
+              const float rv = fmaf(-alpha, w[j], sr[rr]);
+              sr[rr] = rv;
+              float zv = rv;
+              if (DIAG) {
+                zv = mi[j] * rv;
+                w[j] = zv;
+              }
+              dot.add(rv, zv);
+              if (to_l >= 0) fbox_put(halo + to_l + i, zv, epoch);
+              if (to_r >= 0) fbox_put(halo + to_r + i, zv, epoch);
+              if (i == rim_b) fbox_put(halo + to_b, zv, epoch);
+              if (i == rim_t) fbox_put(halo + to_t, zv, epoch);
+            }
+          }
+          if (DIAG) tmem_put(tw_ + ch * MC, w);
+        }
+      }
+      give(dot);
+      load_coefs(0, ka);  // of the next phase A
+      poll();
+      {
+        int o = o0;
+        for (int ch = 0; ch < nch; ++ch) {
+          float d[MC];
+          tmem_get(td_ + ch * MC, d);
+#pragma unroll
+          for (int j = 0; j < MC; ++j, o += P)
+            if (ch * MC + j < mine) d[j] = fmaf(alpha, sp[o], d[j]);
+          tmem_put(td_ + ch * MC, d);
+        }
+        tmem_put_done();
+      }
+      bool got = false;
+      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+        got = true;
+#pragma unroll
+        for (int q = 0; q < PH; ++q)
+          if (ho[q] >= 0) {
+            const unsigned long long x = fbox_get(halo + hh[q]);
+            got = got && (unsigned)x == epoch;
+            hs[q] = __uint_as_float((unsigned)(x >> 32));
+          }
+      }
+      if (!got) X.fail = 1;
+    } else {
+      rr_ = exchange_sum(&X, inboxes(), epoch, ctas, 1, g.extra, rro, nullptr);
+      beta_ = rr_ / rro;
+      if (lane == 0) {
+        sh_beta = (float)beta_;
+        if (blockIdx.x == 0 && S.hist_b) S.hist_b[n] = beta_;
+        if (!finite_bits(beta_)) {
+          sh_status = EXIT_BREAKDOWN;
+          S.n = n;
+        } else {
+          S.n = n;
+          S.rr = rr_;
+          mix_finish(&S);
+          sh_status = S.status;
+        }
+      }
+      rro_prev = rro;
+      rro = rr_;
+    }
+    ++epoch;
+    ++n;
+    upd = true;
+    any = true;
+    __syncthreads();
+    if (X.fail || sh_status != RUN) break;
+  }
+  const bool failed = X.fail != 0;
+  // p in the buffer the next step reads, r (and z), d
+  float* const pout = ((n - 1) & 1) ? f.p2 : f.p;
+  {
+    int o = o0, rr = r0, c = c0;
+    for (int ch = 0; ch < (failed ? 0 : nch); ++ch) {
+      float z[MC], d[MC];
+      if (DIAG) tmem_get(tw_ + ch * MC, z);
+      tmem_get(td_ + ch * MC, d);
+#pragma unroll
+      for (int j = 0; j < MC; ++j, o += P, rr += rst, c += ld) {
+        if (ch * MC + j < mine) {
+          pout[c] = sp[o];
+          f.r[c] = sr[rr];
+          if (DIAG && any) f.z[c] = z[j];
+          f.d[c] = d[j];
+        }
+      }
+    }
+  }
+  __syncthreads();  // every warp is done with tensor memory
+  if (wid == 0) tmem_free(sh_tmem);
+  if (failed) {
+    if (t == 0) g.ms->status = EXIT_TIMEOUT;
+    return;
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    S.status = sh_status;
+    S.pw = pw;
+    S.alpha = alpha_;
+    S.d_pending = 0;
+    if (any) {
+      S.rr = rr_;
+      S.beta = beta_;
+      S.rro = rro;
+      S.rro_prev = rro_prev;
+      S.p_pending = 1;
+    }
+    *g.ms = S;
   }
 }
 
@@ -683,6 +1165,69 @@ cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int ma
   PersistLaunch l(persist_ctas(p), p.cs, plan_smem(p), s);
   ++launch_counter();
   return cudaLaunchKernelExC(&l.cfg, (const void*)kVariants[p.variant].k[a.precond == 2 ? 1 : 0], args);
+}
+
+namespace {
+
+using MixPersistKernel = void (*)(MixPersistArgs);
+const MixPersistKernel kMixKernels[2] = {k_persistent_mix<false>, k_persistent_mix<true>};  // without / with jac_diag
+size_t mix_plan_smem(const PersistPlan& p) {
+  return ((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw) * sizeof(float);
+}
+
+// The tiling with the fewest cycles an iteration (16 a row of a warp, 3200 for each of the two
+// sums' exchange when there is more than one tile); tiles at least 32 columns wide, where
+// the mesh is, for the sake of the coefficients' loads.
+bool mix_plan(int nx, int ny, int ctas, PersistPlan* out) {
+  double best = 0.0;
+  bool found = false;
+  if (ctas > PERSIST_MAX_CTAS) ctas = PERSIST_MAX_CTAS;
+  for (int g0 = 1; g0 <= ctas && g0 <= nx; ++g0) {
+    const int tw = (nx + g0 - 1) / g0;
+    if (tw > PT || (tw < 32 && g0 > 1)) continue;
+    PersistPlan p;
+    p.cs = 1;
+    p.tw = tw;
+    p.gx = (nx + tw - 1) / tw;
+    for (int many = 0; many < 2; ++many) {
+      int gy = many ? ctas / p.gx : 1;
+      if (gy > ny) gy = ny;
+      if (gy < 1) continue;
+      p.th = (ny + gy - 1) / gy;
+      p.gy = (ny + p.th - 1) / p.th;
+      p.ry = PT / tw < p.th ? PT / tw : p.th;
+      p.rows = (p.th + p.ry - 1) / p.ry;
+      p.variant = 0;
+      const int halo = 2 * (p.tw + p.th);
+      if (p.rows > MROWS || halo > PH * PT || mix_plan_smem(p) > PERSIST_SMEM_MAX) continue;
+      const double cost =
+          (double)((p.ry * tw + 31) / 32) * p.rows * 16.0 + 0.5 * halo + (p.gx * p.gy > 1 ? 6400.0 : 0.0);
+      if (!found || cost < best) {
+        best = cost;
+        *out = p;
+        found = true;
+      }
+    }
+  }
+  return found;
+}
+
+}  // namespace
+
+bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
+  const int diag = precond == 2 ? 1 : 0;
+  const int ctas = persist_clusters((const void*)kMixKernels[diag], 1, PERSIST_SMEM_MAX);
+  if (!mix_plan(nx, ny, ctas, out)) return false;
+  return persist_clusters((const void*)kMixKernels[diag], 1, mix_plan_smem(*out)) >= persist_ctas(*out);
+}
+
+cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState* ms, const PersistPlan& p, int max_run,
+                                  unsigned epoch, void* box, cudaStream_t s, int extra) {
+  MixPersistArgs g{m, L, ms, p, max_run, epoch, static_cast<ulonglong2*>(box), extra};
+  void* args[] = {&g};
+  PersistLaunch l(persist_ctas(p), p.cs, mix_plan_smem(p), s);
+  ++launch_counter();
+  return cudaLaunchKernelExC(&l.cfg, (const void*)kMixKernels[m.mi ? 1 : 0], args);
 }
 
 }  // namespace tl
