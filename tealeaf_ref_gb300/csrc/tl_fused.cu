@@ -661,6 +661,134 @@ __global__ void __launch_bounds__(FT, 7) k_cheby_iter_ws(Fields f, Layout L, con
   cp_wait<0>();
 }
 
+// ---- the five-point operator as one staged sweep ----------------------------------------------
+// The drop-in kernels that apply A to a field and leave the result, with the ring and the staging of
+// k_cheby_iter_ws: unit m holds v of row m (with the columns left and right of the thread's two), cy
+// of row m, and cx (with cx(j+2)), Di and u0 of row m-1; Di v runs on the integer pipes.  Per cell the
+// arithmetic of apply_A (tl_kernels.cu), so its bits.
+//   AP_W    w = A v, p.w                      (tea_leaf_cg_calc_w_kernel, v = p)
+//   AP_R    r = u0 - A v                      (tea_leaf_calc_residual_kernel, v = u)
+//   AP_RN   the same with r.r
+//   (w and r together, the first half of a Chebyshev iteration, gains nothing this way.)
+// Bound by the FP64 pipe (4 operations a cell, 1 for the sum or the difference; Di v is on the
+// integer pipes): at 8192^2 a call of AP_W takes 605 us against the 726 of one cell per thread with
+// direct loads, AP_R 610 against 706.
+constexpr int ASLOT = 5 * SROW + 3 * FT;
+constexpr size_t APPLY_SMEM = (size_t)2 * ASLOT * sizeof(double);
+template <int MODE>
+struct EpiApply {
+  LoopState* st;
+  int mode;
+  __device__ void operator()(double (&acc)[1]) const {
+    if (mode == RED_INIT_RESIDUAL) {
+      st->old_error = acc[0];
+      st->initial_residual = sqrt(fabs(acc[0]));
+    }
+    st->red[0] = acc[0];
+  }
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(FT, 7) k_apply_ws(Fields f, Layout L, Reduce rd, int mode, int rows_per_cta) {
+  extern __shared__ __align__(16) double aring[];
+  enum { B_V = 0, B_CY, B_CX, B_DI, B_U0 };
+  constexpr bool RES = MODE != AP_W;
+  auto arr = [&](int m, int a_) { return aring + (m & 1) * ASLOT + a_ * SROW; };
+  auto own = [&](int m, int e) { return aring + (m & 1) * ASLOT + 5 * SROW + e * FT + threadIdx.x; };
+  const double* __restrict__ v = RES ? f.u : f.p;
+  const double* __restrict__ u0 = f.u0;
+  const double* __restrict__ cx = f.cx;
+  const double* __restrict__ cy = f.cy;
+  const double* __restrict__ di = f.di;
+  double* __restrict__ w = f.w;
+  double* __restrict__ r = f.r;
+  const int t = threadIdx.x;
+  const int ja = blockIdx.x * SW + 1 + 2 * t;
+  const int o = 2 * t + 2;
+  const bool active = ja <= L.nx, has_b = ja + 1 <= L.nx;
+  const int k0 = blockIdx.y * rows_per_cta + 1;
+  const int k1 = min(k0 + rows_per_cta - 1, L.ny);
+  const int ld = L.ld;
+
+  auto stage = [&](int m) {
+    if (m <= k1 + 1 && active) {
+      const long long c = L.at(ja, m);  // row m: up to ny + 1, the halo row
+      cp16(arr(m, B_V) + o, v + c);
+      cp8(own(m, 0), v + c - 1);
+      if (has_b) cp8(own(m, 1), v + c + 2);
+      const long long c0 = c - ld;  // row m - 1
+      cp16(arr(m, B_CY) + o, cy + c);
+      cp16(arr(m, B_CX) + o, cx + c0);
+      if (has_b) cp8(own(m, 2), cx + c0 + 2);
+      cp16(arr(m, B_DI) + o, di + c0);
+      if (RES) cp16(arr(m, B_U0) + o, u0 + c0);
+    }
+    cp_commit();
+  };
+
+  double acc[1] = {0.0}, acc_b = 0.0;
+  double2 vm = make_double2(0.0, 0.0), vc = vm, vn = vm, cyc = vm;
+  double nl = 0.0, nr = 0.0;
+  if (active) {
+    const long long c = L.at(ja, k0);
+    vc = *reinterpret_cast<const double2*>(v + c);
+    vm = *reinterpret_cast<const double2*>(v + c - ld);
+    cyc = *reinterpret_cast<const double2*>(cy + c);
+    nl = v[c - 1];
+    if (has_b) nr = v[c + 2];
+  }
+  stage(k0 + 1);
+  for (int k = k0; k <= k1; ++k) {
+    stage(k + 2);
+    cp_wait<1>();  // unit k+1 has landed
+    const int m = k + 1;
+    if (active) {
+      vn = *reinterpret_cast<const double2*>(arr(m, B_V) + o);
+      const double nl_n = *own(m, 0), nr_n = has_b ? *own(m, 1) : 0.0;
+      const long long c = L.at(ja, k);
+      const double2 cyn = *reinterpret_cast<const double2*>(arr(m, B_CY) + o);
+      const double2 cxa = *reinterpret_cast<const double2*>(arr(m, B_CX) + o);
+      const double2 dd = *reinterpret_cast<const double2*>(arr(m, B_DI) + o);
+      double2 b = make_double2(0.0, 0.0);
+      if (RES) b = *reinterpret_cast<const double2*>(arr(m, B_U0) + o);
+      double wa = dmul_int(dd.x, vc.x);
+      wa = fma(-cyn.x, vn.x, wa);
+      wa = fma(-cyc.x, vm.x, wa);
+      wa = fma(-cxa.y, vc.y, wa);
+      wa = fma(-cxa.x, nl, wa);
+      const double ra = RES ? b.x - wa : 0.0;
+      if (MODE == AP_W) acc[0] = fma(wa, vc.x, acc[0]);
+      if (MODE == AP_RN) acc[0] = fma(ra, ra, acc[0]);
+      if (has_b) {
+        double wb = dmul_int(dd.y, vc.y);
+        wb = fma(-cyn.y, vn.y, wb);
+        wb = fma(-cyc.y, vm.y, wb);
+        wb = fma(-*own(m, 2), nr, wb);
+        wb = fma(-cxa.y, vc.x, wb);
+        const double rb = RES ? b.y - wb : 0.0;
+        if (MODE == AP_W) acc_b = fma(wb, vc.y, acc_b);
+        if (MODE == AP_RN) acc_b = fma(rb, rb, acc_b);
+        if (MODE == AP_W) *reinterpret_cast<double2*>(w + c) = make_double2(wa, wb);
+        if (RES) *reinterpret_cast<double2*>(r + c) = make_double2(ra, rb);
+      } else {
+        if (MODE == AP_W) w[c] = wa;
+        if (RES) r[c] = ra;
+      }
+      cyc = cyn;
+      vm = vc;
+      vc = vn;
+      nl = nl_n;
+      nr = nr_n;
+    }
+  }
+  cp_wait<0>();
+  if (MODE == AP_W || MODE == AP_RN) {
+    acc[0] += acc_b;
+    __syncthreads();  // every thread is done with the ring: it becomes the block sum's scratch
+    grid_reduce_in<1>(acc, rd, EpiApply<MODE>{rd.st, mode}, aring);
+  }
+}
+
 // Applies a pending deferred u update (LoopState::u_pending) when the CG loop stops.
 __global__ void __launch_bounds__(FT) k_flush_u(LoopArgs a) {
   const LoopState* st = a.rd.st;
@@ -1018,6 +1146,27 @@ void launch_fused_jacobi(const LoopArgs& a, const double* un, double* u_out, cud
     case 0x7f: k_fused_jacobi<0x7f><<<grid, 256, 0, s>>>(a.f, a.L, a.rd, un, u_out, a.rx, a.ry); break;
     case 0x40: k_fused_jacobi<0x40><<<grid, 256, 0, s>>>(a.f, a.L, a.rd, un, u_out, a.rx, a.ry); break;
     default: k_fused_jacobi<0><<<grid, 256, 0, s>>>(a.f, a.L, a.rd, un, u_out, a.rx, a.ry); break;
+  }
+}
+
+namespace {
+template <int MODE>
+void launch_apply_mode(const Fields& f, const Layout& L, const Reduce& rd, int mode, cudaStream_t s) {
+  static const long long slots = resident_ctas((const void*)k_apply_ws<MODE>, FT, APPLY_SMEM);
+  const int ns = strips(L);
+  int rows = wave_rows(L.ny, ns, slots);
+  const int min_rows = (int)(((long long)L.ny * ns + MAX_REDUCE_BLOCKS - 1) / MAX_REDUCE_BLOCKS);
+  if (rows < min_rows) rows = min_rows;
+  ++launch_counter();
+  k_apply_ws<MODE><<<dim3(ns, (L.ny + rows - 1) / rows), FT, APPLY_SMEM, s>>>(f, L, rd, mode, rows);
+}
+}  // namespace
+
+void launch_apply(int what, const Fields& f, const Layout& L, const Reduce& rd, int mode, cudaStream_t s) {
+  switch (what) {
+    case AP_W: launch_apply_mode<AP_W>(f, L, rd, mode, s); break;
+    case AP_R: launch_apply_mode<AP_R>(f, L, rd, mode, s); break;
+    default: launch_apply_mode<AP_RN>(f, L, rd, mode, s); break;
   }
 }
 

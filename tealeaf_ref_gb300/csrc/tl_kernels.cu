@@ -38,6 +38,17 @@ inline dim3 row_grid(const Layout& L, bool reducing) {
   return dim3(gx, gy);
 }
 
+// two columns a thread: a reducing kernel on 27 CTAs per SM striding over rows.  The u, r update with
+// its sum took 86, 148 and 529 us at 3001 x 1999 (jac_diag), 4096^2 and 8192^2, against 89, 163 and 582
+// with 6 per SM, 86, 156 and 553 with 16, and 99, 149 and 507 with 54 (more partials to sum).
+inline dim3 pair_grid(const Layout& L, bool reducing) {
+  const int gx = (L.nx + 2 * TB - 1) / (2 * TB);
+  int gy = reducing ? (27 * sm_count() + gx - 1) / gx : L.ny;
+  if (gy > L.ny) gy = L.ny;
+  if (gy > 65535) gy = 65535;
+  return dim3(gx, gy);
+}
+
 #define FOR_ROWS(L)                                                   \
   const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;             \
   for (int k = blockIdx.y + 1; k <= (L).ny; k += gridDim.y)
@@ -525,33 +536,64 @@ __global__ void k_cg_calc_w(Fields f, Layout L, Reduce rd) {
   grid_reduce<1>(v, rd, EpiMode<1>{rd.st, RED_STORE});
 }
 
+// The drop-in CG updates, two columns a thread (16-byte accesses; interior rows start on 128 bytes):
+// bound by HBM, 40 to 64 bytes a cell.
 // tea_leaf_cg_calc_ur_kernel (cg_kernel.f90:198-304) for none / jac_diag; for jac_block the
 // u/r update runs here (MODE 2) and z and r.z come from k_block_solve + k_dot.
 template <int MODE>
-__global__ void k_cg_calc_ur(Fields f, Layout L, double alpha, Reduce rd) {
+__global__ void __launch_bounds__(TB) k_cg_calc_ur(Fields f, Layout L, double alpha, Reduce rd) {
   double v[1] = {0.0};
-  FOR_ROWS(L) {
-    if (j > L.nx) continue;
-    const long long c = L.at(j, k);
-    f.u[c] = fma(alpha, f.p[c], f.u[c]);
-    const double r = fma(-alpha, f.w[c], f.r[c]);
-    f.r[c] = r;
-    if (MODE == 0) v[0] = fma(r, r, v[0]);
-    if (MODE == 1) {
-      const double z = f.mi[c] * r;
-      f.z[c] = z;
-      v[0] = fma(r, z, v[0]);
+  const int j = 2 * (blockIdx.x * TB + threadIdx.x) + 1;
+  if (j <= L.nx) {
+    const bool two = j < L.nx;
+    for (int k = blockIdx.y + 1; k <= L.ny; k += gridDim.y) {
+      const long long c = L.at(j, k);
+      const double2 p = *reinterpret_cast<const double2*>(f.p + c);
+      const double2 w = *reinterpret_cast<const double2*>(f.w + c);
+      double2 u = *reinterpret_cast<const double2*>(f.u + c);
+      double2 r = *reinterpret_cast<const double2*>(f.r + c);
+      u.x = fma(alpha, p.x, u.x);
+      u.y = fma(alpha, p.y, u.y);
+      r.x = fma(-alpha, w.x, r.x);
+      r.y = fma(-alpha, w.y, r.y);
+      double2 z = r;
+      if (MODE == 1) {
+        const double2 mi = *reinterpret_cast<const double2*>(f.mi + c);
+        z.x = mi.x * r.x;
+        z.y = mi.y * r.y;
+      }
+      if (two) {
+        *reinterpret_cast<double2*>(f.u + c) = u;
+        *reinterpret_cast<double2*>(f.r + c) = r;
+        if (MODE == 1) *reinterpret_cast<double2*>(f.z + c) = z;
+      } else {
+        f.u[c] = u.x;
+        f.r[c] = r.x;
+        if (MODE == 1) f.z[c] = z.x;
+      }
+      if (MODE != 2) {
+        v[0] = fma(r.x, z.x, v[0]);
+        if (two) v[0] = fma(r.y, z.y, v[0]);
+      }
     }
   }
   if (MODE != 2) grid_reduce<1>(v, rd, EpiMode<1>{rd.st, RED_STORE});
 }
 
 // tea_leaf_cg_calc_p_kernel (cg_kernel.f90:306-347)
-__global__ void k_cg_calc_p(Fields f, Layout L, double beta, int use_z) {
-  FOR_ROWS(L) {
-    if (j > L.nx) continue;
+__global__ void __launch_bounds__(TB) k_cg_calc_p(Fields f, Layout L, double beta, const double* __restrict__ src) {
+  const int j = 2 * (blockIdx.x * TB + threadIdx.x) + 1;
+  if (j > L.nx) return;
+  for (int k = blockIdx.y + 1; k <= L.ny; k += gridDim.y) {
     const long long c = L.at(j, k);
-    f.p[c] = fma(beta, f.p[c], use_z ? f.z[c] : f.r[c]);
+    double2 p = *reinterpret_cast<const double2*>(f.p + c);
+    const double2 s = *reinterpret_cast<const double2*>(src + c);
+    p.x = fma(beta, p.x, s.x);
+    p.y = fma(beta, p.y, s.y);
+    if (j < L.nx)
+      *reinterpret_cast<double2*>(f.p + c) = p;
+    else
+      f.p[c] = p.x;
   }
 }
 
@@ -565,7 +607,7 @@ __global__ void k_cheby_wr(Fields f, Layout L) {
     f.r[c] = f.u0[c] - w;
   }
 }
-// phase 2 (init): p = (r|z)/theta, u += p
+// tea_leaf_kernel_cheby_init (cheby_kernel.f90:30-109) after w and r: p = (r|z)/theta, u += p
 __global__ void k_cheby_init_pu(Fields f, Layout L, double theta, int use_z) {
   FOR_ROWS(L) {
     if (j > L.nx) continue;
@@ -726,11 +768,32 @@ void launch_copy_interior(double* dst, const double* src, const Layout& L, cudaS
 void launch_copy_all(double* dst, const double* src, const Layout& L, cudaStream_t s) {
   cudaMemcpyAsync(dst, src, (size_t)L.elems() * sizeof(double), cudaMemcpyDeviceToDevice, s);
 }
+// Below this many cells one cell per thread; above it the staged sweep (launch_apply, tl_fused.cu),
+// whose CTAs march over at least eight rows: w = A p with its sum and the call's 15 us took 35.1
+// against 36.0 us at 1000^2 and 89.9 against 77.1 at 3001 x 1999, the residual 20.5 against 23.4 and
+// 73.8 against 69.3.
+constexpr long long APPLY_STAGED_MIN_CELLS = 2LL << 20;
+inline bool apply_staged(const Layout& L) { return (long long)L.nx * L.ny >= APPLY_STAGED_MIN_CELLS; }
+
 void launch_residual(const Fields& f, const Layout& L, const Reduce* rd, int mode, cudaStream_t s) {
+  if (apply_staged(L)) {
+    launch_apply(rd ? AP_RN : AP_R, f, L, rd ? *rd : Reduce{}, mode, s);
+    return;
+  }
   if (rd)
     { ++launch_counter(); k_residual<true><<<row_grid(L, true), TB, 0, s>>>(f, L, *rd, mode); }
   else
     { ++launch_counter(); k_residual<false><<<row_grid(L, false), TB, 0, s>>>(f, L, Reduce{}, mode); }
+}
+void launch_cg_calc_w(const Fields& f, const Layout& L, const Reduce& rd, cudaStream_t s) {
+  if (apply_staged(L)) {
+    launch_apply(AP_W, f, L, rd, RED_STORE, s);
+    return;
+  }
+  { ++launch_counter(); k_cg_calc_w<<<row_grid(L, true), TB, 0, s>>>(f, L, rd); }
+}
+void launch_cheby_wr(const Fields& f, const Layout& L, cudaStream_t s) {
+  { ++launch_counter(); k_cheby_wr<<<row_grid(L, false), TB, 0, s>>>(f, L); }
 }
 void launch_norm2(const double* a, const Layout& L, const Reduce& rd, int mode, cudaStream_t s) {
   { ++launch_counter(); k_norm2<<<row_grid(L, true), TB, 0, s>>>(a, L, rd, mode); }
@@ -766,34 +829,28 @@ void launch_cg_init(const Fields& f, const Layout& L, const Geometry& g, const R
   if (g.precond != 1) launch_precond(f, L, g, f.r, f.z, s);
   { ++launch_counter(); k_cg_init<<<row_grid(L, true), TB, 0, s>>>(f, L, g.precond, rd, mode); }
 }
-void launch_cg_calc_w(const Fields& f, const Layout& L, const Reduce& rd, cudaStream_t s) {
-  { ++launch_counter(); k_cg_calc_w<<<row_grid(L, true), TB, 0, s>>>(f, L, rd); }
-}
 void launch_cg_calc_ur(const Fields& f, const Layout& L, const Geometry& g, double alpha, const Reduce& rd,
                        cudaStream_t s) {
   if (g.precond == 3) {
-    { ++launch_counter(); k_cg_calc_ur<2><<<row_grid(L, true), TB, 0, s>>>(f, L, alpha, rd); }
+    { ++launch_counter(); k_cg_calc_ur<2><<<pair_grid(L, false), TB, 0, s>>>(f, L, alpha, rd); }
     launch_precond(f, L, g, f.r, f.z, s);
     launch_dot(f.r, f.z, nullptr, L, rd, RED_STORE, s);
   } else if (g.precond == 2) {
-    { ++launch_counter(); k_cg_calc_ur<1><<<row_grid(L, true), TB, 0, s>>>(f, L, alpha, rd); }
+    { ++launch_counter(); k_cg_calc_ur<1><<<pair_grid(L, true), TB, 0, s>>>(f, L, alpha, rd); }
   } else {
-    { ++launch_counter(); k_cg_calc_ur<0><<<row_grid(L, true), TB, 0, s>>>(f, L, alpha, rd); }
+    { ++launch_counter(); k_cg_calc_ur<0><<<pair_grid(L, true), TB, 0, s>>>(f, L, alpha, rd); }
   }
 }
 void launch_cg_calc_p(const Fields& f, const Layout& L, double beta, bool use_z, cudaStream_t s) {
-  { ++launch_counter(); k_cg_calc_p<<<row_grid(L, false), TB, 0, s>>>(f, L, beta, use_z ? 1 : 0); }
+  { ++launch_counter(); k_cg_calc_p<<<pair_grid(L, false), TB, 0, s>>>(f, L, beta, use_z ? f.z : f.r); }
 }
 void launch_cheby_init(const Fields& f, const Layout& L, const Geometry& g, double theta, cudaStream_t s) {
-  { ++launch_counter(); k_cheby_wr<<<row_grid(L, false), TB, 0, s>>>(f, L); }
+  launch_cheby_wr(f, L, s);
   if (g.precond != 1) launch_precond(f, L, g, f.r, f.z, s);
   { ++launch_counter(); k_cheby_init_pu<<<row_grid(L, false), TB, 0, s>>>(f, L, theta, g.precond != 1); }
 }
-void launch_cheby_wr(const Fields& f, const Layout& L, cudaStream_t s) {
-  { ++launch_counter(); k_cheby_wr<<<row_grid(L, false), TB, 0, s>>>(f, L); }
-}
 void launch_cheby_iterate(const Fields& f, const Layout& L, const Geometry& g, double a, double b, cudaStream_t s) {
-  { ++launch_counter(); k_cheby_wr<<<row_grid(L, false), TB, 0, s>>>(f, L); }
+  launch_cheby_wr(f, L, s);
   if (g.precond != 1) launch_precond(f, L, g, f.r, f.z, s);
   { ++launch_counter(); k_cheby_iter_pu<<<row_grid(L, false), TB, 0, s>>>(f, L, a, b, g.precond != 1); }
 }

@@ -84,6 +84,10 @@ void launch_dot(const double* a, const double* b, const double* bminus /*nullabl
                 const Reduce& rd, int mode, cudaStream_t s);
 void launch_jacobi(const Fields& f, const Layout& L, const Geometry& g, const Reduce& rd, cudaStream_t s);
 
+// the five-point operator as one staged sweep (tl_fused.cu), for the launchers above on large meshes
+enum { AP_W = 0, AP_R, AP_RN };  // w = A p, p.w | r = u0 - A u | and r.r
+void launch_apply(int what, const Fields& f, const Layout& L, const Reduce& rd, int mode, cudaStream_t s);
+
 // ---- fused solver loop (device-resident scalars) ------------------------
 struct LoopArgs {
   Fields f;
