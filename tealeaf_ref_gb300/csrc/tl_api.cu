@@ -100,13 +100,14 @@ struct tl_ctx {
   cudaGraphExec_t cg_prof_exec = nullptr;
   LoopArgs cg_prof_key{};
   long long cg_prof_nk = 0;
-  // the persistent on-chip loops: FP64 CG, and the FP32 process of the precision form
+  // the persistent on-chip loops: FP64 CG, the FP32 process of the precision form, the FP64
+  // polynomial steps
   struct Persist {
     int state = -1;  // -1 not yet planned, 0 the mesh does not fit, 1 plan holds
     PersistPlan plan{};
     void* box = nullptr;  // what its CTAs exchange partial sums and rims in
     unsigned epoch = 0;   // number of the next sum
-  } pcg, pmix;
+  } pcg, pmix, ppoly;
   // host transfers: an upload and a download stream (tl_stage_state, tl_fetch_field) and
   // XFER_FIELDS staging fields -- two staged (density, energy1) pairs, the fetch snapshot, and
   // two for the synchronous uploads / downloads.  A host array moves as one contiguous copy
@@ -373,13 +374,13 @@ bool use_persistent(tl_ctx* c, tl_ctx::Persist& p, F&& prepare) {
 }
 
 // the numbers of the next launch's sums; when they start (again), no box holds one
-int next_epoch(tl_ctx* c, tl_ctx::Persist& p, unsigned* epoch) {
+int next_epoch(tl_ctx* c, tl_ctx::Persist& p, unsigned* epoch, unsigned sums = 2 * PERSIST_RUN) {
   if (p.epoch == 0 || p.epoch > 0xf0000000u) {
     CK(cudaMemsetAsync(p.box, 0, persist_box_bytes(p.plan), c->stream));
     p.epoch = 1;
   }
   *epoch = p.epoch;
-  p.epoch += 2 * PERSIST_RUN;
+  p.epoch += sums;
   return TL_OK;
 }
 
@@ -391,6 +392,24 @@ int run_persistent(tl_ctx* c, const LoopArgs& la) {
   // out (about a second) and the solve reports TL_ERR_TIMEOUT -- the test of the bounded wait
   const char* ex = getenv("TL_CG_BARRIER_EXTRA");
   CK(launch_persistent_cg(la, c->pcg.plan, PERSIST_RUN, epoch, c->pcg.box, c->stream, ex && ex[0] == '1' ? 1 : 0));
+  return TL_OK;
+}
+
+// The FP64 polynomial steps on chip; TL_POLY_PERSISTENT=0 forces them off.
+bool use_persistent_poly(tl_ctx* c) {
+  const char* e = getenv("TL_POLY_PERSISTENT");
+  return !c->g.reflective && !(e && e[0] == '0') && use_persistent(c, c->ppoly, poly_persist_prepare);
+}
+
+// steps first .. first + steps - 1 (from 1) of the coefficients on the device
+int run_persistent_poly(tl_ctx* c, bool ppcg, const double* u_in, int first, int steps) {
+  unsigned epoch;
+  int rc = next_epoch(c, c->ppoly, &epoch, steps);
+  if (rc) return rc;
+  const char* ex = getenv("TL_CG_BARRIER_EXTRA");  // 2: one tile sends no rims, so its neighbours' waits run out
+  CK(launch_persistent_poly(c->f, c->L, c->ppoly.plan, ppcg, c->g.precond == TL_PREC_JAC_DIAG, u_in, c->ch_a + first,
+                            c->ch_b + first, steps, epoch, c->ppoly.box, c->counter + MIX_ERR_WORD,
+                            ex && ex[0] == '2', c->stream));
   return TL_OK;
 }
 
@@ -694,6 +713,7 @@ int tl_destroy(tl_ctx* c) {
   if (c->down) cudaStreamDestroy(c->down);
   cudaFree(c->pcg.box);
   cudaFree(c->pmix.box);
+  cudaFree(c->ppoly.box);
   if (c->cg_exec) cudaGraphExecDestroy(c->cg_exec);
   if (c->cg_prof_exec) cudaGraphExecDestroy(c->cg_prof_exec);
   if (c->mix_exec) cudaGraphExecDestroy(c->mix_exec);
@@ -739,7 +759,8 @@ int tl_device_bytes(const tl_ctx* c, unsigned long long* bytes) {
   *bytes = c->slab_bytes + sizeof(double) * 4 * MAX_REDUCE_BLOCKS + 256 + sizeof(LoopState) +
            sizeof(double) * 2 * ((size_t)c->hist_cap + c->ch_cap) + c->mix_bytes + (c->tape ? c->tape_bytes : 0) +
            (c->xfer ? (size_t)tl_ctx::XFER_FIELDS * c->field_stride : 0) +
-           (c->pcg.box ? persist_box_bytes(c->pcg.plan) : 0) + (c->pmix.box ? persist_box_bytes(c->pmix.plan) : 0);
+           (c->pcg.box ? persist_box_bytes(c->pcg.plan) : 0) + (c->pmix.box ? persist_box_bytes(c->pmix.plan) : 0) +
+           (c->ppoly.box ? persist_box_bytes(c->ppoly.plan) : 0);
   return TL_OK;
 }
 
@@ -1263,16 +1284,16 @@ int sync_mix(tl_ctx* c) {
   return TL_OK;
 }
 
-// TL_ERR_TIMEOUT (the word cleared) if a blocked FP32 sweep set the error word: a staged row did
-// not arrive within its bounded wait (1), or its shared memory was misaligned for TMA (2).
+// TL_ERR_TIMEOUT (the word cleared) if a blocked FP32 sweep or the on-chip polynomial steps set the
+// error word: a staged row or a rim did not arrive within its bounded wait (1), or its shared memory was misaligned for TMA (2).
 int check_mix_err(tl_ctx* c) {
   unsigned werr = 0;
-  CK(cudaMemcpyAsync(&werr, c->mix.err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(&werr, c->counter + MIX_ERR_WORD, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (!werr) return TL_OK;
-  CK(cudaMemsetAsync(c->mix.err, 0, sizeof(unsigned), c->stream));
+  CK(cudaMemsetAsync(c->counter + MIX_ERR_WORD, 0, sizeof(unsigned), c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  return fail(TL_ERR_TIMEOUT, werr == 1 ? "tl_tea_leaf: a staged row of a blocked FP32 sweep did not arrive in time"
+  return fail(TL_ERR_TIMEOUT, werr == 1 ? "tl_tea_leaf: a staged row or a tile's rim did not arrive in time"
                                         : "tl_tea_leaf: shared memory misaligned for the blocked FP32 sweep");
 }
 
@@ -1488,6 +1509,7 @@ struct Solver {
   const tl_solve_opts* o;
   int use_cg, use_cheby, use_ppcg, use_jacobi;
   std::vector<double> ch_a, ch_b;
+  bool poly_used = false;  // the on-chip polynomial steps ran: the error word tells whether a wait ran out
 
   // reductions through the per-kernel path, result on the host
   int norm(const double* a, double* out) {
@@ -1578,6 +1600,12 @@ struct Solver {
     if (!fused) launch_ppcg_init_sd(c->f, c->L, c->g, c->theta, c->stream);
     const int h = c->halo_depth;
     int rc;
+    if (inner_steps > 0 && use_ppcg_inner_sweep() && use_persistent_poly(c)) {
+      poly_used = true;
+      if ((rc = run_persistent_poly(c, true, nullptr, 1, inner_steps))) return rc;
+      if (!fused) launch_copy_interior(c->f.z, c->f.utemp, c->L, c->stream);
+      return check_launch("ppcg_inner_steps");
+    }
     if (!c->g.reflective && c->g.precond == TL_PREC_NONE && use_ppcg_inner_sweep()) {
       // one sweep per step, sd ping-ponging between its two fields (the halo exchanges are
       // no-ops without reflective boundaries)
@@ -1647,12 +1675,12 @@ struct Solver {
       if (H.status == EXIT_BREAKDOWN) {
         // a blocked FP32 inner sweep that gave up waiting leaves void values behind, which can
         // break the outer iteration down before the rrn sweep reports the timeout
-        if (mixed && (rc = check_mix_err(c))) return rc;
+        if ((rc = check_mix_err(c))) return rc;
         return fail(TL_ERR_BREAKDOWN, "tl_tea_leaf: non-finite PPCG scalar");
       }
       if (H.status == EXIT_TIMEOUT) {
         const int e = check_mix_err(c);
-        return e ? e : fail(TL_ERR_TIMEOUT, "tl_tea_leaf: a blocked FP32 sweep gave up waiting");
+        return e ? e : fail(TL_ERR_TIMEOUT, "tl_tea_leaf: an inner sweep gave up waiting");
       }
       if (H.status != RUN) break;
     }
@@ -1947,6 +1975,11 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
           S.ch_b.resize(inner + 2, 0.0);
         }
         c->cn = c->eigmax / c->eigmin;
+        if (!mixed && use_persistent_poly(c)) {
+          const size_t n_ch = std::min(S.ch_a.size(), (size_t)c->ch_cap);
+          CK(cudaMemcpyAsync(c->ch_a, S.ch_a.data(), sizeof(double) * n_ch, cudaMemcpyHostToDevice, c->stream));
+          CK(cudaMemcpyAsync(c->ch_b, S.ch_b.data(), sizeof(double) * n_ch, cudaMemcpyHostToDevice, c->stream));
+        }
         // p currently lives in whichever CG buffer the last iteration wrote; step 3 rebuilds p
         launch_ppcg_init(c->f, c->L, c->g, 2, ppcg_active, c->rd(), RED_STORE, c->stream);
         if ((rc = mixed ? S.run_ppcg_inner_steps32(inner) : S.run_ppcg_inner_steps(inner))) return rc;
@@ -2001,6 +2034,26 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
           const double gamm = (std::sqrt(c->cn) - 1.0) / (std::sqrt(c->cn) + 1.0);
           est_itc = (int)std::lround(std::log(it_alpha) / std::log(gamm));
           cheby_calc_steps = 1;
+        } else if (use_cheby_sweep() && use_persistent_poly(c)) {
+          // on chip, the iterations up to the next whose residual is checked, or at which the loop
+          // ends: in between the error is the last one's repeated square root (tea_solve.f90:273,402)
+          int run = 0;
+          while (true) {
+            const int at = n + run;
+            ++run;
+            if ((at >= est_itc && at % 10 == 0) || at >= max_iters || run >= PERSIST_RUN) break;
+            const double next = std::sqrt(std::fabs(error));
+            if (next < o->eps * initial_residual) break;
+            error = next;
+          }
+          S.poly_used = true;
+          if ((rc = run_persistent_poly(c, false, u_alt ? c->f.u1 : c->f.u, cheby_calc_steps, run))) return rc;
+          u_alt = wr_stale = false;
+          cheby_calc_steps += run - 1;
+          n += run - 1;
+          if (n >= est_itc && n % 10 == 0) {
+            if ((rc = S.norm(c->f.r, &error))) return rc;
+          }
         } else {
           if ((rc = prof_begin(c))) return rc;
           cheby_iterate(S.ch_a[cheby_calc_steps], S.ch_b[cheby_calc_steps],
@@ -2065,7 +2118,7 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
     if ((rc = reduce_result(c, &exact_error))) return rc;
     exact_error = std::sqrt(exact_error);
   }
-  if (mixed && (rc = check_mix_err(c))) return rc;
+  if ((mixed || S.poly_used) && (rc = check_mix_err(c))) return rc;
   if (finalise) {
     finalise_sweep(c, flush_in_finalise);
     if ((rc = do_halo(c, M(TL_FIELD_ENERGY1), 1))) return rc;

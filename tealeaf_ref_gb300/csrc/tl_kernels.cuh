@@ -132,6 +132,14 @@ size_t persist_box_bytes(const PersistPlan& p);  // its grid sums' inboxes and t
 // no earlier launch on these boxes (zeroed once) has used them or higher ones
 cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch,
                                  void* box, cudaStream_t s, int extra = 0);
+// the FP64 polynomial steps on chip (no reflective boundaries; no preconditioner or jac_diag): `steps`
+// PPCG inner steps on sd, rtemp, utemp, or Chebyshev iterations from u_in and p into u and p (w and r,
+// and z with jac_diag, of the last one), with the coefficients ch_a[0..steps), ch_b[0..steps) in device
+// memory.  The boxes are persist_box_bytes, zeroed once; epoch .. epoch + steps - 1 as above.
+bool poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out);
+cudaError_t launch_persistent_poly(const Fields& f, const Layout& L, const PersistPlan& p, bool ppcg, bool diag,
+                                   const double* u_in, const double* ch_a, const double* ch_b, int steps,
+                                   unsigned epoch, void* box, unsigned* err, bool hold, cudaStream_t s);
 // one Jacobi iteration from un into u_out (the two swap every iteration), error and the loop's
 // test in the epilogue
 void launch_fused_jacobi(const LoopArgs& a, const double* un, double* u_out, cudaStream_t s);

@@ -1096,8 +1096,9 @@ int persist_clusters(const void* k, int cs, size_t smem) {
 
 int persist_ctas(const PersistPlan& p) { return (p.gx * p.gy + p.cs - 1) / p.cs * p.cs; }
 
+// the inboxes of two sums and the halo boxes of two steps
 size_t persist_box_bytes(const PersistPlan& p) {
-  return (size_t)persist_ctas(p) * (2 * SLOTS + 2 * (p.th + p.tw)) * sizeof(ulonglong2);
+  return (size_t)persist_ctas(p) * (2 * SLOTS + 4 * (p.th + p.tw)) * sizeof(ulonglong2);
 }
 
 // The tiling of an nx x ny mesh with the least cycles an iteration: FP64 instructions of a warp on
@@ -1228,6 +1229,293 @@ cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState*
   PersistLaunch l(persist_ctas(p), p.cs, mix_plan_smem(p), s);
   ++launch_counter();
   return cudaLaunchKernelExC(&l.cfg, (const void*)kMixKernels[m.mi ? 1 : 0], args);
+}
+
+
+// ---- the FP64 polynomial steps on chip ----------------------------------------------------------
+// The PPCG inner steps (tea_leaf_kernel_ppcg_inner, ppcg_kernel.f90:204-310) and the Chebyshev
+// iterations (tea_leaf_kernel_cheby_iterate, cheby_kernel.f90:111-200) of a mesh that fits, many steps a
+// launch.  Tiles, rims and the waits are those of the CG kernel above; the steps need no sum, so a step
+// costs its FP64 work and one hop for the rim.  The stencil variable x (sd; u) with its halo, the face
+// coefficients and Di are in shared memory, the cell's other two values (rtemp, utemp; u0, p) in
+// registers.  Every product and sum is that of the one-step kernels, in their order; Di x and b times
+// the residual run on the integer pipes, as in the staged sweeps of tl_fused.cu.  Same bits.
+//
+// A PPCG solve of 124 inner steps an outer iteration took, per inner step, 2.2 us at 60^2 against 13.6
+// with a launch a step, 2.7 / 14.9 at 256^2, 6.0 / 15.0 at 512^2, 11.8 / 19.3 at 777 x 813 and 17.3 /
+// 21.7 at 1000^2, where the FP64 pipe's share is 11; 332 Chebyshev iterations with their presteps 3.8
+// against 14.4 us each at 128^2 and 21.9 against 24.7 at 1000^2.
+namespace {
+
+constexpr int QT = 512;  // threads per CTA, all of which own cells
+enum { ON_PPCG = 0, ON_CHEBY = 1 };
+struct PolyPersistArgs {
+  Fields f;
+  Layout L;
+  PersistPlan pl;
+  const double* x_in;             // u where it lies now (Chebyshev); the steps leave it in f.u
+  const double *ch_a, *ch_b;      // coefficients of the first step ..
+  int steps;
+  unsigned epoch;                 // number of the first step's rims
+  ulonglong2* box;                // halo boxes, by parity of the number
+  unsigned* err;                  // set when a wait ran out: the results are void
+  int hold;                       // test of the bounded wait: the first tile sends no rims
+};
+
+template <int M, int MODE, bool DIAG>
+__global__ void __launch_bounds__(QT, 1) k_persistent_poly(PolyPersistArgs g) {
+  constexpr bool PPCG = MODE == ON_PPCG;
+  __shared__ int sh_fail;
+  extern __shared__ __align__(16) double qsm[];
+  const Layout L = g.L;
+  const Fields& f = g.f;
+  const int t = threadIdx.x;
+  if (t == 0) sh_fail = *reinterpret_cast<volatile unsigned*>(g.err) != 0u;
+
+  const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
+  const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;
+  const int tw = min(g.pl.tw, L.nx - j0), th = min(g.pl.th, L.ny - k0);
+  const int P = g.pl.tw + 2, ry = g.pl.ry;
+  const int asz = (g.pl.th + 2) * P;
+  double* const sx = qsm;
+  double* const scx = qsm + asz;
+  double* const scy = qsm + 2 * asz;
+  double* const sdi = qsm + 3 * asz;
+  const double* const xin = PPCG ? f.sd : g.x_in;
+
+  const int tx = t % g.pl.tw, ty = t / g.pl.tw;
+  const int mine = (tx < tw && ty < ry && ty < th) ? (th - 1 - ty) / ry + 1 : 0;
+  const int o0 = (ty + 1) * P + tx + 1;
+  const int c0 = (int)L.at(j0 + tx + 1, k0 + ty + 1);
+  const int ostep = ry * P, cstep = ry * L.ld;
+  const int i_first = ty == 0 ? 0 : -1, i_last = (mine > 0 && (th - 1 - ty) % ry == 0) ? mine - 1 : -1;
+
+  const int hbox = 2 * (g.pl.th + g.pl.tw), hall = (int)gridDim.x * hbox;
+  int ho[PH], hh[PH];
+#pragma unroll
+  for (int q = 0; q < PH; ++q) {
+    const int h = t + q * QT;
+    ho[q] = -1;
+    hh[q] = 0;
+    int x = -1, y = h;
+    bool in = y < th, is = in && j0 > 0;
+    if (h >= g.pl.th) x = tw, y = h - g.pl.th, in = y < th, is = in && j0 + tw < L.nx;
+    if (h >= 2 * g.pl.th) x = h - 2 * g.pl.th, y = -1, in = x < tw, is = in && k0 > 0;
+    if (h >= 2 * g.pl.th + g.pl.tw) x = h - 2 * g.pl.th - g.pl.tw, y = th, in = x < tw, is = in && k0 + th < L.ny;
+    if (in && h < hbox) {
+      const int o = (y + 1) * P + x + 1;
+      sx[o] = xin[L.at(j0 + x + 1, k0 + y + 1)];  // off the domain: the field's halo, which stays
+      if (is) {
+        ho[q] = o;
+        hh[q] = (int)blockIdx.x * hbox + h;
+      }
+    }
+  }
+  const bool sends = !(g.hold && blockIdx.x == 0);
+  const int to_l = (sends && tx == 0 && j0 > 0) ? ((int)blockIdx.x - 1) * hbox + g.pl.th + ty : -1;
+  const int to_r = (sends && tx == tw - 1 && j0 + tw < L.nx) ? ((int)blockIdx.x + 1) * hbox + ty : -1;
+  const int rim_b = sends && k0 > 0 ? i_first : -1, rim_t = sends && k0 + th < L.ny ? i_last : -1;
+  const int to_b = ((int)blockIdx.x - g.pl.gx) * hbox + 2 * g.pl.th + g.pl.tw + tx;
+  const int to_t = ((int)blockIdx.x + g.pl.gx) * hbox + 2 * g.pl.th + tx;
+
+  double r[M], s[M];  // PPCG: rtemp, utemp; Chebyshev: u0 and then the residual of the step, p
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const int o = o0 + i * ostep, c = c0 + i * cstep;
+    r[i] = s[i] = 0.0;
+    if (i < mine) {
+      sx[o] = xin[c];
+      r[i] = PPCG ? f.rtemp[c] : f.u0[c];
+      s[i] = PPCG ? f.utemp[c] : f.p[c];
+      sdi[o] = f.di[c];
+      scx[o] = f.cx[c];
+      scy[o] = f.cy[c];
+      if (tx == tw - 1) scx[o + 1] = f.cx[c + 1];
+      if (i == i_last) scy[o + P] = f.cy[c + L.ld];
+    }
+  }
+  __syncthreads();
+  if (sh_fail) return;
+
+  unsigned epoch = g.epoch;
+  bool failed = false;
+  for (int step = 0; step < g.steps; ++step, ++epoch) {
+    const bool last = step + 1 == g.steps;
+    const double ca = __ldg(g.ch_a + step), cb = __ldg(g.ch_b + step);
+    ulonglong2* const halo = g.box + (size_t)(epoch & 1u) * hall;
+    int o = fresh(o0), c = fresh(c0);
+    // the residual of the owned cells (x is complete in shared memory)
+#pragma unroll
+    for (int i = 0; i < M; ++i, o += ostep, c += cstep) {
+      if (i < mine) {
+        double a = dmul_int(sdi[o], sx[o]);
+        a = fma(-scy[o + P], sx[o + P], a);
+        a = fma(-scy[o], sx[o - P], a);
+        a = fma(-scx[o + 1], sx[o + 1], a);
+        a = fma(-scx[o], sx[o - 1], a);
+        const double res = r[i] - a;
+        r[i] = res;
+        if (!PPCG && last) {
+          f.w[c] = a;
+          f.r[c] = res;
+        }
+      }
+    }
+    __syncthreads();  // every read of x is done
+    o = fresh(o0), c = fresh(c0);
+    int l = fresh(to_l), e = fresh(to_r);
+#pragma unroll
+    for (int i = 0; i < M; ++i, o += ostep, c += cstep, l += ry, e += ry) {
+      if (i < mine) {
+        double z = r[i];
+        if (DIAG) {
+          z = __ldg(f.mi + c) * z;
+          if (!PPCG && last) f.z[c] = z;
+        }
+        const double bz = dmul_int(cb, z);
+        double x = sx[o];
+        if (PPCG) {
+          x = fma(ca, x, bz);
+          s[i] = s[i] + x;
+        } else {
+          s[i] = fma(ca, s[i], bz);
+          x = x + s[i];
+          r[i] = __ldg(f.u0 + c);
+        }
+        sx[o] = x;
+        if (to_l >= 0) box_put(halo + l, x, epoch);
+        if (to_r >= 0) box_put(halo + e, x, epoch);
+        if (i == rim_b) box_put(halo + to_b, x, epoch);
+        if (i == rim_t) box_put(halo + to_t, x, epoch);
+      }
+    }
+    if (!last) {
+      bool got = false;
+      double hv[PH];
+      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+        got = true;
+#pragma unroll
+        for (int q = 0; q < PH; ++q)
+          if (ho[q] >= 0) {
+            const ulonglong2 v = box_get(halo + hh[q]);
+            got = got && box_is(v, epoch);
+            hv[q] = box_value(v);
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < PH; ++q)
+        if (ho[q] >= 0) sx[ho[q]] = hv[q];
+      if (!got) sh_fail = 1;
+      __syncthreads();
+      if (sh_fail) {
+        failed = true;
+        break;
+      }
+    }
+  }
+  if (failed) {
+    if (t == 0) atomicExch(g.err, 1u);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const int o = o0 + i * ostep, c = c0 + i * cstep;
+    if (i < mine) {
+      if (PPCG) {
+        f.sd[c] = sx[o];
+        f.rtemp[c] = r[i];
+        f.utemp[c] = s[i];
+      } else {
+        f.u[c] = sx[o];
+        f.p[c] = s[i];
+      }
+    }
+  }
+}
+
+using PolyPersistKernel = void (*)(PolyPersistArgs);
+struct PolyPersistVariant {
+  int m;
+  PolyPersistKernel k[2][2];  // PPCG / Chebyshev, without / with jac_diag
+};
+#define POLY_VARIANT(M)                                                                      \
+  {M,                                                                                        \
+   {{k_persistent_poly<M, ON_PPCG, false>, k_persistent_poly<M, ON_PPCG, true>},             \
+    {k_persistent_poly<M, ON_CHEBY, false>, k_persistent_poly<M, ON_CHEBY, true>}}}
+const PolyPersistVariant kPolyVariants[] = {POLY_VARIANT(1), POLY_VARIANT(2), POLY_VARIANT(4),
+                                            POLY_VARIANT(7), POLY_VARIANT(10), POLY_VARIANT(14)};
+size_t poly_plan_smem(const PersistPlan& p) { return (size_t)4 * (p.th + 2) * (p.tw + 2) * sizeof(double); }
+
+// The tiling with the fewest cycles a step: 7 FP64 instructions of a warp a row (17 cycles of the SM's
+// four pipes each), the halo, and the rim's hop (1500 cycles) when there is more than one tile.
+bool poly_plan(int nx, int ny, int ctas, PersistPlan* out) {
+  double best = 0.0;
+  bool found = false;
+  for (int g0 = 1; g0 <= ctas && g0 <= nx; ++g0) {
+    const int tw = (nx + g0 - 1) / g0;
+    if (tw > QT) continue;
+    PersistPlan p{};
+    p.cs = 1;
+    p.tw = tw;
+    p.gx = (nx + tw - 1) / tw;
+    for (int many = 0; many < 2; ++many) {
+      int gy = many ? ctas / p.gx : 1;
+      if (gy > ny) gy = ny;
+      if (gy < 1) continue;
+      p.th = (ny + gy - 1) / gy;
+      p.gy = (ny + p.th - 1) / p.th;
+      p.ry = QT / tw < p.th ? QT / tw : p.th;
+      const int m = (p.th + p.ry - 1) / p.ry;
+      p.variant = -1;
+      for (int v = (int)(sizeof(kPolyVariants) / sizeof(kPolyVariants[0])) - 1; v >= 0; --v)
+        if (kPolyVariants[v].m >= m) p.variant = v;
+      const int halo = 2 * (p.tw + p.th);
+      if (p.variant < 0 || halo > PH * QT || poly_plan_smem(p) > PERSIST_SMEM_MAX) continue;
+      const double cost =
+          (double)((p.ry * tw + 31) / 32) * m * 119.0 + 0.5 * halo + 4.0 * p.th + (p.gx * p.gy > 1 ? 1500.0 : 0.0);
+      if (!found || cost < best) {
+        best = cost;
+        *out = p;
+        found = true;
+      }
+    }
+  }
+  return found;
+}
+
+// threads of one CTA differ between the kernels
+int poly_ctas(const void* k, size_t smem) {
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM_MAX) != cudaSuccess ||
+      cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, QT, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return sms * per_sm;
+}
+
+}  // namespace
+
+bool poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
+  const int diag = precond == 2 ? 1 : 0;
+  const int ctas = poly_ctas((const void*)kPolyVariants[0].k[0][diag], PERSIST_SMEM_MAX);
+  if (!poly_plan(nx, ny, ctas, out)) return false;
+  for (int mode = 0; mode < 2; ++mode)
+    if (poly_ctas((const void*)kPolyVariants[out->variant].k[mode][diag], poly_plan_smem(*out)) < persist_ctas(*out))
+      return false;
+  return true;
+}
+
+cudaError_t launch_persistent_poly(const Fields& f, const Layout& L, const PersistPlan& p, bool ppcg, bool diag,
+                                   const double* u_in, const double* ch_a, const double* ch_b, int steps,
+                                   unsigned epoch, void* box, unsigned* err, bool hold, cudaStream_t s) {
+  PolyPersistArgs g{f, L, p, u_in, ch_a, ch_b, steps, epoch, static_cast<ulonglong2*>(box), err, hold ? 1 : 0};
+  void* args[] = {&g};
+  ++launch_counter();
+  return cudaLaunchCooperativeKernel((const void*)kPolyVariants[p.variant].k[ppcg ? 0 : 1][diag ? 1 : 0],
+                                     dim3(persist_ctas(p)), dim3(QT), args, poly_plan_smem(p), s);
 }
 
 }  // namespace tl

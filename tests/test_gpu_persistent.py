@@ -65,3 +65,57 @@ def test_persistent_fp32_steps_match_the_sweeps(size, case, monkeypatch):
     assert i1.kernel_launches < i0.kernel_launches, "the persistent kernel did not run"
     assert i1.cg_calc_steps == i0.cg_calc_steps == 8 and i1.outer_iterations == i0.outer_iterations
     assert np.max(np.abs(u1 - u0)) <= 8 * 2 * 8 * 2.0 ** -23 * np.max(np.abs(u0 - b))
+
+
+POLY_SIZES = [(9, 9), (22, 21), (1, 700), (700, 1), (97, 131), (301, 499), (600, 433), (777, 813), (1000, 1000)]
+
+
+@pytest.mark.parametrize("precond", ["none", "jac_diag"])
+@pytest.mark.parametrize("solver", ["ppcg", "chebyshev"])
+@pytest.mark.parametrize("size", POLY_SIZES, ids=["%dx%d" % s for s in POLY_SIZES])
+def test_on_chip_polynomial_steps_give_the_same_bits(size, solver, precond, monkeypatch):
+    """The FP64 PPCG inner steps and Chebyshev iterations on chip against the sweeps in memory: the
+    same bits in every field, over two time steps (with odd and even step counts, and residual checks
+    between launches)."""
+    from tealeaf_ref_gb300 import native
+
+    d = small_deck(nx=size[0], ny=size[1], solver=solver, precond=precond, ppcg_inner_steps=7, ch_cg_presteps=6,
+                   ch_cg_epslim=1e30, max_iters=14 if solver == "ppcg" else 87, steps=2)
+    fields = ["u", "w", "r", "p", "sd", "rtemp", "utemp"] + (["z"] if precond == "jac_diag" else [])
+    runs = []
+    for form in ("0", "1"):
+        monkeypatch.setenv("TL_POLY_PERSISTENT", form)
+        with native.Chunk.from_deck(d) as c:
+            infos = [c.tea_leaf(d) for _ in range(2)]
+            runs.append((infos, {f: c.download(f) for f in fields}))
+    (i0, f0), (i1, f1) = runs
+    assert sum(i.cheby_calc_steps for i in i0) > 0
+    assert sum(i.kernel_launches for i in i1) < sum(i.kernel_launches for i in i0), "the on-chip steps did not run"
+    for a, b in zip(i0, i1):
+        assert (a.n_exit, a.error, a.cheby_calc_steps, a.ppcg_inner_iters) == \
+               (b.n_exit, b.error, b.cheby_calc_steps, b.ppcg_inner_iters)
+    for f in fields:
+        assert np.array_equal(f0[f], f1[f]), f
+
+
+@pytest.mark.parametrize("solver", ["ppcg", "chebyshev"])
+def test_on_chip_polynomial_wait_is_bounded(solver, monkeypatch):
+    """One tile keeps its rim to itself: its neighbours' waits run out after about a second, the solve
+    returns TL_ERR_TIMEOUT, and the context then solves normally."""
+    from tealeaf_ref_gb300 import native
+
+    d = small_deck(nx=200, ny=160, solver=solver, ppcg_inner_steps=6, ch_cg_presteps=10, ch_cg_epslim=1e30,
+                   max_iters=60, steps=1)
+    with native.Chunk.from_deck(d) as c:
+        want = c.tea_leaf(d)
+        c.generate(d)
+        c.reset_eigen()
+        monkeypatch.setenv("TL_CG_BARRIER_EXTRA", "2")
+        with pytest.raises(native.TeaLeafError) as e:
+            c.tea_leaf(d)
+        assert e.value.code == -5  # TL_ERR_TIMEOUT
+        monkeypatch.delenv("TL_CG_BARRIER_EXTRA")
+        c.generate(d)
+        c.reset_eigen()
+        got = c.tea_leaf(d)
+        assert (got.n_exit, got.error) == (want.n_exit, want.error)
