@@ -38,12 +38,14 @@ inline dim3 row_grid(const Layout& L, bool reducing) {
   return dim3(gx, gy);
 }
 
-// two columns a thread: a reducing kernel on 27 CTAs per SM striding over rows.  The u, r update with
-// its sum took 86, 148 and 529 us at 3001 x 1999 (jac_diag), 4096^2 and 8192^2, against 89, 163 and 582
-// with 6 per SM, 86, 156 and 553 with 16, and 99, 149 and 507 with 54 (more partials to sum).
+// Two columns a thread; a reducing kernel strides over rows on 27 CTAs per SM from two million cells
+// on, on 6 below.  The u, r update with its sum took 86, 148 and 529 us at 3001 x 1999 (jac_diag),
+// 4096^2 and 8192^2 on 27, against 89, 163 and 582 on 6, 86, 156 and 553 on 16, and 99, 149 and 507 on
+// 54 (more partials to sum); at 1000^2 27.5 on 27 against 25.2 on 6.
 inline dim3 pair_grid(const Layout& L, bool reducing) {
   const int gx = (L.nx + 2 * TB - 1) / (2 * TB);
-  int gy = reducing ? (27 * sm_count() + gx - 1) / gx : L.ny;
+  const int per_sm = (long long)L.nx * L.ny >= 2LL << 20 ? 27 : 6;
+  int gy = reducing ? (per_sm * sm_count() + gx - 1) / gx : L.ny;
   if (gy > L.ny) gy = L.ny;
   if (gy > 65535) gy = 65535;
   return dim3(gx, gy);
