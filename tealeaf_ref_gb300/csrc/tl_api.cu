@@ -142,7 +142,7 @@ struct tl_ctx {
   double* tape_field(int i) const { return reinterpret_cast<double*>(tape + (size_t)i * field_stride); }
 
   double* slot(int s) const { return reinterpret_cast<double*>(slab + (size_t)s * field_stride); }
-  Reduce rd() const { return Reduce{partials, counter, st, hist_a, hist_b, ch_a, ch_b}; }
+  Reduce rd() const { return Reduce{partials, counter, st, hist_a, hist_b, ch_a, ch_b, st_host ? st_host->red : nullptr}; }
   LoopArgs loop() const { return LoopArgs{f, L, rd(), g.precond, g.reflective, g.ry, g.rx}; }
 };
 
@@ -189,9 +189,10 @@ int push_state(tl_ctx* c) {
   return TL_OK;
 }
 
+// the sums of the reducing kernel queued last, which its epilogue wrote into the pinned mirror: a copy
+// queued behind the kernel costs a call some 4 us more
 int reduce_result(tl_ctx* c, double* out, int lanes = 1) {
-  int rc = sync_state(c);
-  if (rc) return rc;
+  CK(cudaStreamSynchronize(c->stream));
   for (int i = 0; i < lanes; ++i) out[i] = c->st_host->red[i];
   return TL_OK;
 }
@@ -391,7 +392,8 @@ int run_persistent(tl_ctx* c, const LoopArgs& la) {
   // TL_CG_BARRIER_EXTRA=1: the grid sums wait for one partial that never comes, so every wait runs
   // out (about a second) and the solve reports TL_ERR_TIMEOUT -- the test of the bounded wait
   const char* ex = getenv("TL_CG_BARRIER_EXTRA");
-  CK(launch_persistent_cg(la, c->pcg.plan, PERSIST_RUN, epoch, c->pcg.box, c->stream, ex && ex[0] == '1' ? 1 : 0));
+  CK(launch_persistent_cg(la, c->pcg.plan, PERSIST_RUN, epoch, c->pcg.box, c->st_host, c->stream,
+                          ex && ex[0] == '1' ? 1 : 0));
   return TL_OK;
 }
 
@@ -1775,8 +1777,9 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
     launch_jacobi_denominator(c->f, c->L, c->g, c->stream);
   }
   if ((rc = check_launch("tea_leaf init"))) return rc;
-  if ((rc = sync_state(c))) return rc;
-  const double initial_residual = H.initial_residual;
+  // CG runs on without the host: its initial residual comes with the first batch's state
+  if (!S.use_cg && (rc = sync_state(c))) return rc;
+  double initial_residual = H.initial_residual;
 
   // ---- iteration (tea_solve.f90:152-414) ----
   int n = 1;
@@ -1839,7 +1842,8 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
       LoopArgs la = c->loop();
       const int n_before = n;
       bool sampled = false;  // the timed graph form: only iteration TIMED_ITER of the batch is timed
-      if (use_persistent(c, c->pcg, persist_prepare)) {
+      const bool persistent = use_persistent(c, c->pcg, persist_prepare);
+      if (persistent) {
         if (H.u_pending) launch_flush_u(la, c->stream);  // of the batched kernels (none normally)
         if ((rc = run_persistent(c, la))) return rc;
       } else if (!c->prof && use_graphs()) {
@@ -1857,7 +1861,11 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
         }
       }
       if ((rc = check_launch("cg batch"))) return rc;
-      if ((rc = sync_state(c))) return rc;
+      if (persistent)
+        CK(cudaStreamSynchronize(c->stream));  // the kernel wrote the state into the mirror too
+      else if ((rc = sync_state(c)))
+        return rc;
+      initial_residual = H.initial_residual;
       if (c->prof) {
         // iterations of this batch that did work (the rest returned on the status word); the
         // graph form times its sampled iteration only
@@ -1883,7 +1891,7 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
         // the CG phase stops here: apply the deferred u += alpha p of its last iteration -- in
         // the finalise sweep when nothing reads u before it (a CG solve without check_result)
         if (S.use_cg && finalise && !o->check_result) {
-          flush_in_finalise = true;
+          flush_in_finalise = H.u_pending != 0;
         } else {
           launch_flush_u(la, c->stream);
           H.u_pending = 0;

@@ -148,6 +148,7 @@ struct Reduce {
   double* hist_b;      // cg_betas
   const double* ch_a;  // Chebyshev / PPCG coefficients, 1-based
   const double* ch_b;
+  double* red_host;    // where a caller on the host reads the sums after its stream has synchronised
 };
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -679,12 +679,14 @@ template <int MODE>
 struct EpiApply {
   LoopState* st;
   int mode;
+  double* host;
   __device__ void operator()(double (&acc)[1]) const {
     if (mode == RED_INIT_RESIDUAL) {
       st->old_error = acc[0];
       st->initial_residual = sqrt(fabs(acc[0]));
     }
     st->red[0] = acc[0];
+    if (host) host[0] = acc[0];
   }
 };
 
@@ -785,7 +787,7 @@ __global__ void __launch_bounds__(FT, 7) k_apply_ws(Fields f, Layout L, Reduce r
   if (MODE == AP_W || MODE == AP_RN) {
     acc[0] += acc_b;
     __syncthreads();  // every thread is done with the ring: it becomes the block sum's scratch
-    grid_reduce_in<1>(acc, rd, EpiApply<MODE>{rd.st, mode}, aring);
+    grid_reduce_in<1>(acc, rd, EpiApply<MODE>{rd.st, mode, rd.red_host}, aring);
   }
 }
 

@@ -62,6 +62,7 @@ template <int NV>
 struct EpiMode {
   LoopState* st;
   int mode;
+  double* host;  // the caller's copy of the sums, in mapped host memory
   __device__ void operator()(double (&acc)[NV]) const {
     switch (mode) {
       case RED_INIT_RESIDUAL:
@@ -75,7 +76,10 @@ struct EpiMode {
         break;
     }
 #pragma unroll
-    for (int i = 0; i < NV; ++i) st->red[i] = acc[i];
+    for (int i = 0; i < NV; ++i) {
+      st->red[i] = acc[i];
+      if (host) host[i] = acc[i];
+    }
   }
 };
 
@@ -334,7 +338,7 @@ __global__ void k_field_summary(Fields f, Layout L, double cell_vol, Reduce rd) 
     const long long c = L.at(j, k);
     summary_terms(v, cell_vol, f.density[c], f.energy1[c], f.u[c]);
   }
-  grid_reduce<4>(v, rd, EpiMode<4>{rd.st, RED_STORE});
+  grid_reduce<4>(v, rd, EpiMode<4>{rd.st, RED_STORE, rd.red_host});
 }
 
 // tea_leaf_kernel_finalise (common_kernel.f90:179-206) fused with field_summary_kernel
@@ -358,7 +362,7 @@ __global__ void k_finalise_summary(Fields f, Layout L, double cell_vol, Reduce r
     f.energy1[c] = e;
     summary_terms(v, cell_vol, rho, e, u);
   }
-  grid_reduce<4>(v, rd, EpiMode<4>{rd.st, RED_STORE});
+  grid_reduce<4>(v, rd, EpiMode<4>{rd.st, RED_STORE, rd.red_host});
 }
 
 // update_halo_cell (update_halo_kernel.f90:136-195) at depth 1: left/right columns first
@@ -421,7 +425,7 @@ __global__ void k_residual(Fields f, Layout L, Reduce rd, int mode) {
     f.r[c] = r;
     if (NORM) v[0] = fma(r, r, v[0]);
   }
-  if (NORM) grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode});
+  if (NORM) grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode, rd.red_host});
 }
 
 // tea_leaf_calc_2norm_kernel (common_kernel.f90:246-274)
@@ -432,7 +436,7 @@ __global__ void k_norm2(const double* __restrict__ a, Layout L, Reduce rd, int m
     const double x = a[L.at(j, k)];
     v[0] = fma(x, x, v[0]);
   }
-  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode});
+  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode, rd.red_host});
 }
 
 // sum a.(b - bminus)  (ppcg_calc_zrnorm, ppcg_calc_rrn, cg_init's r.p)
@@ -445,7 +449,7 @@ __global__ void k_dot(const double* __restrict__ a, const double* __restrict__ b
     const double y = bm ? (b[c] - bm[c]) : b[c];
     v[0] = fma(a[c], y, v[0]);
   }
-  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode});
+  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode, rd.red_host});
 }
 
 // tea_leaf_kernel_finalise (common_kernel.f90:179-206)
@@ -522,7 +526,7 @@ __global__ void k_cg_init(Fields f, Layout L, int precond, Reduce rd, int mode) 
     f.p[c] = p;
     v[0] = fma(f.r[c], p, v[0]);
   }
-  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode});
+  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode, rd.red_host});
 }
 
 // tea_leaf_cg_calc_w_kernel (cg_kernel.f90:114-156)
@@ -535,7 +539,7 @@ __global__ void k_cg_calc_w(Fields f, Layout L, Reduce rd) {
     f.w[c] = w;
     v[0] = fma(w, f.p[c], v[0]);
   }
-  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, RED_STORE});
+  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, RED_STORE, rd.red_host});
 }
 
 // The drop-in CG updates, two columns a thread (16-byte accesses; interior rows start on 128 bytes):
@@ -579,7 +583,7 @@ __global__ void __launch_bounds__(TB) k_cg_calc_ur(Fields f, Layout L, double al
       }
     }
   }
-  if (MODE != 2) grid_reduce<1>(v, rd, EpiMode<1>{rd.st, RED_STORE});
+  if (MODE != 2) grid_reduce<1>(v, rd, EpiMode<1>{rd.st, RED_STORE, rd.red_host});
 }
 
 // tea_leaf_cg_calc_p_kernel (cg_kernel.f90:306-347)
@@ -661,7 +665,7 @@ __global__ void k_ppcg_init(Fields f, Layout L, int step, int pz, int pr, Reduce
     f.p[c] = p;
     v[0] = fma(f.r[c], p, v[0]);
   }
-  if (step != 2) grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode});
+  if (step != 2) grid_reduce<1>(v, rd, EpiMode<1>{rd.st, mode, rd.red_host});
 }
 
 // tea_leaf_kernel_ppcg_inner (ppcg_kernel.f90:204-310), phase 1: rtemp -= A sd
@@ -697,7 +701,7 @@ __global__ void k_jacobi(Fields f, Layout L, Reduce rd, double rx, double ry) {
     f.u[c] = u;
     v[0] += fabs(u - un[c]);
   }
-  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, RED_STORE});
+  grid_reduce<1>(v, rd, EpiMode<1>{rd.st, RED_STORE, rd.red_host});
 }
 
 // the Jacobi denominator (jacobi_kernel.f90:67-69, exact operation order) and its reciprocal

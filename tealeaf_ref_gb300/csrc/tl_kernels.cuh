@@ -129,9 +129,10 @@ struct PersistPlan {
 bool persist_prepare(int nx, int ny, int precond, PersistPlan* out);
 size_t persist_box_bytes(const PersistPlan& p);  // its grid sums' inboxes and the tiles' halo boxes
 // up to max_run iterations in one launch; epoch .. epoch + 2 max_run - 1 number its grid sums, and
-// no earlier launch on these boxes (zeroed once) has used them or higher ones
+// no earlier launch on these boxes (zeroed once) has used them or higher ones.  The state is left in
+// a.rd.st and in st_host (mapped host memory)
 cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch,
-                                 void* box, cudaStream_t s, int extra = 0);
+                                 void* box, LoopState* st_host, cudaStream_t s, int extra = 0);
 // the FP64 polynomial steps on chip (no reflective boundaries; no preconditioner or jac_diag): `steps`
 // PPCG inner steps on sd, rtemp, utemp, or Chebyshev iterations from u_in and p into u and p (w and r,
 // and z with jac_diag, of the last one), with the coefficients ch_a[0..steps), ch_b[0..steps) in device

@@ -62,6 +62,7 @@ struct PersistArgs {
   int max_run;
   unsigned epoch;   // number of the launch's first grid sum
   ulonglong2* box;  // by parity of the sum's number, an inbox per CTA; then the tiles' halo boxes
+  LoopState* st_host;
   int extra;        // partials waited for beyond the grid's (the test of the bounded wait)
 };
 
@@ -252,7 +253,10 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
     cluster_sync();  // every CTA's box is empty before a peer writes into it
   else
     __syncthreads();
-  if (sh_status != RUN) return;  // in every CTA
+  if (sh_status != RUN) {  // in every CTA
+    if (blockIdx.x == 0 && t == 0) *g.st_host = S;
+    return;
+  }
 
   const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
   const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;  // first cell of the tile, from 0
@@ -557,7 +561,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
   }
   if (cs > 1) cluster_sync();  // no CTA leaves while a peer may still write into its shared memory
   if (X.fail) {
-    if (t == 0) g.a.rd.st->status = EXIT_TIMEOUT;
+    if (t == 0) g.a.rd.st->status = g.st_host->status = EXIT_TIMEOUT;
     return;
   }
   // ---- the fields and the state as the loop's kernels leave them (w = A p_n formed again) ----
@@ -596,6 +600,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       }
     }
     *g.a.rd.st = S;
+    *g.st_host = S;
   }
 }
 
@@ -1160,8 +1165,8 @@ bool persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
 }
 
 cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch, void* box,
-                                 cudaStream_t s, int extra) {
-  PersistArgs g{a, p, max_run, epoch, static_cast<ulonglong2*>(box), extra};
+                                 LoopState* st_host, cudaStream_t s, int extra) {
+  PersistArgs g{a, p, max_run, epoch, static_cast<ulonglong2*>(box), st_host, extra};
   void* args[] = {&g};
   PersistLaunch l(persist_ctas(p), p.cs, plan_smem(p), s);
   ++launch_counter();
