@@ -231,6 +231,10 @@ template <int M, bool DIAG>
 __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
   constexpr bool PREG = M <= 4, UREG = M <= 6, DISM = M <= 14;
   constexpr int MG = M < 6 ? M : 6;  // rows whose loads from the fields are in flight together
+  // Where the FP64 pipe bounds the iteration the products Di p and Mi r run on the integer pipes
+  // (dmul_int, the same bits): 14.8 -> 14.2 us at 700^2, 23.7 -> 22.5 at 777 x 1013 with jac_diag, 24.6 ->
+  // 23.5 at 1000^2.  Above 14 cells a thread its registers spill (26.2 -> 27.0 us at 1024^2).
+  constexpr bool EMU = M > 2 && M <= 14;
   __shared__ LoopState S;
   __shared__ Exchange X;
   __shared__ double sh_alpha, sh_beta;
@@ -425,7 +429,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
           const int i = i0 + j;
           if (i < M && i < mine) {
             const double pc = PREG ? pr[i] : sp[o];
-            double wv = (DISM ? sdi[o] : di[DISM ? 0 : j]) * pc;
+            const double dd = DISM ? sdi[o] : di[DISM ? 0 : j];
+            double wv = EMU ? dmul_int(dd, pc) : dd * pc;
             wv = fma(-scy[o + P], sp[o + P], wv);
             wv = fma(-scy[o], sp[o - P], wv);
             wv = fma(-scx[o + 1], sp[o + 1], wv);
@@ -476,7 +481,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
             r[i] = rv;
             double zv = rv;
             if (DIAG) {
-              zv = (UREG ? mi[UREG ? i : 0] : mg[UREG ? 0 : j]) * rv;
+              const double mm = UREG ? mi[UREG ? i : 0] : mg[UREG ? 0 : j];
+              zv = EMU ? dmul_int(mm, rv) : mm * rv;
               w[i] = zv;
             }
             if (to_l >= 0) box_put(halo + l, zv, epoch);
