@@ -339,7 +339,7 @@ bool writes_setup_input(int field) {
          field == TL_FIELD_MI;
 }
 
-// The persistent on-chip loops take every plain or jac_diag CG whose mesh fits: FP64 to about 1100^2
+// The persistent on-chip loops take every plain or jac_diag CG whose mesh fits: FP64 to about 1400^2
 // cells, the FP32 process of the precision form to about 2050^2.  TL_CG_PERSISTENT=0 forces them off.
 constexpr int PERSIST_RUN = 1024;  // iterations per launch at most (the host reads the status between)
 

@@ -32,10 +32,9 @@
 //
 // Time per CG iteration, the solve's set-up included, against the form before it (up to 640K cells
 // one persistent kernel with the fields in memory and two barriers an iteration, above the batched
-// sweeps of tl_fused.cu in CUDA graphs): 64^2 3.9 against 12 us, 128^2 5.9 / 13.8, 256^2 7.2 / 14.5,
-// 512^2 10.4 / 27.6, 777 x 1013 with jac_diag 23.7 / 43.9, 1000^2 24.5 / 47, 1024^2 26.0 / 42.4.
-// Every mesh that fits runs here: the largest, 1100^2, is where it gains least.  The FP64 pipe's
-// share is 1.1 us at 256^2 and 17 us at 1000^2.
+// sweeps of tl_fused.cu in CUDA graphs): 64^2 3.8 against 12 us, 128^2 5.9 / 13.8, 256^2 7.2 / 14.5,
+// 512^2 10.2 / 27.6, 700^2 14.2 / 34.8, 777 x 1013 with jac_diag 22.3 / 43.9; larger meshes, to about
+// 1400^2, take k_persistent_cg_wide.  The FP64 pipe's share is 1.1 us at 256^2 and 8 us at 700^2.
 #include "tl_mixed.cuh"
 
 namespace tl {
@@ -224,17 +223,84 @@ __device__ __noinline__ double exchange_sum(Exchange* x, ulonglong2* in, unsigne
 //   2  owners only: p is complete in shared memory;
 //   3  the words of the inbox are added up (the polling warps arrive, the first warp waits);
 //   0  the sum's outcome is in shared memory (all).
-// M: cells a thread may own.  From sizes up on a tile's share grows past the registers and the
-// shared memory: p of the owned cells stays in registers too up to 4, u and Mi up to 6 (they are in
-// the fields otherwise, u updated in the wait for beta), and Di is read from the field above 14.
+// The loop's scalars in the first warp (tea_solve.f90:341-369), and their epilogues.
+struct CgScalars {
+  double rro, inv_rro = 0.0, pw, alpha, beta, rrn;
+  uint64_t goal2;
+  bool check_switch, error_due = false;
+  int max_iters;
+
+  __device__ __forceinline__ explicit CgScalars(const LoopState& S)
+      : rro(S.rro), pw(S.pw), alpha(S.alpha), beta(S.beta), rrn(S.rrn), check_switch(S.check_switch != 0),
+        max_iters(S.max_iters) {
+    const double goal = S.eps * S.initial_residual;
+    goal2 = emu::bits(goal > 1e-140 ? goal * goal * (1.0 + 1e-12) : INFINITY);
+  }
+  // pw is known: alpha
+  __device__ __forceinline__ void after_pw(LoopState* S, int n, double* sh_alpha, int* sh_status, double* hist) {
+    alpha = rro / pw;
+    if ((threadIdx.x & 31) == 0) {
+      *sh_alpha = alpha;
+      if (!finite_bits(alpha)) {
+        S->status = EXIT_BREAKDOWN;
+        S->n_exit = n;
+        *sh_status = EXIT_BREAKDOWN;
+      }
+      if (blockIdx.x == 0) hist[n] = alpha;
+    }
+  }
+  // rrn is known: beta, the error, the loop's tests
+  __device__ __forceinline__ void after_rrn(LoopState* S, int n, double* sh_beta, int* sh_status, double* hist) {
+    // rrn / rro from the reciprocal of rro: one correction gives the correctly rounded quotient
+    // in the normal range (P. Markstein, IBM J. Res. Dev. 34(1), 1990); else the division
+    double b = rrn * inv_rro;
+    b = fma(fma(-b, rro, rrn), inv_rro, b);
+    const unsigned eb = expo(b), eo = expo(rro);
+    if (eb < 300u || eb > 1700u || eo < 300u || eo > 1700u) b = rrn / rro;
+    beta = b;
+    // without the square root when the outcome is plain: the error is far enough above the goal
+    // (goal2: its square with a margin; non-negative doubles order as their bits) and nothing
+    // else can stop the loop.  The error itself is then left to the launch's end.
+    error_due = !check_switch && n < max_iters && (emu::bits(rrn) & ~emu::SIGN) > goal2 && expo(rrn) < 2000u;
+    if ((threadIdx.x & 31) == 0) {
+      *sh_beta = b;
+      if (!error_due) {
+        S->n = n;
+        loop_finish_iteration(S, rrn);
+        *sh_status = S->status;
+      }
+      if (blockIdx.x == 0) hist[n] = b;
+    }
+    rro = rrn;
+  }
+  // one thread: the state after `done` iterations, the next being n
+  __device__ __forceinline__ void store(LoopState& S, int n, int done) const {
+    S.u_pending = 0;
+    S.pw = pw;
+    S.alpha = alpha;
+    S.cg_calc_steps += done;
+    if (done > 0) {
+      S.rrn = rrn;
+      S.beta = beta;
+      S.rro = rro;
+      S.p_pending = 1;
+      if (error_due) {
+        S.n = n;
+        S.error = S.old_error = sqrt(fabs(rrn));
+      }
+    }
+  }
+};
+
+// M: cells a thread may own.  p of the owned cells stays in registers too up to 4, u and Mi up to 6 (they
+// are in the fields otherwise, u updated in the wait for beta).
 template <int M, bool DIAG>
 __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
-  constexpr bool PREG = M <= 4, UREG = M <= 6, DISM = M <= 14;
+  constexpr bool PREG = M <= 4, UREG = M <= 6;
   constexpr int MG = M < 6 ? M : 6;  // rows whose loads from the fields are in flight together
   // Where the FP64 pipe bounds the iteration the products Di p and Mi r run on the integer pipes
-  // (dmul_int, the same bits): 14.8 -> 14.2 us at 700^2, 23.7 -> 22.5 at 777 x 1013 with jac_diag, 24.6 ->
-  // 23.5 at 1000^2.  Above 14 cells a thread its registers spill (26.2 -> 27.0 us at 1024^2).
-  constexpr bool EMU = M > 2 && M <= 14;
+  // (dmul_int, the same bits): 14.8 -> 14.2 us at 700^2; 7.2 -> 7.3 at 256^2, one cell a thread.
+  constexpr bool EMU = M > 2;
   __shared__ LoopState S;
   __shared__ Exchange X;
   __shared__ double sh_alpha, sh_beta;
@@ -337,7 +403,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
         pr[i] = pold[c];
       else
         sp[o] = pold[c];
-      if (DISM) sdi[o] = f.di[c];
+      sdi[o] = f.di[c];
       scx[o] = f.cx[c];
       scy[o] = f.cy[c];
       if (tx == tw - 1) scx[o + 1] = f.cx[c + 1];
@@ -345,13 +411,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
     }
   }
 
-  // scalars of the loop, in the first warp
-  const double goal = S.eps * S.initial_residual;
-  const uint64_t goal2 = emu::bits(goal > 1e-140 ? goal * goal * (1.0 + 1e-12) : INFINITY);
-  double rro = S.rro, inv_rro = 0.0, pw = S.pw, alpha_ = S.alpha, beta_ = S.beta, rrn = S.rrn;
-  const bool check_switch = S.check_switch != 0;
-  const int max_iters = S.max_iters;
-  bool error_due = false;
+  CgScalars C(S);  // in the first warp
   unsigned epoch = g.epoch;
   __syncthreads();
 
@@ -413,24 +473,15 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       bar_sync<2, PT>();
       double acc = 0.0;
       o = fresh(o0);
-      c = fresh(c0);
 #pragma unroll
       for (int i0 = 0; i0 < M; i0 += MG) {
         if (i0 >= mine) break;
-        double di[DISM ? 1 : MG];
-        if (!DISM) {
-#pragma unroll
-          for (int j = 0; j < MG; ++j)
-            if (i0 + j < mine) di[j] = __ldg(f.di + c + j * cstep);
-          c += MG * cstep;
-        }
 #pragma unroll
         for (int j = 0; j < MG; ++j, o += ostep) {
           const int i = i0 + j;
           if (i < M && i < mine) {
             const double pc = PREG ? pr[i] : sp[o];
-            const double dd = DISM ? sdi[o] : di[DISM ? 0 : j];
-            double wv = EMU ? dmul_int(dd, pc) : dd * pc;
+            double wv = EMU ? dmul_int(sdi[o], pc) : sdi[o] * pc;
             wv = fma(-scy[o + P], sp[o + P], wv);
             wv = fma(-scy[o], sp[o - P], wv);
             wv = fma(-scx[o + 1], sp[o + 1], wv);
@@ -443,17 +494,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       give(acc);
       poll();
     } else {
-      pw = exchange_sum(&X, inboxes(), epoch, ctas, cs, g.extra, rro, &inv_rro);
-      alpha_ = rro / pw;
-      if (lane == 0) {
-        sh_alpha = alpha_;
-        if (!finite_bits(alpha_)) {
-          S.status = EXIT_BREAKDOWN;
-          S.n_exit = n;
-          sh_status = EXIT_BREAKDOWN;
-        }
-        if (blockIdx.x == 0) g.a.rd.hist_a[n] = alpha_;
-      }
+      C.pw = exchange_sum(&X, inboxes(), epoch, ctas, cs, g.extra, C.rro, &C.inv_rro);
+      C.after_pw(&S, n, &sh_alpha, &sh_status, g.a.rd.hist_a);
     }
     ++epoch;
     __syncthreads();
@@ -532,28 +574,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       }
       if (!got) X.fail = 1;
     } else {
-      rrn = exchange_sum(&X, inboxes(), epoch, ctas, cs, g.extra, rro, nullptr);
-      // rrn / rro from the reciprocal of rro: one correction gives the correctly rounded quotient
-      // in the normal range (P. Markstein, IBM J. Res. Dev. 34(1), 1990); else the division
-      double b = rrn * inv_rro;
-      b = fma(fma(-b, rro, rrn), inv_rro, b);
-      const unsigned eb = expo(b), eo = expo(rro);
-      if (eb < 300u || eb > 1700u || eo < 300u || eo > 1700u) b = rrn / rro;
-      beta_ = b;
-      // without the square root when the outcome is plain: the error is far enough above the goal
-      // (goal2: its square with a margin; non-negative doubles order as their bits) and nothing
-      // else can stop the loop.  The error itself is then left to the launch's end.
-      error_due = !check_switch && n < max_iters && (emu::bits(rrn) & ~emu::SIGN) > goal2 && expo(rrn) < 2000u;
-      if (lane == 0) {
-        sh_beta = b;
-        if (!error_due) {
-          S.n = n;
-          loop_finish_iteration(&S, rrn);
-          sh_status = S.status;
-        }
-        if (blockIdx.x == 0) g.a.rd.hist_b[n] = b;
-      }
-      rro = rrn;
+      C.rrn = exchange_sum(&X, inboxes(), epoch, ctas, cs, g.extra, C.rro, nullptr);
+      C.after_rrn(&S, n, &sh_beta, &sh_status, g.a.rd.hist_b);
     }
     ++epoch;
     updated = true;
@@ -578,7 +600,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
     const int o = o0 + i * ostep, c = c0 + i * cstep;
     if (i < mine) {
       const double pc = sp[o];
-      double wv = (DISM ? sdi[o] : f.di[c]) * pc;
+      double wv = sdi[o] * pc;
       wv = fma(-scy[o + P], sp[o + P], wv);
       wv = fma(-scy[o], sp[o - P], wv);
       wv = fma(-scx[o + 1], sp[o + 1], wv);
@@ -591,20 +613,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
     }
   }
   if (blockIdx.x == 0 && t == 0) {
-    S.u_pending = 0;
-    S.pw = pw;
-    S.alpha = alpha_;
-    S.cg_calc_steps += done;
-    if (done > 0) {
-      S.rrn = rrn;
-      S.beta = beta_;
-      S.rro = rro;
-      S.p_pending = 1;
-      if (error_due) {
-        S.n = n;
-        S.error = S.old_error = sqrt(fabs(rrn));
-      }
-    }
+    C.store(S, n, done);
     *g.a.rd.st = S;
     *g.st_host = S;
   }
@@ -1055,19 +1064,393 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
   }
 }
 
+// ---- the FP64 CG loop on larger tiles ----------------------------------------------------------
+// k_persistent_cg's loop laid out as k_persistent_mix: p with its halo and r in shared memory, w and u in
+// tensor memory, the coefficients (and Mi) streamed from the fields through L2, a group of rows ahead.
+// 16 bytes a cell in shared memory take meshes of up to 2.1 million cells.  It runs where k_persistent_cg's
+// tiles do not fit (11 cells a thread, about 800K cells): at 700^2 it takes 14.5 us an iteration against
+// 14.2, at 777 x 1013 and 1000^2 it is even with larger tiles there (22.3 and 22.9 us), which spilled from
+// 14 cells a thread on (26.2 us at 1024^2 against 24.1).  Against the batched sweeps: 1000^2 22.9 us an
+// iteration against 42.1, 1024^2 24.1 / 42.4, 1100^2 with jac_diag 31.2 / 50.4, 1200^2 28.9 / 48.1, 1300 x
+// 1400 37.1 / 61.7.  The FP64 pipe's share is 17 us at 1000^2, 31 at 1300 x 1400.
+constexpr int WROWS = 32;  // rows a thread may own
+constexpr int WC = 4;      // rows handled together
+__device__ __forceinline__ void tmem_put(unsigned a, const double (&v)[4]) {
+  float w[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    w[2 * i] = __int_as_float(__double2loint(v[i]));
+    w[2 * i + 1] = __int_as_float(__double2hiint(v[i]));
+  }
+  tmem_put(a, w);
+}
+__device__ __forceinline__ void tmem_get(unsigned a, double (&v)[4]) {
+  float w[8];
+  tmem_get(a, w);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __hiloint2double(__float_as_int(w[2 * i + 1]), __float_as_int(w[2 * i]));
+}
+
+template <bool DIAG>
+__global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg_wide(PersistArgs g) {
+  __shared__ LoopState S;
+  __shared__ Exchange X;
+  __shared__ double sh_alpha, sh_beta;
+  __shared__ int sh_status;
+  __shared__ unsigned sh_tmem;
+  extern __shared__ __align__(16) double wsm[];
+  const Layout L = g.a.L;
+  const Fields& f = g.a.f;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const bool owner = wid != 0;
+  const int to = t - 32;
+  const int ctas = gridDim.x;
+  if (t == 0) {
+    S = *g.a.rd.st;
+    sh_status = S.status;
+    sh_beta = S.beta;
+    X.fail = 0;
+  }
+  __syncthreads();
+  if (sh_status != RUN) {
+    if (blockIdx.x == 0 && t == 0) *g.st_host = S;
+    return;
+  }
+  if (wid == 0) tmem_alloc(&sh_tmem);
+
+  const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
+  const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;
+  const int tw = min(g.pl.tw, L.nx - j0), th = min(g.pl.th, L.ny - k0);
+  const int P = g.pl.tw + 2, rows = g.pl.rows;
+  double* const sp = wsm;
+  double* const sr = wsm + (g.pl.th + 2) * P;
+
+  // the thread's column and rows y0 .. y0+mine-1
+  const int tx = owner ? to % g.pl.tw : 0, seg = owner ? to / g.pl.tw : 0, y0 = seg * rows;
+  const int mine = (owner && tx < tw && seg < g.pl.ry) ? max(0, min(rows, th - y0)) : 0;
+  const int o0 = (y0 + 1) * P + tx + 1, r0 = y0 * g.pl.tw + tx;
+  const int c0 = (int)L.at(j0 + tx + 1, k0 + y0 + 1);
+  const int ld = L.ld, rst = g.pl.tw;
+  const bool at_l = tx == 0 && j0 == 0, at_r = tx == tw - 1 && j0 + tw == L.nx;
+  const int i_first = y0 == 0 ? 0 : -1, i_last = (mine > 0 && y0 + mine == th) ? mine - 1 : -1;
+  const int i_b = k0 == 0 ? i_first : -1, i_t = k0 + th == L.ny ? i_last : -1;
+
+  const int hbox = 2 * (g.pl.th + g.pl.tw);
+  ulonglong2* const halo = g.box + (size_t)2 * ctas * SLOTS;
+  int ho[PH], hh[PH];
+  double hp[PH], hs[PH];
+  double* const src = DIAG ? f.z : f.r;
+  int n = S.n;
+  const double* const pold = (n & 1) ? f.p : f.p2;
+  bool upd = S.p_pending != 0;
+#pragma unroll
+  for (int q = 0; q < PH; ++q) {
+    const int h = to + q * PT;
+    ho[q] = -1;
+    hh[q] = 0;
+    hp[q] = hs[q] = 0.0;
+    int x = -1, y = h;
+    bool is = j0 > 0 && y < th;
+    if (h >= g.pl.th) x = tw, y = h - g.pl.th, is = j0 + tw < L.nx && y < th;
+    if (h >= 2 * g.pl.th) x = h - 2 * g.pl.th, y = -1, is = k0 > 0 && x < tw;
+    if (h >= 2 * g.pl.th + g.pl.tw) x = h - 2 * g.pl.th - g.pl.tw, y = th, is = k0 + th < L.ny && x < tw;
+    if (is && owner && h < hbox) {
+      ho[q] = (y + 1) * P + x + 1;
+      hh[q] = (int)blockIdx.x * hbox + h;
+      const int c = (int)L.at(j0 + x + 1, k0 + y + 1);
+      hp[q] = pold[c];
+      if (upd) hs[q] = src[c];
+    }
+  }
+  const int to_l = (mine && tx == 0 && j0 > 0) ? ((int)blockIdx.x - 1) * hbox + g.pl.th + y0 : -1;
+  const int to_r = (mine && tx == tw - 1 && j0 + tw < L.nx) ? ((int)blockIdx.x + 1) * hbox + y0 : -1;
+  const int rim_b = k0 > 0 ? i_first : -1, rim_t = k0 + th < L.ny ? i_last : -1;
+  const int to_b = ((int)blockIdx.x - g.pl.gx) * hbox + 2 * g.pl.th + g.pl.tw + tx;
+  const int to_t = ((int)blockIdx.x + g.pl.gx) * hbox + 2 * g.pl.th + tx;
+
+  __syncthreads();
+  // this thread's words of tensor memory: w (z between phases B and A with DIAG), then u
+  const unsigned tw_ = sh_tmem + ((unsigned)(wid & 3) << 21) + (unsigned)(wid >> 2) * 128u, td_ = tw_ + 2 * WROWS;
+  const int nch = owner ? (rows + WC - 1) / WC : 0;
+  {
+    int o = o0, rr = r0, c = c0;
+    for (int ch = 0; ch < nch; ++ch) {
+      double z[WC], d[WC];
+#pragma unroll
+      for (int j = 0; j < WC; ++j, o += P, rr += rst, c += ld) {
+        z[j] = d[j] = 0.0;
+        if (ch * WC + j < mine) {
+          const double p = pold[c];
+          sp[o] = p;
+          sr[rr] = f.r[c];
+          if (DIAG) z[j] = f.z[c];
+          d[j] = f.u[c];
+        }
+      }
+      tmem_put(tw_ + ch * 2 * WC, z);
+      tmem_put(td_ + ch * 2 * WC, d);
+    }
+    tmem_put_done();
+  }
+
+  CgScalars C(S);  // in the first warp
+  unsigned epoch = g.epoch;
+  __syncthreads();
+
+  auto give = [&](double v) {
+    const Fix s = warp_fix(v);
+    if (lane == 0) X.part[wid - 1] = s;
+    bar_arrive<1, PTHREADS>();
+  };
+  const int nwait = ctas > 1 ? ctas + g.extra : 0, nq = (nwait + 31) / 32;
+  auto poll = [&] {
+    if (wid > nq) return;
+    const int slot = (wid - 1) * 32 + lane;
+    const ulonglong2* in = g.box + ((size_t)(epoch & 1u) * ctas + blockIdx.x) * SLOTS + slot;
+    ulonglong2 x = make_ulonglong2(0ull, 0ull);
+    bool here = slot >= nwait;
+    for (unsigned tries = 0; !here && tries < PERSIST_POLL_LIMIT; ++tries) {
+      x = box_get(in);
+      here = box_is(x, epoch);
+    }
+    if (!here) X.fail = 1;
+    __syncwarp();
+    const Fix q = warp_fix(slot < nwait ? box_value(x) : 0.0);
+    if (lane == 0) X.inbox[wid - 1] = q;
+    bar_arrive(3, 32 * (nq + 1));
+  };
+  auto inboxes = [&] { return g.box + (size_t)(epoch & 1u) * ctas * SLOTS; };
+  struct Coefs {
+    double di[WC], cl[WC], cr[WC], ct[WC];  // Di, the left, right and upper face of a group of rows
+  } ka, kb;
+  auto load_coefs = [&](int ch, Coefs& k) {
+    int c = c0 + ch * WC * ld;
+#pragma unroll
+    for (int j = 0; j < WC; ++j, c += ld) {
+      k.di[j] = k.cl[j] = k.cr[j] = k.ct[j] = 0.0;
+      if (ch * WC + j < mine) {
+        k.di[j] = __ldg(f.di + c);
+        k.cl[j] = __ldg(f.cx + c);
+        k.cr[j] = __ldg(f.cx + c + 1);
+        k.ct[j] = __ldg(f.cy + c + ld);
+      }
+    }
+  };
+  load_coefs(0, ka);
+
+  int done = 0;
+  bool any = false;  // phase B of the last iteration ran
+  for (; done < g.max_run; ++done) {
+    // ---- phase A: p_n, w = A p_n, p.w ----
+    any = false;
+    if (owner) {
+      const double beta = sh_beta;
+      {
+        // the even iterations' p is what the loop leaves in the field p
+        double* const pf = (n & 1) ? nullptr : f.p;
+        int o = o0, rr = r0, c = c0;
+        for (int ch = 0; ch < nch; ++ch) {
+          double z[WC];
+          if (DIAG) tmem_get(tw_ + ch * 2 * WC, z);
+#pragma unroll
+          for (int j = 0; j < WC; ++j, o += P, rr += rst, c += ld) {
+            const int i = ch * WC + j;
+            if (i < mine) {
+              double p = sp[o];
+              if (upd) p = fma(beta, p, DIAG ? z[j] : sr[rr]);
+              sp[o] = p;
+              if (pf) pf[c] = p;
+              if (at_l) sp[o - 1] = p;
+              if (at_r) sp[o + 1] = p;
+              if (i == i_b) sp[o - P] = p;
+              if (i == i_t) sp[o + P] = p;
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < PH; ++q)
+        if (ho[q] >= 0) {
+          if (upd) hp[q] = fma(beta, hp[q], hs[q]);
+          sp[ho[q]] = hp[q];
+        }
+      bar_sync<2, PT>();
+      double dot = 0.0;
+      {
+        int o = o0;
+        double pb = 0.0, pc = 0.0, cyb = 0.0;
+        if (mine > 0) pb = sp[o - P], pc = sp[o], cyb = __ldg(f.cy + c0);
+        auto rows_of = [&](int ch, const Coefs& k) {
+          double w[WC];
+#pragma unroll
+          for (int j = 0; j < WC; ++j, o += P) {
+            w[j] = 0.0;
+            if (ch * WC + j < mine) {
+              const double pt = sp[o + P];
+              double a = dmul_int(k.di[j], pc);
+              a = fma(-k.ct[j], pt, a);
+              a = fma(-cyb, pb, a);
+              a = fma(-k.cr[j], sp[o + 1], a);
+              a = fma(-k.cl[j], sp[o - 1], a);
+              w[j] = a;
+              dot = fma(a, pc, dot);
+              pb = pc;
+              pc = pt;
+              cyb = k.ct[j];
+            }
+          }
+          tmem_put(tw_ + ch * 2 * WC, w);
+        };
+        // two groups of coefficients: the next one's loads are in flight while one is used
+        for (int ch = 0; ch < nch; ch += 2) {
+          if (ch + 1 < nch) load_coefs(ch + 1, kb);
+          rows_of(ch, ka);
+          if (ch + 1 < nch) {
+            if (ch + 2 < nch) load_coefs(ch + 2, ka);
+            rows_of(ch + 1, kb);
+          }
+        }
+        tmem_put_done();
+      }
+      give(dot);
+      poll();
+    } else {
+      C.pw = exchange_sum(&X, inboxes(), epoch, ctas, 1, g.extra, C.rro, &C.inv_rro);
+      C.after_pw(&S, n, &sh_alpha, &sh_status, g.a.rd.hist_a);
+    }
+    ++epoch;
+    __syncthreads();
+    if (X.fail || sh_status != RUN) break;
+    // ---- phase B: r -= alpha w, z = Mi r, r.z; the rim to the neighbours; d += alpha p_n ----
+    if (owner) {
+      const double alpha = sh_alpha;
+      double dot = 0.0;
+      {
+        int rr = r0, c = c0;
+        for (int ch = 0; ch < nch; ++ch) {
+          double w[WC], mi[WC];
+          if (DIAG) {
+#pragma unroll
+            for (int j = 0; j < WC; ++j, c += ld)
+              mi[j] = ch * WC + j < mine ? __ldg(f.mi + c) : 0.0;
+          }
+          tmem_get(tw_ + ch * 2 * WC, w);
+#pragma unroll
+          for (int j = 0; j < WC; ++j, rr += rst) {
+            const int i = ch * WC + j;
+            if (i < mine) {
+              const double rv = fma(-alpha, w[j], sr[rr]);
+              sr[rr] = rv;
+              double zv = rv;
+              if (DIAG) {
+                zv = dmul_int(mi[j], rv);
+                w[j] = zv;
+              }
+              dot = fma(rv, zv, dot);
+              if (to_l >= 0) box_put(halo + to_l + i, zv, epoch);
+              if (to_r >= 0) box_put(halo + to_r + i, zv, epoch);
+              if (i == rim_b) box_put(halo + to_b, zv, epoch);
+              if (i == rim_t) box_put(halo + to_t, zv, epoch);
+            }
+          }
+          if (DIAG) tmem_put(tw_ + ch * 2 * WC, w);
+        }
+      }
+      give(dot);
+      load_coefs(0, ka);  // of the next phase A
+      poll();
+      {
+        int o = o0;
+        for (int ch = 0; ch < nch; ++ch) {
+          double d[WC];
+          tmem_get(td_ + ch * 2 * WC, d);
+#pragma unroll
+          for (int j = 0; j < WC; ++j, o += P)
+            if (ch * WC + j < mine) d[j] = fma(alpha, sp[o], d[j]);
+          tmem_put(td_ + ch * 2 * WC, d);
+        }
+        tmem_put_done();
+      }
+      bool got = false;
+      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+        got = true;
+#pragma unroll
+        for (int q = 0; q < PH; ++q)
+          if (ho[q] >= 0) {
+            const ulonglong2 x = box_get(halo + hh[q]);
+            got = got && box_is(x, epoch);
+            hs[q] = box_value(x);
+          }
+      }
+      if (!got) X.fail = 1;
+    } else {
+      C.rrn = exchange_sum(&X, inboxes(), epoch, ctas, 1, g.extra, C.rro, nullptr);
+      C.after_rrn(&S, n, &sh_beta, &sh_status, g.a.rd.hist_b);
+    }
+    ++epoch;
+    ++n;
+    upd = true;
+    any = true;
+    __syncthreads();
+    if (X.fail || sh_status != RUN) {
+      ++done;
+      break;
+    }
+  }
+  const bool failed = X.fail != 0;
+  // the fields and the state as the loop's kernels leave them
+  double* const pout = ((any ? n - 1 : n) & 1) ? f.p2 : f.p;
+  {
+    int o = o0, rr = r0, c = c0;
+    for (int ch = 0; ch < (failed ? 0 : nch); ++ch) {
+      double z[WC], d[WC];
+      tmem_get(tw_ + ch * 2 * WC, z);
+      tmem_get(td_ + ch * 2 * WC, d);
+#pragma unroll
+      for (int j = 0; j < WC; ++j, o += P, rr += rst, c += ld) {
+        if (ch * WC + j < mine) {
+          pout[c] = sp[o];
+          f.r[c] = sr[rr];
+          f.u[c] = d[j];
+          if (!DIAG || !any) {
+            f.w[c] = z[j];
+          } else {  // z took w's place: w = A p_n formed again
+            f.z[c] = z[j];
+            double a = dmul_int(f.di[c], sp[o]);
+            a = fma(-f.cy[c + ld], sp[o + P], a);
+            a = fma(-f.cy[c], sp[o - P], a);
+            a = fma(-f.cx[c + 1], sp[o + 1], a);
+            a = fma(-f.cx[c], sp[o - 1], a);
+            f.w[c] = a;
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();  // every warp is done with tensor memory
+  if (wid == 0) tmem_free(sh_tmem);
+  if (failed) {
+    if (t == 0) g.a.rd.st->status = g.st_host->status = EXIT_TIMEOUT;
+    return;
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    C.store(S, n, done);
+    *g.a.rd.st = S;
+    *g.st_host = S;
+  }
+}
+
 using PersistKernel = void (*)(PersistArgs);
 struct PersistVariant {
   int m;
   PersistKernel k[2];  // without / with jac_diag
 };
 #define PERSIST_VARIANT(M) {M, {k_persistent_cg<M, false>, k_persistent_cg<M, true>}}
-const PersistVariant kVariants[] = {PERSIST_VARIANT(1), PERSIST_VARIANT(2),  PERSIST_VARIANT(4),  PERSIST_VARIANT(6),
-                                    PERSIST_VARIANT(8), PERSIST_VARIANT(11), PERSIST_VARIANT(14), PERSIST_VARIANT(18)};
+const PersistVariant kVariants[] = {PERSIST_VARIANT(1), PERSIST_VARIANT(2), PERSIST_VARIANT(4),
+                                    PERSIST_VARIANT(6), PERSIST_VARIANT(8), PERSIST_VARIANT(11)};
 
-// p, cx, cy and, up to 14 cells a thread, Di
-size_t plan_smem(const PersistPlan& p) {
-  return (size_t)(kVariants[p.variant].m <= 14 ? 4 : 3) * (p.th + 2) * (p.tw + 2) * sizeof(double);
-}
+// p, cx, cy and Di
+size_t plan_smem(const PersistPlan& p) { return (size_t)4 * (p.th + 2) * (p.tw + 2) * sizeof(double); }
 
 // A launch of a plan: cooperative (its CTAs wait for one another), in clusters.
 struct PersistLaunch {
@@ -1159,38 +1542,14 @@ bool persist_plan(int nx, int ny, const int (&clusters)[5], PersistPlan* out) {
   return found;
 }
 
-// Plans the mesh for the current device; false if it does not fit on chip.
-bool persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
-  int clusters[5];
-  const int diag = precond == 2 ? 1 : 0;
-  const void* k0 = (const void*)kVariants[0].k[diag];
-  for (int i = 0; i < 5; ++i) clusters[i] = persist_clusters(k0, 1 << i, PERSIST_SMEM_MAX);
-  if (!persist_plan(nx, ny, clusters, out)) return false;
-  const int n = persist_clusters((const void*)kVariants[out->variant].k[diag], out->cs, plan_smem(*out));
-  return n * out->cs >= persist_ctas(*out);
-}
-
-cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch, void* box,
-                                 LoopState* st_host, cudaStream_t s, int extra) {
-  PersistArgs g{a, p, max_run, epoch, static_cast<ulonglong2*>(box), st_host, extra};
-  void* args[] = {&g};
-  PersistLaunch l(persist_ctas(p), p.cs, plan_smem(p), s);
-  ++launch_counter();
-  return cudaLaunchKernelExC(&l.cfg, (const void*)kVariants[p.variant].k[a.precond == 2 ? 1 : 0], args);
-}
+constexpr int WIDE = 100;  // PersistPlan::variant of k_persistent_cg_wide
 
 namespace {
-
-using MixPersistKernel = void (*)(MixPersistArgs);
-const MixPersistKernel kMixKernels[2] = {k_persistent_mix<false>, k_persistent_mix<true>};  // without / with jac_diag
-size_t mix_plan_smem(const PersistPlan& p) {
-  return ((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw) * sizeof(float);
-}
-
 // The tiling with the fewest cycles an iteration (16 a row of a warp, 3200 for each of the two
 // sums' exchange when there is more than one tile); tiles at least 32 columns wide, where
 // the mesh is, for the sake of the coefficients' loads.
-bool mix_plan(int nx, int ny, int ctas, PersistPlan* out) {
+template <typename F>
+bool rows_plan(int nx, int ny, int ctas, int max_rows, F&& smem, PersistPlan* out) {
   double best = 0.0;
   bool found = false;
   if (ctas > PERSIST_MAX_CTAS) ctas = PERSIST_MAX_CTAS;
@@ -1211,7 +1570,7 @@ bool mix_plan(int nx, int ny, int ctas, PersistPlan* out) {
       p.rows = (p.th + p.ry - 1) / p.ry;
       p.variant = 0;
       const int halo = 2 * (p.tw + p.th);
-      if (p.rows > MROWS || halo > PH * PT || mix_plan_smem(p) > PERSIST_SMEM_MAX) continue;
+      if (p.rows > max_rows || halo > PH * PT || smem(p) > PERSIST_SMEM_MAX) continue;
       const double cost =
           (double)((p.ry * tw + 31) / 32) * p.rows * 16.0 + 0.5 * halo + (p.gx * p.gy > 1 ? 6400.0 : 0.0);
       if (!found || cost < best) {
@@ -1223,13 +1582,53 @@ bool mix_plan(int nx, int ny, int ctas, PersistPlan* out) {
   }
   return found;
 }
+}  // namespace
+
+const PersistKernel kWideKernels[2] = {k_persistent_cg_wide<false>, k_persistent_cg_wide<true>};
+size_t wide_plan_smem(const PersistPlan& p) {
+  return ((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw) * sizeof(double);
+}
+const void* cg_kernel(const PersistPlan& p, int precond) {
+  const int diag = precond == 2 ? 1 : 0;
+  return p.variant == WIDE ? (const void*)kWideKernels[diag] : (const void*)kVariants[p.variant].k[diag];
+}
+size_t cg_smem(const PersistPlan& p) { return p.variant == WIDE ? wide_plan_smem(p) : plan_smem(p); }
+
+// Plans the mesh for the current device; false if it does not fit on chip.
+bool persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
+  int clusters[5];
+  const void* k0 = (const void*)kVariants[0].k[precond == 2 ? 1 : 0];
+  for (int i = 0; i < 5; ++i) clusters[i] = persist_clusters(k0, 1 << i, PERSIST_SMEM_MAX);
+  if (!persist_plan(nx, ny, clusters, out)) {
+    if (!rows_plan(nx, ny, clusters[0], WROWS, wide_plan_smem, out)) return false;
+    out->variant = WIDE;
+  }
+  return persist_clusters(cg_kernel(*out, precond), out->cs, cg_smem(*out)) * out->cs >= persist_ctas(*out);
+}
+
+cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch, void* box,
+                                 LoopState* st_host, cudaStream_t s, int extra) {
+  PersistArgs g{a, p, max_run, epoch, static_cast<ulonglong2*>(box), st_host, extra};
+  void* args[] = {&g};
+  PersistLaunch l(persist_ctas(p), p.cs, cg_smem(p), s);
+  ++launch_counter();
+  return cudaLaunchKernelExC(&l.cfg, cg_kernel(p, a.precond), args);
+}
+
+namespace {
+
+using MixPersistKernel = void (*)(MixPersistArgs);
+const MixPersistKernel kMixKernels[2] = {k_persistent_mix<false>, k_persistent_mix<true>};  // without / with jac_diag
+size_t mix_plan_smem(const PersistPlan& p) {
+  return ((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw) * sizeof(float);
+}
 
 }  // namespace
 
 bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const int diag = precond == 2 ? 1 : 0;
   const int ctas = persist_clusters((const void*)kMixKernels[diag], 1, PERSIST_SMEM_MAX);
-  if (!mix_plan(nx, ny, ctas, out)) return false;
+  if (!rows_plan(nx, ny, ctas, MROWS, mix_plan_smem, out)) return false;
   return persist_clusters((const void*)kMixKernels[diag], 1, mix_plan_smem(*out)) >= persist_ctas(*out);
 }
 
