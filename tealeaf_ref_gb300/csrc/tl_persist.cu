@@ -625,11 +625,16 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
 // here: 128 words a thread); the operator's coefficients stay in the fields, which the L2 cache
 // (and, for small tiles, the SM's own) holds.  8 bytes a cell in shared memory take meshes of up to
 // 4.3 million cells, 2048^2 among them.  A thread owns consecutive rows of a column, so a row's
-// upper face is the next row's lower one; the coefficients of the next group of rows are in flight
-// while one is used.  Time per iteration, the replacements included, against the sweeps' two
-// launches: 512^2 10.3 against 25.0 us, 1000^2 13.4 / 34.0, 1500 x 1999 24.5 / 48.0, 2048^2 32.4 /
-// 50.4, with jac_diag 37.1 / 55.5; with w in registers and d in its field 2048^2 took 46.7 us.  The
-// sums' exchange bounds it up to about 1000^2, the coefficients' way from L2 above.
+// upper face is the next row's lower one; rows go in groups of MC, whose loads precede its stores (the
+// compiler cannot tell the arrays of shared memory apart, and a load behind a store waits for it), and the
+// coefficients of the next group are in flight while one is used.  d is updated before the wait for beta's
+// partials, in the time they take; the rim's columns are sent by whole warps.  Time per iteration, the
+// replacements included, against the sweeps' two launches: 512^2 10.0 against 25.0 us, 1000^2 12.3 / 34.0,
+// 1500 x 1999 17.7 / 48.0, 2048^2 21.3 / 50.4, with jac_diag 25.4 / 55.5.  Row by row, with a test of
+// the row, a test of the mesh's walls and a store to the neighbour's box in each, 2048^2 took 32.4 us and
+// 1000^2 13.2: the walls are mirrored by the neighbours' offsets, and what has no row works on a cell of
+// zeros.  The sums' exchange, 6 us, bounds it up to about 1000^2, the coefficients' way from L2 (13 bytes
+// a cell) above; taking the right face from the next lane instead of loading it gave nothing.
 // The dot products are the sweeps': Dot2 per thread, then exact integers.
 struct MixPersistArgs {
   MixFields m;
@@ -674,7 +679,6 @@ __device__ __forceinline__ Fix warp_fix(const Dot2& d) {
 // 32 lanes of its number modulo 4; the four warps of a quarter take 128 columns each, 2 MROWS words a
 // thread.
 constexpr int MROWS = 64;  // rows a thread may own
-constexpr int MC = 8;      // rows handled together
 __device__ __forceinline__ void tmem_alloc(unsigned* at) {  // a whole warp
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                    (unsigned)__cvta_generic_to_shared(at))
@@ -690,6 +694,15 @@ __device__ __forceinline__ void tmem_put(unsigned a, const float (&v)[8]) {
                "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
                : "memory");
 }
+__device__ __forceinline__ void tmem_put(unsigned a, const float (&v)[4]) {
+  __syncwarp();
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_put(unsigned a, const float (&v)[2]) {
+  __syncwarp();
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(a), "f"(v[0]), "f"(v[1]) : "memory");
+}
 // before the words are read again
 __device__ __forceinline__ void tmem_put_done() {
   __syncwarp();
@@ -703,7 +716,23 @@ __device__ __forceinline__ void tmem_get(unsigned a, float (&v)[8]) {
                : "memory");
 }
 
-template <bool DIAG>
+__device__ __forceinline__ void tmem_get(unsigned a, float (&v)[4]) {
+  __syncwarp();
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+               : "r"(a)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_get(unsigned a, float (&v)[2]) {
+  __syncwarp();
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];\n tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0]), "=f"(v[1])
+               : "r"(a)
+               : "memory");
+}
+
+// MC: rows handled together.
+template <bool DIAG, int MC>
 __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g) {
   __shared__ MixState S;
   __shared__ Exchange X;
@@ -730,18 +759,28 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
   const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
   const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;
   const int tw = min(g.pl.tw, L.nx - j0), th = min(g.pl.th, L.ny - k0);
-  const int P = g.pl.tw + 2, rows = g.pl.rows;
+  const int P = g.pl.tw + 2;
   float* const sp = fsm;
   float* const sr = fsm + (g.pl.th + 2) * P;
 
-  // the thread's column and rows y0 .. y0+mine-1
-  const int tx = owner ? to % g.pl.tw : 0, seg = owner ? to / g.pl.tw : 0, y0 = seg * rows;
-  const int mine = (owner && tx < tw && seg < g.pl.ry) ? max(0, min(rows, th - y0)) : 0;
-  const int o0 = (y0 + 1) * P + tx + 1, r0 = y0 * g.pl.tw + tx;
-  const int c0 = (int)L.at(j0 + tx + 1, k0 + y0 + 1);
-  const int ld = L.ld, rst = g.pl.tw;
+  // the thread's column and rows y0 .. y0+mine-1: the rows split evenly, so that two threads' differ by
+  // one at most.  The lanes left over of a warp that owns cells, and the rows left over of the last group of
+  // rows, work on a cell of zeros past the tile: no row is a branch
+  const int tx = owner ? to % g.pl.tw : 0, seg = owner ? to / g.pl.tw : 0;
+  const int q_ = th / g.pl.ry, rem = th - q_ * g.pl.ry;
+  const int mine = (owner && tx < tw && seg < g.pl.ry) ? q_ + (seg < rem) : 0, y0 = seg * q_ + min(seg, rem);
+  const int own = mine ? mine : q_ + (rem > 0);
+  const bool warp_owns = __any_sync(0xffffffffu, mine > 0);
+  const int nfull = warp_owns ? (int)__reduce_min_sync(0xffffffffu, (unsigned)own) / MC : 0;  // groups of MC rows
+  const int nch = warp_owns ? ((int)__reduce_max_sync(0xffffffffu, (unsigned)own) + MC - 1) / MC : 0;
+  const int rz = g.pl.th * g.pl.tw, oz = (g.pl.th + 2) * P + rz;  // the cell of zeros, from sr and from sp
+  const int r0 = mine ? y0 * g.pl.tw + tx : rz, o0 = mine ? (y0 + 1) * P + tx + 1 : oz;
+  const int c0 = mine ? (int)L.at(j0 + tx + 1, k0 + y0 + 1) : (int)L.at(j0 + 1, k0 + 1);
+  const int ld = L.ld, os = mine ? P : 0, rs = mine ? g.pl.tw : 0, cs = mine ? ld : 0;
   const bool at_l = tx == 0 && j0 == 0, at_r = tx == tw - 1 && j0 + tw == L.nx;
-  const int i_first = y0 == 0 ? 0 : -1, i_last = (mine > 0 && y0 + mine == th) ? mine - 1 : -1;
+  // the neighbours' offsets: a reflecting wall mirrors the cell
+  const int lo = (at_l || !mine) ? 0 : -1, ro = (at_r || !mine) ? 0 : 1;
+  const int i_first = (mine > 0 && y0 == 0) ? 0 : -1, i_last = (mine > 0 && y0 + mine == th) ? mine - 1 : -1;
   const int i_b = k0 == 0 ? i_first : -1, i_t = k0 + th == L.ny ? i_last : -1;
 
   const int hbox = 2 * (g.pl.th + g.pl.tw);
@@ -780,7 +819,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
   __syncthreads();
   // this thread's words of tensor memory: w (z between phases B and A with DIAG), then d
   const unsigned tw_ = sh_tmem + ((unsigned)(wid & 3) << 21) + (unsigned)(wid >> 2) * (2 * MROWS), td_ = tw_ + MROWS;
-  const int nch = owner ? (rows + MC - 1) / MC : 0;
+  if (t == 0) sp[oz] = 0.f;
   {
     int o = o0, rr = r0, c = c0;
     // the deferred d += alpha p of an earlier step (its p is the one read here)
@@ -789,7 +828,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
     for (int ch = 0; ch < nch; ++ch) {
       float z[MC], d[MC];
 #pragma unroll
-      for (int j = 0; j < MC; ++j, o += P, rr += rst, c += ld) {
+      for (int j = 0; j < MC; ++j, o += os, rr += rs, c += cs) {
         z[j] = d[j] = 0.f;
         if (ch * MC + j < mine) {
           const float p = pold[c];
@@ -836,19 +875,30 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
   struct Coefs {
     float di[MC], cl[MC], cr[MC], ct[MC];  // Di, the left, right and upper face of a group of rows
   } ka, kb;
-  auto load_coefs = [&](int ch, Coefs& k) {
-    int c = c0 + ch * MC * ld;
+  const std::true_type full;
+  const std::false_type part;
+  auto load_group = [&](int ch, Coefs& k, auto f_) {
+    const int left = own - ch * MC, c1 = decltype(f_)::value || left > 0 ? c0 + ch * MC * cs : c0;
+    const float *pd = f.di + c1, *px = f.cx + c1, *py = f.cy + c1 + ld;
 #pragma unroll
-    for (int j = 0; j < MC; ++j, c += ld) {
-      k.di[j] = k.cl[j] = k.cr[j] = k.ct[j] = 0.f;
-      if (ch * MC + j < mine) {
-        k.di[j] = __ldg(f.di + c);
-        k.cl[j] = __ldg(f.cx + c);
-        k.cr[j] = __ldg(f.cx + c + 1);
-        k.ct[j] = __ldg(f.cy + c + ld);
-      }
+    for (int j = 0; j < MC; ++j) {
+      k.di[j] = __ldg(pd);
+      k.cl[j] = __ldg(px);
+      k.cr[j] = __ldg(px + 1);
+      k.ct[j] = __ldg(py);
+      if (decltype(f_)::value || j + 1 < left) pd += cs, px += cs, py += cs;
     }
   };
+  auto load_coefs = [&](int ch, Coefs& k) {
+    if (ch < nfull) load_group(ch, k, full);
+    else if (ch < nch) load_group(ch, k, part);
+  };
+  // a sweep over the thread's groups of rows
+  auto sweep = [&](auto&& group) {
+    for (int ch = 0; ch < nfull; ++ch) group(ch, full);
+    if (nfull < nch) group(nfull, part);
+  };
+
   load_coefs(0, ka);
 
   bool any = false;
@@ -856,26 +906,27 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
     // ---- phase A: p_n, w = A p_n, p.w ----
     if (owner) {
       const float beta = sh_beta;
-      {
-        int o = o0, rr = r0;
-        for (int ch = 0; ch < nch; ++ch) {
-          float z[MC];
+      if (upd) {
+        sweep([&](int ch, auto f_) {
+          // a group's loads before its stores, which the compiler cannot tell apart
+          const int o = o0 + ch * MC * os, rr = r0 + ch * MC * rs, left = own - ch * MC;
+          float p[MC], z[MC];
+#pragma unroll
+          for (int j = 0; j < MC; ++j) {
+            const bool in = decltype(f_)::value || j < left;
+            p[j] = sp[in ? o + j * os : oz];
+            if (!DIAG) z[j] = sr[in ? rr + j * rs : rz];
+          }
           if (DIAG) tmem_get(tw_ + ch * MC, z);
 #pragma unroll
-          for (int j = 0; j < MC; ++j, o += P, rr += rst) {
-            const int i = ch * MC + j;
-            if (i < mine) {
-              float p = sp[o];
-              if (upd) p = fmaf(beta, p, DIAG ? z[j] : sr[rr]);
-              sp[o] = p;
-              if (at_l) sp[o - 1] = p;
-              if (at_r) sp[o + 1] = p;
-              if (i == i_b) sp[o - P] = p;
-              if (i == i_t) sp[o + P] = p;
-            }
+          for (int j = 0; j < MC; ++j) {
+            const bool in = decltype(f_)::value || j < left;
+            sp[in ? o + j * os : oz] = fmaf(beta, p[j], z[j]);
           }
-        }
+        });
       }
+      if (i_b >= 0) sp[o0 - P] = sp[o0];
+      if (i_t >= 0) sp[o0 + mine * P] = sp[o0 + (mine - 1) * P];
 #pragma unroll
       for (int q = 0; q < PH; ++q)
         if (ho[q] >= 0) {
@@ -887,36 +938,39 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
       {
         int o = o0;
         float pb = 0.f, pc = 0.f, cyb = 0.f;
-        if (mine > 0) pb = sp[o - P], pc = sp[o], cyb = __ldg(f.cy + c0);
-        auto rows_of = [&](int ch, const Coefs& k) {
+        if (nch > 0) pb = sp[o - os], pc = sp[o], cyb = __ldg(f.cy + c0);
+        auto rows_of = [&](int ch, const Coefs& k, auto f_) {
+          const int left = own - ch * MC;
           float w[MC];
 #pragma unroll
-          for (int j = 0; j < MC; ++j, o += P) {
-            w[j] = 0.f;
-            if (ch * MC + j < mine) {
-              const float pt = sp[o + P];
-              float a = k.di[j] * pc;
-              a = fmaf(-k.ct[j], pt, a);
-              a = fmaf(-cyb, pb, a);
-              a = fmaf(-k.cr[j], sp[o + 1], a);
-              a = fmaf(-k.cl[j], sp[o - 1], a);
-              w[j] = a;
-              dot.add(a, pc);
-              pb = pc;
-              pc = pt;
-              cyb = k.ct[j];
-            }
+          for (int j = 0; j < MC; ++j) {
+            const bool in = decltype(f_)::value || j < left;
+            if (!in) pb = pc = 0.f;
+            const float pt = sp[in ? o + os : oz];
+            float a = k.di[j] * pc;
+            a = fmaf(-k.ct[j], pt, a);
+            a = fmaf(-cyb, pb, a);
+            a = fmaf(-k.cr[j], sp[in ? o + ro : oz], a);
+            a = fmaf(-k.cl[j], sp[in ? o + lo : oz], a);
+            w[j] = a;
+            dot.add(a, pc);
+            pb = pc;
+            pc = pt;
+            cyb = k.ct[j];
+            o += os;
           }
           tmem_put(tw_ + ch * MC, w);
         };
+        auto rows = [&](int ch, const Coefs& k) {
+          if (ch < nfull) rows_of(ch, k, full);
+          else if (ch < nch) rows_of(ch, k, part);
+        };
         // two groups of coefficients: the next one's loads are in flight while one is used
         for (int ch = 0; ch < nch; ch += 2) {
-          if (ch + 1 < nch) load_coefs(ch + 1, kb);
-          rows_of(ch, ka);
-          if (ch + 1 < nch) {
-            if (ch + 2 < nch) load_coefs(ch + 2, ka);
-            rows_of(ch + 1, kb);
-          }
+          load_coefs(ch + 1, kb);
+          rows(ch, ka);
+          load_coefs(ch + 2, ka);
+          rows(ch + 1, kb);
         }
         tmem_put_done();
       }
@@ -938,52 +992,58 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
     if (owner) {
       const float alpha = sh_alpha;
       Dot2 dot;
-      {
-        int rr = r0, c = c0;
-        for (int ch = 0; ch < nch; ++ch) {
-          float w[MC], mi[MC];
-          if (DIAG) {
+      sweep([&](int ch, auto f_) {
+        const int rr = r0 + ch * MC * rs, left = own - ch * MC;
+        float w[MC], r[MC], mi[MC];
 #pragma unroll
-            for (int j = 0; j < MC; ++j, c += ld)
-              mi[j] = ch * MC + j < mine ? __ldg(f.mi + c) : 0.f;
-          }
-          tmem_get(tw_ + ch * MC, w);
-#pragma unroll
-          for (int j = 0; j < MC; ++j, rr += rst) {
-            const int i = ch * MC + j;
-            if (i < mine) {
-              const float rv = fmaf(-alpha, w[j], sr[rr]);
-              sr[rr] = rv;
-              float zv = rv;
-              if (DIAG) {
-                zv = mi[j] * rv;
-                w[j] = zv;
-              }
-              dot.add(rv, zv);
-              if (to_l >= 0) fbox_put(halo + to_l + i, zv, epoch);
-              if (to_r >= 0) fbox_put(halo + to_r + i, zv, epoch);
-              if (i == rim_b) fbox_put(halo + to_b, zv, epoch);
-              if (i == rim_t) fbox_put(halo + to_t, zv, epoch);
-            }
-          }
-          if (DIAG) tmem_put(tw_ + ch * MC, w);
+        for (int j = 0; j < MC; ++j) {
+          const bool in = decltype(f_)::value || j < left;
+          r[j] = sr[in ? rr + j * rs : rz];
+          if (DIAG) mi[j] = __ldg(f.mi + (in ? c0 + (ch * MC + j) * cs : c0));
         }
-      }
+        tmem_get(tw_ + ch * MC, w);
+#pragma unroll
+        for (int j = 0; j < MC; ++j) {
+          r[j] = fmaf(-alpha, w[j], r[j]);
+          sr[decltype(f_)::value || j < left ? rr + j * rs : rz] = r[j];
+          w[j] = DIAG ? mi[j] * r[j] : r[j];
+          dot.add(r[j], w[j]);
+        }
+        if (DIAG) tmem_put(tw_ + ch * MC, w);
+      });
+      // the rim: a column's rows are its owner's, and the whole warp sends them
+      auto rim = [&](int rr, int c) {
+        const float r = sr[rr];
+        return DIAG ? __ldg(f.mi + c) * r : r;
+      };
+      if (rim_b >= 0) fbox_put(halo + to_b, rim(r0 + rim_b * rs, c0 + rim_b * cs), epoch);
+      if (rim_t >= 0) fbox_put(halo + to_t, rim(r0 + rim_t * rs, c0 + rim_t * cs), epoch);
+      __syncwarp();
+      auto columns = [&](int to_) {
+        for (unsigned m = __ballot_sync(0xffffffffu, to_ >= 0); m; m &= m - 1) {
+          const int l = __ffs(m) - 1;
+          const int h = __shfl_sync(0xffffffffu, to_, l), r1 = __shfl_sync(0xffffffffu, r0, l),
+                    c1 = __shfl_sync(0xffffffffu, c0, l), have = __shfl_sync(0xffffffffu, mine, l);
+          for (int i = lane; i < have; i += 32) fbox_put(halo + h + i, rim(r1 + i * g.pl.tw, c1 + i * ld), epoch);
+        }
+      };
+      columns(to_l);
+      columns(to_r);
       give(dot);
+      // d += alpha p_n while the sum is under way
+      sweep([&](int ch, auto f_) {
+        const int o = o0 + ch * MC * os, left = own - ch * MC;
+        float d[MC], p[MC];
+#pragma unroll
+        for (int j = 0; j < MC; ++j) p[j] = sp[decltype(f_)::value || j < left ? o + j * os : oz];
+        tmem_get(td_ + ch * MC, d);
+#pragma unroll
+        for (int j = 0; j < MC; ++j) d[j] = fmaf(alpha, p[j], d[j]);
+        tmem_put(td_ + ch * MC, d);
+      });
+      tmem_put_done();
       load_coefs(0, ka);  // of the next phase A
       poll();
-      {
-        int o = o0;
-        for (int ch = 0; ch < nch; ++ch) {
-          float d[MC];
-          tmem_get(td_ + ch * MC, d);
-#pragma unroll
-          for (int j = 0; j < MC; ++j, o += P)
-            if (ch * MC + j < mine) d[j] = fmaf(alpha, sp[o], d[j]);
-          tmem_put(td_ + ch * MC, d);
-        }
-        tmem_put_done();
-      }
       bool got = false;
       for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
         got = true;
@@ -1032,7 +1092,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
       if (DIAG) tmem_get(tw_ + ch * MC, z);
       tmem_get(td_ + ch * MC, d);
 #pragma unroll
-      for (int j = 0; j < MC; ++j, o += P, rr += rst, c += ld) {
+      for (int j = 0; j < MC; ++j, o += os, rr += rs, c += cs) {
         if (ch * MC + j < mine) {
           pout[c] = sp[o];
           f.r[c] = sr[rr];
@@ -1618,18 +1678,23 @@ cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int ma
 namespace {
 
 using MixPersistKernel = void (*)(MixPersistArgs);
-const MixPersistKernel kMixKernels[2] = {k_persistent_mix<false>, k_persistent_mix<true>};  // without / with jac_diag
+const MixPersistKernel kMixKernels[2][2] = {{k_persistent_mix<false, 2>, k_persistent_mix<true, 2>},   // without / with
+                                            {k_persistent_mix<false, 4>, k_persistent_mix<true, 4>}};  // jac_diag
+// Groups of 4 rows, of 2 where a thread owns 6 at most (to about 700^2): 200 x 300 11.2 us against 11.5, 300
+// x 400 10.6 / 10.7, 700^2 10.8 / 10.8; 900 x 950 11.9 / 11.6, 1300^2 15.3 / 14.5, 2048^2 22.6 / 21.3.
+// Groups of 8 spill: 13.0 us at 200 x 300, 22.5 at 2048^2.
+const void* mix_kernel(const PersistPlan& p, bool diag) { return (const void*)kMixKernels[p.rows > 6][diag]; }
 size_t mix_plan_smem(const PersistPlan& p) {
-  return ((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw) * sizeof(float);
+  return ((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw + 1) * sizeof(float);
 }
 
 }  // namespace
 
 bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
-  const int diag = precond == 2 ? 1 : 0;
-  const int ctas = persist_clusters((const void*)kMixKernels[diag], 1, PERSIST_SMEM_MAX);
+  const bool diag = precond == 2;
+  const int ctas = persist_clusters((const void*)kMixKernels[1][diag], 1, PERSIST_SMEM_MAX);
   if (!rows_plan(nx, ny, ctas, MROWS, mix_plan_smem, out)) return false;
-  return persist_clusters((const void*)kMixKernels[diag], 1, mix_plan_smem(*out)) >= persist_ctas(*out);
+  return persist_clusters(mix_kernel(*out, diag), 1, mix_plan_smem(*out)) >= persist_ctas(*out);
 }
 
 cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState* ms, const PersistPlan& p, int max_run,
@@ -1638,7 +1703,7 @@ cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState*
   void* args[] = {&g};
   PersistLaunch l(persist_ctas(p), p.cs, mix_plan_smem(p), s);
   ++launch_counter();
-  return cudaLaunchKernelExC(&l.cfg, (const void*)kMixKernels[m.mi ? 1 : 0], args);
+  return cudaLaunchKernelExC(&l.cfg, mix_kernel(p, m.mi != nullptr), args);
 }
 
 

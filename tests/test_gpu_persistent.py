@@ -41,7 +41,8 @@ def test_persistent_iterations_match_the_sweeps(size, case, monkeypatch):
         assert np.max(np.abs(f1[f] - f0[f])) <= 1e-11 * np.max(np.abs(f0[f])), f
 
 
-MIXED_SIZES = [(20, 20), (1, 3000), (3000, 1), (301, 199), (511, 513), (1000, 1000), (1499, 1999), (2048, 2048)]
+MIXED_SIZES = [(20, 20), (1, 3000), (3000, 1), (1, 40000), (40000, 1), (301, 199), (511, 513), (701, 699), (745, 753),
+               (1000, 1000), (2047, 1021), (1499, 1999), (2048, 2048)]
 
 
 @pytest.mark.parametrize("case", [dict(), dict(precond="jac_diag", reflective=True)], ids=["none", "diag-reflective"])
