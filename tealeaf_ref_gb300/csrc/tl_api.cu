@@ -100,14 +100,14 @@ struct tl_ctx {
   cudaGraphExec_t cg_prof_exec = nullptr;
   LoopArgs cg_prof_key{};
   long long cg_prof_nk = 0;
-  // the persistent on-chip loops: FP64 CG, the FP32 process of the precision form, the FP64
-  // polynomial steps
+  // the persistent on-chip loops: FP64 CG, the FP32 process of the precision form, the FP64 and the
+  // FP32 polynomial steps
   struct Persist {
     int state = -1;  // -1 not yet planned, 0 the mesh does not fit, 1 plan holds
     PersistPlan plan{};
     void* box = nullptr;  // what its CTAs exchange partial sums and rims in
     unsigned epoch = 0;   // number of the next sum
-  } pcg, pmix, ppoly;
+  } pcg, pmix, ppoly, pmpoly;
   // host transfers: an upload and a download stream (tl_stage_state, tl_fetch_field) and
   // XFER_FIELDS staging fields -- two staged (density, energy1) pairs, the fetch snapshot, and
   // two for the synchronous uploads / downloads.  A host array moves as one contiguous copy
@@ -415,6 +415,27 @@ int run_persistent_poly(tl_ctx* c, bool ppcg, const double* u_in, int first, int
   return TL_OK;
 }
 
+// The FP32 polynomial steps on chip; off with TL_POLY_PERSISTENT=0, or where the environment says how the
+// blocked sweeps shall run.
+bool use_persistent_mix_poly(tl_ctx* c) {
+  const char* e = getenv("TL_POLY_PERSISTENT");
+  if (e && e[0] == '0') return false;
+  for (const char* n : {"TL_POLY_STEPS_PER_SWEEP", "TL_POLY_COLS", "TL_POLY_TMA", "TL_POLY_TEST_HOLD"})
+    if (getenv(n)) return false;
+  return use_persistent(c, c->pmpoly, mix_poly_persist_prepare);
+}
+
+// steps 1 .. steps of the coefficients on the device
+int run_persistent_mix_poly(tl_ctx* c, bool ppcg, int steps) {
+  unsigned epoch;
+  int rc = next_epoch(c, c->pmpoly, &epoch, steps);
+  if (rc) return rc;
+  const char* ex = getenv("TL_CG_BARRIER_EXTRA");  // 2: as for run_persistent_poly
+  CK(launch_persistent_mix_poly(c->mix, c->L, c->pmpoly.plan, ppcg, c->f.r, c->f.z, c->theta, c->ch_a + 1, c->ch_b + 1,
+                                steps, epoch, c->pmpoly.box, c->counter + MIX_ERR_WORD, ex && ex[0] == '2', c->stream));
+  return TL_OK;
+}
+
 int run_persistent_mix(tl_ctx* c) {
   unsigned epoch;
   int rc = next_epoch(c, c->pmix, &epoch);
@@ -716,6 +737,7 @@ int tl_destroy(tl_ctx* c) {
   cudaFree(c->pcg.box);
   cudaFree(c->pmix.box);
   cudaFree(c->ppoly.box);
+  cudaFree(c->pmpoly.box);
   if (c->cg_exec) cudaGraphExecDestroy(c->cg_exec);
   if (c->cg_prof_exec) cudaGraphExecDestroy(c->cg_prof_exec);
   if (c->mix_exec) cudaGraphExecDestroy(c->mix_exec);
@@ -762,7 +784,8 @@ int tl_device_bytes(const tl_ctx* c, unsigned long long* bytes) {
            sizeof(double) * 2 * ((size_t)c->hist_cap + c->ch_cap) + c->mix_bytes + (c->tape ? c->tape_bytes : 0) +
            (c->xfer ? (size_t)tl_ctx::XFER_FIELDS * c->field_stride : 0) +
            (c->pcg.box ? persist_box_bytes(c->pcg.plan) : 0) + (c->pmix.box ? persist_box_bytes(c->pmix.plan) : 0) +
-           (c->ppoly.box ? persist_box_bytes(c->ppoly.plan) : 0);
+           (c->ppoly.box ? persist_box_bytes(c->ppoly.plan) : 0) +
+           (c->pmpoly.box ? persist_box_bytes(c->pmpoly.plan) : 0);
   return TL_OK;
 }
 
@@ -1526,7 +1549,11 @@ struct Solver {
     if (inner_steps < 0) return TL_OK;
     int rc;
     if ((rc = prof_begin(c))) return rc;
-    launch_poly_ppcg_inner(c->f, c->mix, c->L, c->theta, inner_steps, ch_a.data(), ch_b.data(), c->stream);
+    if (inner_steps > 0 && use_persistent_mix_poly(c)) {
+      if ((rc = run_persistent_mix_poly(c, true, inner_steps))) return rc;
+    } else {
+      launch_poly_ppcg_inner(c->f, c->mix, c->L, c->theta, inner_steps, ch_a.data(), ch_b.data(), c->stream);
+    }
     if ((rc = prof_end(c, TL_KERNEL_POLY_STEP, std::max(inner_steps, 1)))) return rc;
     return check_launch("ppcg_inner_steps (FP32)");
   }
@@ -1567,7 +1594,11 @@ struct Solver {
       const int len = std::min(m, budget - total);
       if (len < 1) break;
       if ((rc = prof_begin(c))) return rc;
-      launch_poly_cheby(c->mix, c->L, c->theta, len, ch_a.data(), ch_b.data(), c->stream);
+      if (len > 1 && use_persistent_mix_poly(c)) {
+        if ((rc = run_persistent_mix_poly(c, false, len - 1))) return rc;
+      } else {
+        launch_poly_cheby(c->mix, c->L, c->theta, len, ch_a.data(), ch_b.data(), c->stream);
+      }
       if ((rc = prof_end(c, TL_KERNEL_POLY_STEP, len))) return rc;
       launch_mix_trial(c->f, c->mix, c->L, rd, c->mst, false, c->stream, false);  // m.r = u0 - A (u + d)
       if ((rc = check_launch("mixed chebyshev cycle"))) return rc;
@@ -1983,7 +2014,7 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
           S.ch_b.resize(inner + 2, 0.0);
         }
         c->cn = c->eigmax / c->eigmin;
-        if (!mixed && use_persistent_poly(c)) {
+        if (mixed ? use_persistent_mix_poly(c) : use_persistent_poly(c)) {
           const size_t n_ch = std::min(S.ch_a.size(), (size_t)c->ch_cap);
           CK(cudaMemcpyAsync(c->ch_a, S.ch_a.data(), sizeof(double) * n_ch, cudaMemcpyHostToDevice, c->stream));
           CK(cudaMemcpyAsync(c->ch_b, S.ch_b.data(), sizeof(double) * n_ch, cudaMemcpyHostToDevice, c->stream));

@@ -155,6 +155,14 @@ struct MixFields {
   float* mi;            // FP32 copy of the jac_diag preconditioner Mi = 1/Di (null: no preconditioner)
   float* z;             // jac_diag: z = Mi r of the FP32 CG process (null: no preconditioner)
 };
+// the FP32 polynomial steps on chip: `steps` PPCG inner steps from the FP64 residual r64 into z (FP64), or
+// Chebyshev iterations after the start on m.r into m.d; coefficients, boxes and numbers as for
+// launch_persistent_poly
+bool mix_poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out);
+cudaError_t launch_persistent_mix_poly(const MixFields& m, const Layout& L, const PersistPlan& p, bool ppcg,
+                                       const double* r64, double* z, double theta, const double* ch_a,
+                                       const double* ch_b, int steps, unsigned epoch, void* box, unsigned* err,
+                                       bool hold, cudaStream_t s);
 struct MixState {
   double rro, rro_prev, pw, rr, alpha, beta;  // FP32-vector CG scalars (FP64)
   double rr_max;                              // r.r at the last residual replacement

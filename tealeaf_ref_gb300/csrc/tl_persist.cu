@@ -1959,12 +1959,12 @@ bool poly_plan(int nx, int ny, int ctas, PersistPlan* out) {
 }
 
 // threads of one CTA differ between the kernels
-int poly_ctas(const void* k, size_t smem) {
+int poly_ctas(const void* k, int threads, size_t smem) {
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM_MAX) != cudaSuccess ||
       cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, QT, smem) != cudaSuccess) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -1975,10 +1975,10 @@ int poly_ctas(const void* k, size_t smem) {
 
 bool poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const int diag = precond == 2 ? 1 : 0;
-  const int ctas = poly_ctas((const void*)kPolyVariants[0].k[0][diag], PERSIST_SMEM_MAX);
+  const int ctas = poly_ctas((const void*)kPolyVariants[0].k[0][diag], QT, PERSIST_SMEM_MAX);
   if (!poly_plan(nx, ny, ctas, out)) return false;
   for (int mode = 0; mode < 2; ++mode)
-    if (poly_ctas((const void*)kPolyVariants[out->variant].k[mode][diag], poly_plan_smem(*out)) < persist_ctas(*out))
+    if (poly_ctas((const void*)kPolyVariants[out->variant].k[mode][diag], QT, poly_plan_smem(*out)) < persist_ctas(*out))
       return false;
   return true;
 }
@@ -1991,6 +1991,333 @@ cudaError_t launch_persistent_poly(const Fields& f, const Layout& L, const Persi
   ++launch_counter();
   return cudaLaunchCooperativeKernel((const void*)kPolyVariants[p.variant].k[ppcg ? 0 : 1][diag ? 1 : 0],
                                      dim3(persist_ctas(p)), dim3(QT), args, poly_plan_smem(p), s);
+}
+
+// ---- the FP32 polynomial steps of the precision form on chip ------------------------------------
+// The PPCG inner steps and the Chebyshev iterations on a correction (tl_mixed_poly.cu) of a mesh that
+// fits, all of an outer iteration's or a cycle's steps in one launch.  Tiles, groups of rows and the
+// coefficients' way from L2 are k_persistent_mix's, the rims' way k_persistent_poly's.  The stencil
+// variable x (sd; d) has two buffers with halo in shared memory, so that a step reads one and writes the
+// other and needs one barrier; the cell's other two values (rtemp, utemp; p, the right-hand side) are in
+// tensor memory.  8 bytes a cell in shared memory take meshes of up to about 2040^2.  Every product and
+// sum is that of the one-step kernels, in their order: same bits.
+//
+// A Chebyshev cycle's step took about 7 us at 1999 x 1500 against 15 in the blocked sweeps (four steps a
+// pass over the fields), bound by the coefficients' way from L2.  Whole solves, CG presteps included,
+// against the blocked sweeps: Chebyshev 200 x 300 4.0 ms against 10.4, 512^2 7.2 / 20.6, 1000^2 19.6 /
+// 42.6, 1999 x 1500 59.3 / 94.8, 2040^2 91 / 118; PPCG with 10 inner steps 512^2 11.1 / 21.3, 1000^2 28.3 /
+// 43.6, 1999 x 1500 78.7 / 94.7 (5 inner steps 103 / 120), 2040^2 with 20 inner steps 95 / 105.  Every mesh
+// that fits runs here.
+namespace {
+
+constexpr int YC = 4;  // rows handled together
+struct MixPolyArgs {
+  MixFields m;
+  Layout L;
+  PersistPlan pl;
+  const double* r64;          // PPCG: the FP64 residual the steps start from (Chebyshev: m.r)
+  double* z;                  // PPCG: utemp after the last step
+  float inv_theta;
+  const double *ch_a, *ch_b;  // coefficients of the first step ..
+  int steps;
+  unsigned epoch;             // number of the first step's rims
+  unsigned long long* box;    // halo boxes, by parity of the number
+  unsigned* err;              // set when a wait ran out: the results are void
+  int hold;                   // test of the bounded wait: the first tile sends no rims
+};
+
+__device__ __forceinline__ void tmem_get2(unsigned a, float (&v)[4], unsigned b, float (&w)[4]) {
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%8];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4, %5, %6, %7}, [%9];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3])
+      : "r"(a), "r"(b)
+      : "memory");
+}
+
+template <int MODE, bool DIAG>
+__global__ void __launch_bounds__(PT, 1) k_persistent_mix_poly(MixPolyArgs g) {
+  constexpr bool PPCG = MODE == ON_PPCG;
+  __shared__ int sh_fail;
+  __shared__ unsigned sh_tmem;
+  extern __shared__ __align__(16) float ysm[];
+  const Layout L = g.L;
+  const MixFields& f = g.m;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  if (t == 0) sh_fail = *reinterpret_cast<volatile unsigned*>(g.err) != 0u;
+  __syncthreads();
+  if (sh_fail) return;
+  if (wid == 0) tmem_alloc(&sh_tmem);
+
+  const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
+  const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;
+  const int tw = min(g.pl.tw, L.nx - j0), th = min(g.pl.th, L.ny - k0);
+  const int P = g.pl.tw + 2, asz = (g.pl.th + 2) * P;
+  const int oz = 2 * asz;  // a cell of zeros, for the lanes and rows without a cell
+
+  // the thread's column and rows y0 .. y0+mine-1, split evenly
+  const int tx = t % g.pl.tw, seg = t / g.pl.tw;
+  const int q_ = th / g.pl.ry, rem = th - q_ * g.pl.ry;
+  const int mine = (tx < tw && seg < g.pl.ry) ? q_ + (seg < rem) : 0, y0 = seg * q_ + min(seg, rem);
+  const int own = mine ? mine : q_ + (rem > 0);
+  const bool warp_owns = __any_sync(0xffffffffu, mine > 0);
+  const int nfull = warp_owns ? (int)__reduce_min_sync(0xffffffffu, (unsigned)own) / YC : 0;  // groups of YC rows
+  const int nch = warp_owns ? ((int)__reduce_max_sync(0xffffffffu, (unsigned)own) + YC - 1) / YC : 0;
+  const int o0 = mine ? (y0 + 1) * P + tx + 1 : oz, o_next = mine ? asz : 0;  // in the first buffer; to the second
+  const int c0 = mine ? (int)L.at(j0 + tx + 1, k0 + y0 + 1) : (int)L.at(j0 + 1, k0 + 1);
+  const int ld = L.ld, os = mine ? P : 0, cs = mine ? ld : 0;
+  const bool at_l = tx == 0 && j0 == 0, at_r = tx == tw - 1 && j0 + tw == L.nx;
+  // the neighbours' offsets: PPCG's sd is mirrored at a wall, the correction is zero outside
+  const int lo = ((PPCG && at_l) || !mine) ? 0 : -1, ro = ((PPCG && at_r) || !mine) ? 0 : 1;
+  const int i_first = (mine > 0 && y0 == 0) ? 0 : -1, i_last = (mine > 0 && y0 + mine == th) ? mine - 1 : -1;
+  const int i_b = PPCG && k0 == 0 ? i_first : -1, i_t = PPCG && k0 + th == L.ny ? i_last : -1;
+
+  // the start's value of a cell: z / theta
+  auto start = [&](int c) {
+    const float rv = PPCG ? (float)g.r64[c] : f.r[c];
+    return (DIAG ? f.mi[c] * rv : rv) * g.inv_theta;
+  };
+  const int hbox = 2 * (g.pl.th + g.pl.tw), hall = (int)gridDim.x * hbox;
+  int ho[PH], hh[PH];
+#pragma unroll
+  for (int q = 0; q < PH; ++q) {
+    const int h = t + q * PT;
+    ho[q] = -1;
+    hh[q] = 0;
+    int x = -1, y = h;
+    bool in = y < th, is = in && j0 > 0;
+    if (h >= g.pl.th) x = tw, y = h - g.pl.th, in = y < th, is = in && j0 + tw < L.nx;
+    if (h >= 2 * g.pl.th) x = h - 2 * g.pl.th, y = -1, in = x < tw, is = in && k0 > 0;
+    if (h >= 2 * g.pl.th + g.pl.tw) x = h - 2 * g.pl.th - g.pl.tw, y = th, in = x < tw, is = in && k0 + th < L.ny;
+    if (in && h < hbox) {
+      const int o = (y + 1) * P + x + 1;
+      // off the domain: zero (a mirrored row is written with its cells)
+      const bool mirror = PPCG && !is;
+      if (!mirror) ysm[o] = is ? start((int)L.at(j0 + x + 1, k0 + y + 1)) : 0.f;
+      if (!mirror && !is) ysm[asz + o] = 0.f;
+      if (is) {
+        ho[q] = o;
+        hh[q] = (int)blockIdx.x * hbox + h;
+      }
+    }
+  }
+  const bool sends = !(g.hold && blockIdx.x == 0);
+  const int to_l = (sends && mine && tx == 0 && j0 > 0) ? ((int)blockIdx.x - 1) * hbox + g.pl.th + y0 : -1;
+  const int to_r = (sends && mine && tx == tw - 1 && j0 + tw < L.nx) ? ((int)blockIdx.x + 1) * hbox + y0 : -1;
+  const int rim_b = sends && k0 > 0 ? i_first : -1, rim_t = sends && k0 + th < L.ny ? i_last : -1;
+  const int to_b = ((int)blockIdx.x - g.pl.gx) * hbox + 2 * g.pl.th + g.pl.tw + tx;
+  const int to_t = ((int)blockIdx.x + g.pl.gx) * hbox + 2 * g.pl.th + tx;
+
+  __syncthreads();
+  // this thread's words of tensor memory: rtemp / p, then utemp / the right-hand side
+  const unsigned ta = sh_tmem + ((unsigned)(wid & 3) << 21) + (unsigned)(wid >> 2) * (2 * MROWS), tb = ta + MROWS;
+  if (t == 0) ysm[oz] = 0.f;
+  for (int ch = 0; ch < nch; ++ch) {
+    float a[YC], b[YC];
+#pragma unroll
+    for (int j = 0; j < YC; ++j) {
+      const int i = ch * YC + j, c = c0 + i * cs;
+      a[j] = b[j] = 0.f;
+      if (i < mine) {
+        const float x = start(c);
+        ysm[o0 + i * os] = x;
+        a[j] = PPCG ? (float)g.r64[c] : x;
+        b[j] = PPCG ? x : f.r[c];
+        if (i == i_b) ysm[o0 + i * os - P] = x;
+        if (i == i_t) ysm[o0 + i * os + P] = x;
+      }
+    }
+    tmem_put(ta + ch * YC, a);
+    tmem_put(tb + ch * YC, b);
+  }
+  tmem_put_done();
+
+  struct Coefs {
+    float di[YC], cl[YC], cr[YC], ct[YC], mi[YC];  // Di, the left, right and upper face, Mi of a group of rows
+  } ka, kb;
+  const std::true_type full;
+  const std::false_type part;
+  auto load_group = [&](int ch, Coefs& k, auto f_) {
+    const int left = own - ch * YC, c1 = decltype(f_)::value || left > 0 ? c0 + ch * YC * cs : c0;
+    const float *pd = f.di + c1, *px = f.cx + c1, *py = f.cy + c1 + ld, *pm = DIAG ? f.mi + c1 : nullptr;
+#pragma unroll
+    for (int j = 0; j < YC; ++j) {
+      k.di[j] = __ldg(pd);
+      k.cl[j] = __ldg(px);
+      k.cr[j] = __ldg(px + 1);
+      k.ct[j] = __ldg(py);
+      if (DIAG) k.mi[j] = __ldg(pm);
+      if (decltype(f_)::value || j + 1 < left) {
+        pd += cs, px += cs, py += cs;
+        if (DIAG) pm += cs;
+      }
+    }
+  };
+  auto load_coefs = [&](int ch, Coefs& k) {
+    if (ch < nfull) load_group(ch, k, full);
+    else if (ch < nch) load_group(ch, k, part);
+  };
+  load_coefs(0, ka);
+  __syncthreads();
+
+  unsigned epoch = g.epoch;
+  bool failed = false;
+  int cur = 0, nxt = o_next;  // the buffers' offsets, of this thread's cells
+  int bufn = asz;             // the written buffer's, of the tile's
+  for (int step = 0; step < g.steps; ++step, ++epoch) {
+    const bool last = step + 1 == g.steps;
+    const float ca = (float)__ldg(g.ch_a + step), cb = (float)__ldg(g.ch_b + step);
+    unsigned long long* const halo = g.box + (size_t)(epoch & 1u) * hall;
+    {
+      float pb = 0.f, pc = 0.f, cyb = 0.f;
+      if (nch > 0) pb = ysm[cur + o0 - os], pc = ysm[cur + o0], cyb = __ldg(f.cy + c0);
+      auto rows_of = [&](int ch, const Coefs& k, auto f_) {
+        const int o = o0 + ch * YC * os, left = own - ch * YC;
+        float xl[YC], xr[YC], xt[YC], a[YC], b[YC];
+        // a group's loads before its stores
+#pragma unroll
+        for (int j = 0; j < YC; ++j) {
+          const bool in = decltype(f_)::value || j < left;
+          xt[j] = ysm[in ? cur + o + (j + 1) * os : oz];
+          xr[j] = ysm[in ? cur + o + j * os + ro : oz];
+          xl[j] = ysm[in ? cur + o + j * os + lo : oz];
+        }
+        tmem_get2(ta + ch * YC, a, tb + ch * YC, b);
+#pragma unroll
+        for (int j = 0; j < YC; ++j) {
+          const bool in = decltype(f_)::value || j < left;
+          if (!in) pb = pc = 0.f;
+          float v = k.di[j] * pc;
+          v = fmaf(-k.ct[j], xt[j], v);
+          v = fmaf(-cyb, pb, v);
+          v = fmaf(-k.cr[j], xr[j], v);
+          v = fmaf(-k.cl[j], xl[j], v);
+          const float res = (PPCG ? a[j] : b[j]) - v;
+          const float bz = cb * (DIAG ? k.mi[j] * res : res);
+          float x;
+          if (PPCG) {
+            a[j] = res;
+            x = fmaf(ca, pc, bz);
+            b[j] = b[j] + x;
+          } else {
+            a[j] = fmaf(ca, a[j], bz);
+            x = pc + a[j];
+          }
+          ysm[in ? nxt + o + j * os : oz] = in ? x : 0.f;
+          pb = pc;
+          pc = xt[j];
+          cyb = k.ct[j];
+        }
+        tmem_put(ta + ch * YC, a);
+        if (PPCG) tmem_put(tb + ch * YC, b);
+      };
+      auto rows = [&](int ch, const Coefs& k) {
+        if (ch < nfull) rows_of(ch, k, full);
+        else if (ch < nch) rows_of(ch, k, part);
+      };
+      // two groups of coefficients: the next one's loads are in flight while one is used
+      for (int ch = 0; ch < nch; ch += 2) {
+        load_coefs(ch + 1, kb);
+        rows(ch, ka);
+        load_coefs(ch + 2, ka);
+        rows(ch + 1, kb);
+      }
+      tmem_put_done();
+    }
+    if (!last) {
+      // the rim: a column's rows are its owner's, and the whole warp sends them
+      if (i_b >= 0) ysm[nxt + o0 - P] = ysm[nxt + o0];
+      if (i_t >= 0) ysm[nxt + o0 + mine * P] = ysm[nxt + o0 + (mine - 1) * P];
+      if (rim_b >= 0) fbox_put(halo + to_b, ysm[nxt + o0 + rim_b * P], epoch);
+      if (rim_t >= 0) fbox_put(halo + to_t, ysm[nxt + o0 + rim_t * P], epoch);
+      __syncwarp();
+      auto columns = [&](int to_) {
+        for (unsigned m = __ballot_sync(0xffffffffu, to_ >= 0); m; m &= m - 1) {
+          const int l = __ffs(m) - 1;
+          const int h = __shfl_sync(0xffffffffu, to_, l), o1 = __shfl_sync(0xffffffffu, nxt + o0, l),
+                    have = __shfl_sync(0xffffffffu, mine, l);
+          for (int i = lane; i < have; i += 32) fbox_put(halo + h + i, ysm[o1 + i * P], epoch);
+        }
+      };
+      columns(to_l);
+      columns(to_r);
+      load_coefs(0, ka);
+      bool got = false;
+      float hv[PH];
+      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+        got = true;
+#pragma unroll
+        for (int q = 0; q < PH; ++q)
+          if (ho[q] >= 0) {
+            const unsigned long long v = fbox_get(halo + hh[q]);
+            got = got && (unsigned)v == epoch;
+            hv[q] = __uint_as_float((unsigned)(v >> 32));
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < PH; ++q)
+        if (ho[q] >= 0) ysm[bufn + ho[q]] = hv[q];
+      if (!got) sh_fail = 1;
+      __syncthreads();
+      if (sh_fail) {
+        failed = true;
+        break;
+      }
+    }
+    const int swap = cur;
+    cur = nxt;
+    nxt = swap;
+    bufn = asz - bufn;
+  }
+  for (int ch = 0; ch < (failed ? 0 : nch); ++ch) {
+    float b[YC];
+    if (PPCG) tmem_get(tb + ch * YC, b);
+#pragma unroll
+    for (int j = 0; j < YC; ++j) {
+      const int i = ch * YC + j, c = c0 + i * cs;
+      if (i < mine) {
+        if (PPCG) g.z[c] = (double)b[j];
+        else f.d[c] = ysm[cur + o0 + i * os];
+      }
+    }
+  }
+  __syncthreads();  // every warp is done with tensor memory
+  if (wid == 0) tmem_free(sh_tmem);
+  if (failed && t == 0) atomicExch(g.err, 1u);
+}
+
+using MixPolyKernel = void (*)(MixPolyArgs);
+const MixPolyKernel kMixPolyKernels[2][2] = {  // PPCG / Chebyshev, without / with jac_diag
+    {k_persistent_mix_poly<ON_PPCG, false>, k_persistent_mix_poly<ON_PPCG, true>},
+    {k_persistent_mix_poly<ON_CHEBY, false>, k_persistent_mix_poly<ON_CHEBY, true>}};
+size_t mix_poly_plan_smem(const PersistPlan& p) {
+  return ((size_t)2 * (p.th + 2) * (p.tw + 2) + 1) * sizeof(float);
+}
+
+}  // namespace
+
+bool mix_poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
+  const int diag = precond == 2 ? 1 : 0;
+  const int ctas = poly_ctas((const void*)kMixPolyKernels[0][diag], PT, PERSIST_SMEM_MAX);
+  if (!rows_plan(nx, ny, ctas, MROWS, mix_poly_plan_smem, out)) return false;
+  for (int mode = 0; mode < 2; ++mode)
+    if (poly_ctas((const void*)kMixPolyKernels[mode][diag], PT, mix_poly_plan_smem(*out)) < persist_ctas(*out))
+      return false;
+  return true;
+}
+
+cudaError_t launch_persistent_mix_poly(const MixFields& m, const Layout& L, const PersistPlan& p, bool ppcg,
+                                       const double* r64, double* z, double theta, const double* ch_a,
+                                       const double* ch_b, int steps, unsigned epoch, void* box, unsigned* err,
+                                       bool hold, cudaStream_t s) {
+  MixPolyArgs g{m, L, p, r64, z, (float)(1.0 / theta), ch_a, ch_b, steps, epoch,
+                static_cast<unsigned long long*>(box), err, hold ? 1 : 0};
+  void* args[] = {&g};
+  ++launch_counter();
+  return cudaLaunchCooperativeKernel((const void*)kMixPolyKernels[ppcg ? 0 : 1][m.mi ? 1 : 0], dim3(persist_ctas(p)),
+                                     dim3(PT), args, mix_poly_plan_smem(p), s);
 }
 
 }  // namespace tl

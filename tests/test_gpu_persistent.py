@@ -120,3 +120,56 @@ def test_on_chip_polynomial_wait_is_bounded(solver, monkeypatch):
         c.reset_eigen()
         got = c.tea_leaf(d)
         assert (got.n_exit, got.error) == (want.n_exit, want.error)
+
+
+MIXED_POLY_SIZES = [(9, 9), (1, 700), (700, 1), (97, 131), (301, 499), (640, 613), (999, 1001), (1499, 1999), (2039, 2043)]
+
+
+@pytest.mark.parametrize("case", [dict(), dict(precond="jac_diag", reflective=True)], ids=["none", "diag-reflective"])
+@pytest.mark.parametrize("solver", ["ppcg", "chebyshev"])
+@pytest.mark.parametrize("size", MIXED_POLY_SIZES, ids=["%dx%d" % s for s in MIXED_POLY_SIZES])
+def test_on_chip_fp32_polynomial_steps_give_the_same_bits(size, solver, case, monkeypatch):
+    """The FP32 PPCG inner steps and Chebyshev cycles of the precision form on chip against the blocked
+    sweeps: the same bits in every FP64 field."""
+    from tealeaf_ref_gb300 import native
+
+    d = small_deck(nx=size[0], ny=size[1], solver=solver, ppcg_inner_steps=7, ch_cg_presteps=6, ch_cg_epslim=1e30,
+                   max_iters=14 if solver == "ppcg" else 87, steps=1, **case)
+    o = native.opts_from_deck(d, "mixed")
+    fields = ["u", "r", "p"] + (["w", "z"] if solver == "ppcg" else [])
+    runs = []
+    for form in ("0", "1"):
+        monkeypatch.setenv("TL_POLY_PERSISTENT", form)
+        with native.Chunk.from_deck(d) as c:
+            i = c.tea_leaf(o, d.initial_timestep)
+            runs.append((i, {f: c.download(f) for f in fields}))
+    (i0, f0), (i1, f1) = runs
+    assert i0.cheby_calc_steps > 0
+    assert i1.kernel_launches < i0.kernel_launches, "the on-chip steps did not run"
+    assert (i0.n_exit, i0.error, i0.cheby_calc_steps, i0.ppcg_inner_iters) == \
+           (i1.n_exit, i1.error, i1.cheby_calc_steps, i1.ppcg_inner_iters)
+    for f in fields:
+        assert np.array_equal(f0[f], f1[f]), f
+
+
+@pytest.mark.parametrize("solver", ["ppcg", "chebyshev"])
+def test_on_chip_fp32_polynomial_wait_is_bounded(solver, monkeypatch):
+    """As test_on_chip_polynomial_wait_is_bounded, for the precision form."""
+    from tealeaf_ref_gb300 import native
+
+    d = small_deck(nx=200, ny=160, solver=solver, ppcg_inner_steps=6, ch_cg_presteps=10, ch_cg_epslim=1e30,
+                   max_iters=60, steps=1)
+    o = native.opts_from_deck(d, "mixed")
+    with native.Chunk.from_deck(d) as c:
+        want = c.tea_leaf(o, d.initial_timestep)
+        c.generate(d)
+        c.reset_eigen()
+        monkeypatch.setenv("TL_CG_BARRIER_EXTRA", "2")
+        with pytest.raises(native.TeaLeafError) as e:
+            c.tea_leaf(o, d.initial_timestep)
+        assert e.value.code == -5  # TL_ERR_TIMEOUT
+        monkeypatch.delenv("TL_CG_BARRIER_EXTRA")
+        c.generate(d)
+        c.reset_eigen()
+        got = c.tea_leaf(o, d.initial_timestep)
+        assert (got.n_exit, got.error) == (want.n_exit, want.error)
