@@ -1609,13 +1609,13 @@ namespace {
 // sums' exchange when there is more than one tile); tiles at least 32 columns wide, where
 // the mesh is, for the sake of the coefficients' loads.
 template <typename F>
-bool rows_plan(int nx, int ny, int ctas, int max_rows, F&& smem, PersistPlan* out) {
+bool rows_plan(int nx, int ny, int ctas, int threads, int max_rows, F&& smem, PersistPlan* out) {
   double best = 0.0;
   bool found = false;
   if (ctas > PERSIST_MAX_CTAS) ctas = PERSIST_MAX_CTAS;
   for (int g0 = 1; g0 <= ctas && g0 <= nx; ++g0) {
     const int tw = (nx + g0 - 1) / g0;
-    if (tw > PT || (tw < 32 && g0 > 1)) continue;
+    if (tw > threads || (tw < 32 && g0 > 1)) continue;
     PersistPlan p;
     p.cs = 1;
     p.tw = tw;
@@ -1626,11 +1626,11 @@ bool rows_plan(int nx, int ny, int ctas, int max_rows, F&& smem, PersistPlan* ou
       if (gy < 1) continue;
       p.th = (ny + gy - 1) / gy;
       p.gy = (ny + p.th - 1) / p.th;
-      p.ry = PT / tw < p.th ? PT / tw : p.th;
+      p.ry = threads / tw < p.th ? threads / tw : p.th;
       p.rows = (p.th + p.ry - 1) / p.ry;
       p.variant = 0;
       const int halo = 2 * (p.tw + p.th);
-      if (p.rows > max_rows || halo > PH * PT || smem(p) > PERSIST_SMEM_MAX) continue;
+      if (p.rows > max_rows || halo > PH * threads || smem(p) > PERSIST_SMEM_MAX) continue;
       const double cost =
           (double)((p.ry * tw + 31) / 32) * p.rows * 16.0 + 0.5 * halo + (p.gx * p.gy > 1 ? 6400.0 : 0.0);
       if (!found || cost < best) {
@@ -1660,7 +1660,7 @@ bool persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const void* k0 = (const void*)kVariants[0].k[precond == 2 ? 1 : 0];
   for (int i = 0; i < 5; ++i) clusters[i] = persist_clusters(k0, 1 << i, PERSIST_SMEM_MAX);
   if (!persist_plan(nx, ny, clusters, out)) {
-    if (!rows_plan(nx, ny, clusters[0], WROWS, wide_plan_smem, out)) return false;
+    if (!rows_plan(nx, ny, clusters[0], PT, WROWS, wide_plan_smem, out)) return false;
     out->variant = WIDE;
   }
   return persist_clusters(cg_kernel(*out, precond), out->cs, cg_smem(*out)) * out->cs >= persist_ctas(*out);
@@ -1693,7 +1693,7 @@ size_t mix_plan_smem(const PersistPlan& p) {
 bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const bool diag = precond == 2;
   const int ctas = persist_clusters((const void*)kMixKernels[1][diag], 1, PERSIST_SMEM_MAX);
-  if (!rows_plan(nx, ny, ctas, MROWS, mix_plan_smem, out)) return false;
+  if (!rows_plan(nx, ny, ctas, PT, MROWS, mix_plan_smem, out)) return false;
   return persist_clusters(mix_kernel(*out, diag), 1, mix_plan_smem(*out)) >= persist_ctas(*out);
 }
 
@@ -1973,26 +1973,6 @@ int poly_ctas(const void* k, int threads, size_t smem) {
 
 }  // namespace
 
-bool poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
-  const int diag = precond == 2 ? 1 : 0;
-  const int ctas = poly_ctas((const void*)kPolyVariants[0].k[0][diag], QT, PERSIST_SMEM_MAX);
-  if (!poly_plan(nx, ny, ctas, out)) return false;
-  for (int mode = 0; mode < 2; ++mode)
-    if (poly_ctas((const void*)kPolyVariants[out->variant].k[mode][diag], QT, poly_plan_smem(*out)) < persist_ctas(*out))
-      return false;
-  return true;
-}
-
-cudaError_t launch_persistent_poly(const Fields& f, const Layout& L, const PersistPlan& p, bool ppcg, bool diag,
-                                   const double* u_in, const double* ch_a, const double* ch_b, int steps,
-                                   unsigned epoch, void* box, unsigned* err, bool hold, cudaStream_t s) {
-  PolyPersistArgs g{f, L, p, u_in, ch_a, ch_b, steps, epoch, static_cast<ulonglong2*>(box), err, hold ? 1 : 0};
-  void* args[] = {&g};
-  ++launch_counter();
-  return cudaLaunchCooperativeKernel((const void*)kPolyVariants[p.variant].k[ppcg ? 0 : 1][diag ? 1 : 0],
-                                     dim3(persist_ctas(p)), dim3(QT), args, poly_plan_smem(p), s);
-}
-
 // ---- the FP32 polynomial steps of the precision form on chip ------------------------------------
 // The PPCG inner steps and the Chebyshev iterations on a correction (tl_mixed_poly.cu) of a mesh that
 // fits, all of an outer iteration's or a cycle's steps in one launch.  Tiles, groups of rows and the
@@ -2005,8 +1985,8 @@ cudaError_t launch_persistent_poly(const Fields& f, const Layout& L, const Persi
 // A Chebyshev cycle's step took about 7 us at 1999 x 1500 against 15 in the blocked sweeps (four steps a
 // pass over the fields), bound by the coefficients' way from L2.  Whole solves, CG presteps included,
 // against the blocked sweeps: Chebyshev 200 x 300 4.0 ms against 10.4, 512^2 7.2 / 20.6, 1000^2 19.6 /
-// 42.6, 1999 x 1500 59.3 / 94.8, 2040^2 91 / 118; PPCG with 10 inner steps 512^2 11.1 / 21.3, 1000^2 28.3 /
-// 43.6, 1999 x 1500 78.7 / 94.7 (5 inner steps 103 / 120), 2040^2 with 20 inner steps 95 / 105.  Every mesh
+// 42.6, 1999 x 1500 59.3 / 94.8, 2040^2 84 / 118; PPCG with 10 inner steps 512^2 11.1 / 21.3, 1000^2 28.3 /
+// 43.6, 1999 x 1500 78.7 / 94.7 (5 inner steps 103 / 120), 2040^2 with 20 inner steps 91 / 105.  Every mesh
 // that fits runs here.
 namespace {
 
@@ -2038,7 +2018,7 @@ __device__ __forceinline__ void tmem_get2(unsigned a, float (&v)[4], unsigned b,
 }
 
 template <int MODE, bool DIAG>
-__global__ void __launch_bounds__(PT, 1) k_persistent_mix_poly(MixPolyArgs g) {
+__global__ void __launch_bounds__(QT, 1) k_persistent_mix_poly(MixPolyArgs g) {
   constexpr bool PPCG = MODE == ON_PPCG;
   __shared__ int sh_fail;
   __shared__ unsigned sh_tmem;
@@ -2083,7 +2063,7 @@ __global__ void __launch_bounds__(PT, 1) k_persistent_mix_poly(MixPolyArgs g) {
   int ho[PH], hh[PH];
 #pragma unroll
   for (int q = 0; q < PH; ++q) {
-    const int h = t + q * PT;
+    const int h = t + q * QT;
     ho[q] = -1;
     hh[q] = 0;
     int x = -1, y = h;
@@ -2288,22 +2268,336 @@ __global__ void __launch_bounds__(PT, 1) k_persistent_mix_poly(MixPolyArgs g) {
   if (failed && t == 0) atomicExch(g.err, 1u);
 }
 
+// ---- the FP64 polynomial steps of larger tiles ---------------------------------------------------
+// k_persistent_poly's steps laid out as k_persistent_mix_poly: two buffers of the stencil variable in shared
+// memory, rtemp and utemp (p and u0) in tensor memory, the coefficients from L2.  Same bits.
+// It runs where k_persistent_poly's tiles do not fit (about a million cells), to about 1400^2: 900 inner steps
+// of 18 PPCG outer iterations took 22.0 ms at 1100^2 against 24.3 as sweeps in memory, 30.4 / 33.0 at 1400^2,
+// 23.0 / 34.0 at 1200^2 with jac_diag, 402 Chebyshev iterations 11.5 / 12.4, 15.9 / 16.6 and 12.2 / 20.1.  At
+// 1000^2 the two are even (17.0 and 16.9 ms), at 700^2 k_persistent_poly leads (10.4 and 9.3).  The FP64 pipe
+// bounds it: 7 instructions a cell and step.
+constexpr int VC = 2;  // rows handled together
+__device__ __forceinline__ void tmem_put(unsigned a, const double (&v)[2]) {
+  float w[4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    w[2 * i] = __int_as_float(__double2loint(v[i]));
+    w[2 * i + 1] = __int_as_float(__double2hiint(v[i]));
+  }
+  tmem_put(a, w);
+}
+__device__ __forceinline__ void tmem_get2(unsigned a, double (&v)[2], unsigned b, double (&w)[2]) {
+  float x[4], y[4];
+  tmem_get2(a, x, b, y);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    v[i] = __hiloint2double(__float_as_int(x[2 * i + 1]), __float_as_int(x[2 * i]));
+    w[i] = __hiloint2double(__float_as_int(y[2 * i + 1]), __float_as_int(y[2 * i]));
+  }
+}
+
+template <int MODE, bool DIAG>
+__global__ void __launch_bounds__(QT, 1) k_persistent_poly_wide(PolyPersistArgs g) {
+  constexpr bool PPCG = MODE == ON_PPCG;
+  __shared__ int sh_fail;
+  __shared__ unsigned sh_tmem;
+  extern __shared__ __align__(16) double vsm[];
+  const Layout L = g.L;
+  const Fields& f = g.f;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  if (t == 0) sh_fail = *reinterpret_cast<volatile unsigned*>(g.err) != 0u;
+  __syncthreads();
+  if (sh_fail) return;
+  if (wid == 0) tmem_alloc(&sh_tmem);
+
+  const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
+  const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;
+  const int tw = min(g.pl.tw, L.nx - j0), th = min(g.pl.th, L.ny - k0);
+  const int P = g.pl.tw + 2, asz = (g.pl.th + 2) * P;
+  const int oz = 2 * asz;  // a cell of zeros, for the lanes and rows without a cell
+
+  // the thread's column and rows y0 .. y0+mine-1, split evenly
+  const int tx = t % g.pl.tw, seg = t / g.pl.tw;
+  const int q_ = th / g.pl.ry, rem = th - q_ * g.pl.ry;
+  const int mine = (tx < tw && seg < g.pl.ry) ? q_ + (seg < rem) : 0, y0 = seg * q_ + min(seg, rem);
+  const int own = mine ? mine : q_ + (rem > 0);
+  const bool warp_owns = __any_sync(0xffffffffu, mine > 0);
+  const int nfull = warp_owns ? (int)__reduce_min_sync(0xffffffffu, (unsigned)own) / VC : 0;  // groups of VC rows
+  const int nch = warp_owns ? ((int)__reduce_max_sync(0xffffffffu, (unsigned)own) + VC - 1) / VC : 0;
+  const int o0 = mine ? (y0 + 1) * P + tx + 1 : oz, o_next = mine ? asz : 0;  // in the first buffer; to the second
+  const int c0 = mine ? (int)L.at(j0 + tx + 1, k0 + y0 + 1) : (int)L.at(j0 + 1, k0 + 1);
+  const int ld = L.ld, os = mine ? P : 0, cs = mine ? ld : 0;
+  const int lo = mine ? -1 : 0, ro = mine ? 1 : 0;  // the neighbours' offsets
+  const int i_first = (mine > 0 && y0 == 0) ? 0 : -1, i_last = (mine > 0 && y0 + mine == th) ? mine - 1 : -1;
+
+  const double* const xin = PPCG ? f.sd : g.x_in;
+  const int hbox = 2 * (g.pl.th + g.pl.tw), hall = (int)gridDim.x * hbox;
+  int ho[PH], hh[PH];
+#pragma unroll
+  for (int q = 0; q < PH; ++q) {
+    const int h = t + q * QT;
+    ho[q] = -1;
+    hh[q] = 0;
+    int x = -1, y = h;
+    bool in = y < th, is = in && j0 > 0;
+    if (h >= g.pl.th) x = tw, y = h - g.pl.th, in = y < th, is = in && j0 + tw < L.nx;
+    if (h >= 2 * g.pl.th) x = h - 2 * g.pl.th, y = -1, in = x < tw, is = in && k0 > 0;
+    if (h >= 2 * g.pl.th + g.pl.tw) x = h - 2 * g.pl.th - g.pl.tw, y = th, in = x < tw, is = in && k0 + th < L.ny;
+    if (in && h < hbox) {
+      const int o = (y + 1) * P + x + 1;
+      vsm[o] = vsm[asz + o] = xin[L.at(j0 + x + 1, k0 + y + 1)];  // off the domain: the field's halo, which stays
+      if (is) {
+        ho[q] = o;
+        hh[q] = (int)blockIdx.x * hbox + h;
+      }
+    }
+  }
+  const bool sends = !(g.hold && blockIdx.x == 0);
+  const int to_l = (sends && mine && tx == 0 && j0 > 0) ? ((int)blockIdx.x - 1) * hbox + g.pl.th + y0 : -1;
+  const int to_r = (sends && mine && tx == tw - 1 && j0 + tw < L.nx) ? ((int)blockIdx.x + 1) * hbox + y0 : -1;
+  const int rim_b = sends && k0 > 0 ? i_first : -1, rim_t = sends && k0 + th < L.ny ? i_last : -1;
+  const int to_b = ((int)blockIdx.x - g.pl.gx) * hbox + 2 * g.pl.th + g.pl.tw + tx;
+  const int to_t = ((int)blockIdx.x + g.pl.gx) * hbox + 2 * g.pl.th + tx;
+
+  __syncthreads();
+  // this thread's words of tensor memory: rtemp / p, then utemp / u0
+  const unsigned ta = sh_tmem + ((unsigned)(wid & 3) << 21) + (unsigned)(wid >> 2) * 128u, tb = ta + 2 * WROWS;
+  if (t == 0) vsm[oz] = 0.0;
+  for (int ch = 0; ch < nch; ++ch) {
+    double a[VC], b[VC];
+#pragma unroll
+    for (int j = 0; j < VC; ++j) {
+      const int i = ch * VC + j, c = c0 + i * cs;
+      a[j] = b[j] = 0.0;
+      if (i < mine) {
+        vsm[o0 + i * os] = xin[c];
+        a[j] = PPCG ? f.rtemp[c] : f.p[c];
+        b[j] = PPCG ? f.utemp[c] : f.u0[c];
+      }
+    }
+    tmem_put(ta + ch * 2 * VC, a);
+    tmem_put(tb + ch * 2 * VC, b);
+  }
+  tmem_put_done();
+
+  struct Coefs {
+    double di[VC], cl[VC], cr[VC], ct[VC], mi[VC];  // Di, the left, right and upper face, Mi of a group of rows
+  } ka, kb;
+  const std::true_type full;
+  const std::false_type part;
+  auto load_group = [&](int ch, Coefs& k, auto f_) {
+    const int left = own - ch * VC, c1 = decltype(f_)::value || left > 0 ? c0 + ch * VC * cs : c0;
+    const double *pd = f.di + c1, *px = f.cx + c1, *py = f.cy + c1 + ld, *pm = DIAG ? f.mi + c1 : nullptr;
+#pragma unroll
+    for (int j = 0; j < VC; ++j) {
+      k.di[j] = __ldg(pd);
+      k.cl[j] = __ldg(px);
+      k.cr[j] = __ldg(px + 1);
+      k.ct[j] = __ldg(py);
+      if (DIAG) k.mi[j] = __ldg(pm);
+      if (decltype(f_)::value || j + 1 < left) {
+        pd += cs, px += cs, py += cs;
+        if (DIAG) pm += cs;
+      }
+    }
+  };
+  auto load_coefs = [&](int ch, Coefs& k) {
+    if (ch < nfull) load_group(ch, k, full);
+    else if (ch < nch) load_group(ch, k, part);
+  };
+  load_coefs(0, ka);
+  __syncthreads();
+
+  unsigned epoch = g.epoch;
+  bool failed = false;
+  int cur = 0, nxt = o_next;  // the buffers' offsets, of this thread's cells
+  int bufn = asz;             // the written buffer's, of the tile's
+  for (int step = 0; step < g.steps; ++step, ++epoch) {
+    const bool last = step + 1 == g.steps;
+    const double ca = __ldg(g.ch_a + step), cb = __ldg(g.ch_b + step);
+    ulonglong2* const halo = g.box + (size_t)(epoch & 1u) * hall;
+    {
+      double pb = 0.0, pc = 0.0, cyb = 0.0;
+      if (nch > 0) pb = vsm[cur + o0 - os], pc = vsm[cur + o0], cyb = __ldg(f.cy + c0);
+      auto rows_of = [&](int ch, const Coefs& k, auto f_) {
+        const int o = o0 + ch * VC * os, left = own - ch * VC;
+        double xl[VC], xr[VC], xt[VC], a[VC], b[VC];
+        // a group's loads before its stores
+#pragma unroll
+        for (int j = 0; j < VC; ++j) {
+          const bool in = decltype(f_)::value || j < left;
+          xt[j] = vsm[in ? cur + o + (j + 1) * os : oz];
+          xr[j] = vsm[in ? cur + o + j * os + ro : oz];
+          xl[j] = vsm[in ? cur + o + j * os + lo : oz];
+        }
+        tmem_get2(ta + ch * 2 * VC, a, tb + ch * 2 * VC, b);
+#pragma unroll
+        for (int j = 0; j < VC; ++j) {
+          const bool in = decltype(f_)::value || j < left;
+          if (!in) pb = pc = 0.0;
+          double v = dmul_int(k.di[j], pc);
+          v = fma(-k.ct[j], xt[j], v);
+          v = fma(-cyb, pb, v);
+          v = fma(-k.cr[j], xr[j], v);
+          v = fma(-k.cl[j], xl[j], v);
+          const double res = (PPCG ? a[j] : b[j]) - v;
+          const double z = DIAG ? k.mi[j] * res : res;
+          if (!PPCG && last && in && mine) {
+            const int c = c0 + (ch * VC + j) * cs;
+            f.w[c] = v;
+            f.r[c] = res;
+            if (DIAG) f.z[c] = z;
+          }
+          const double bz = dmul_int(cb, z);
+          double x;
+          if (PPCG) {
+            a[j] = res;
+            x = fma(ca, pc, bz);
+            b[j] = b[j] + x;
+          } else {
+            a[j] = fma(ca, a[j], bz);
+            x = pc + a[j];
+          }
+          vsm[in ? nxt + o + j * os : oz] = in ? x : 0.0;
+          pb = pc;
+          pc = xt[j];
+          cyb = k.ct[j];
+        }
+        tmem_put(ta + ch * 2 * VC, a);
+        if (PPCG) tmem_put(tb + ch * 2 * VC, b);
+      };
+      auto rows = [&](int ch, const Coefs& k) {
+        if (ch < nfull) rows_of(ch, k, full);
+        else if (ch < nch) rows_of(ch, k, part);
+      };
+      // two groups of coefficients: the next one's loads are in flight while one is used
+      for (int ch = 0; ch < nch; ch += 2) {
+        load_coefs(ch + 1, kb);
+        rows(ch, ka);
+        load_coefs(ch + 2, ka);
+        rows(ch + 1, kb);
+      }
+      tmem_put_done();
+    }
+    if (!last) {
+      // the rim: a column's rows are its owner's, and the whole warp sends them
+      if (rim_b >= 0) box_put(halo + to_b, vsm[nxt + o0 + rim_b * P], epoch);
+      if (rim_t >= 0) box_put(halo + to_t, vsm[nxt + o0 + rim_t * P], epoch);
+      __syncwarp();
+      auto columns = [&](int to_) {
+        for (unsigned m = __ballot_sync(0xffffffffu, to_ >= 0); m; m &= m - 1) {
+          const int l = __ffs(m) - 1;
+          const int h = __shfl_sync(0xffffffffu, to_, l), o1 = __shfl_sync(0xffffffffu, nxt + o0, l),
+                    have = __shfl_sync(0xffffffffu, mine, l);
+          for (int i = lane; i < have; i += 32) box_put(halo + h + i, vsm[o1 + i * P], epoch);
+        }
+      };
+      columns(to_l);
+      columns(to_r);
+      load_coefs(0, ka);
+      bool got = false;
+      double hv[PH];
+      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+        got = true;
+#pragma unroll
+        for (int q = 0; q < PH; ++q)
+          if (ho[q] >= 0) {
+            const ulonglong2 v = box_get(halo + hh[q]);
+            got = got && box_is(v, epoch);
+            hv[q] = box_value(v);
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < PH; ++q)
+        if (ho[q] >= 0) vsm[bufn + ho[q]] = hv[q];
+      if (!got) sh_fail = 1;
+      __syncthreads();
+      if (sh_fail) {
+        failed = true;
+        break;
+      }
+    }
+    const int swap = cur;
+    cur = nxt;
+    nxt = swap;
+    bufn = asz - bufn;
+  }
+  for (int ch = 0; ch < (failed ? 0 : nch); ++ch) {
+    double a[VC], b[VC];
+    tmem_get2(ta + ch * 2 * VC, a, tb + ch * 2 * VC, b);
+#pragma unroll
+    for (int j = 0; j < VC; ++j) {
+      const int i = ch * VC + j, c = c0 + i * cs;
+      if (i < mine) {
+        const double x = vsm[cur + o0 + i * os];
+        if (PPCG) {
+          f.sd[c] = x;
+          f.rtemp[c] = a[j];
+          f.utemp[c] = b[j];
+        } else {
+          f.u[c] = x;
+          f.p[c] = a[j];
+        }
+      }
+    }
+  }
+  __syncthreads();  // every warp is done with tensor memory
+  if (wid == 0) tmem_free(sh_tmem);
+  if (failed && t == 0) atomicExch(g.err, 1u);
+}
+
 using MixPolyKernel = void (*)(MixPolyArgs);
 const MixPolyKernel kMixPolyKernels[2][2] = {  // PPCG / Chebyshev, without / with jac_diag
     {k_persistent_mix_poly<ON_PPCG, false>, k_persistent_mix_poly<ON_PPCG, true>},
     {k_persistent_mix_poly<ON_CHEBY, false>, k_persistent_mix_poly<ON_CHEBY, true>}};
+const PolyPersistKernel kPolyWideKernels[2][2] = {  // PPCG / Chebyshev, without / with jac_diag
+    {k_persistent_poly_wide<ON_PPCG, false>, k_persistent_poly_wide<ON_PPCG, true>},
+    {k_persistent_poly_wide<ON_CHEBY, false>, k_persistent_poly_wide<ON_CHEBY, true>}};
+size_t poly_wide_plan_smem(const PersistPlan& p) {
+  return ((size_t)2 * (p.th + 2) * (p.tw + 2) + 1) * sizeof(double);
+}
 size_t mix_poly_plan_smem(const PersistPlan& p) {
   return ((size_t)2 * (p.th + 2) * (p.tw + 2) + 1) * sizeof(float);
 }
 
 }  // namespace
 
+bool poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
+  const int diag = precond == 2 ? 1 : 0;
+  const int ctas = poly_ctas((const void*)kPolyVariants[0].k[0][diag], QT, PERSIST_SMEM_MAX);
+  bool fits = poly_plan(nx, ny, ctas, out);
+  for (int mode = 0; mode < 2 && fits; ++mode)
+    fits = poly_ctas((const void*)kPolyVariants[out->variant].k[mode][diag], QT, poly_plan_smem(*out)) >= persist_ctas(*out);
+  if (fits) return true;
+  const int wide = poly_ctas((const void*)kPolyWideKernels[0][diag], QT, PERSIST_SMEM_MAX);
+  if (!rows_plan(nx, ny, wide, QT, WROWS, poly_wide_plan_smem, out)) return false;
+  out->variant = WIDE;
+  for (int mode = 0; mode < 2; ++mode)
+    if (poly_ctas((const void*)kPolyWideKernels[mode][diag], QT, poly_wide_plan_smem(*out)) < persist_ctas(*out))
+      return false;
+  return true;
+}
+
+cudaError_t launch_persistent_poly(const Fields& f, const Layout& L, const PersistPlan& p, bool ppcg, bool diag,
+                                   const double* u_in, const double* ch_a, const double* ch_b, int steps,
+                                   unsigned epoch, void* box, unsigned* err, bool hold, cudaStream_t s) {
+  PolyPersistArgs g{f, L, p, u_in, ch_a, ch_b, steps, epoch, static_cast<ulonglong2*>(box), err, hold ? 1 : 0};
+  void* args[] = {&g};
+  ++launch_counter();
+  const int mode = ppcg ? 0 : 1, d = diag ? 1 : 0;
+  if (p.variant == WIDE)
+    return cudaLaunchCooperativeKernel((const void*)kPolyWideKernels[mode][d], dim3(persist_ctas(p)), dim3(QT), args,
+                                       poly_wide_plan_smem(p), s);
+  return cudaLaunchCooperativeKernel((const void*)kPolyVariants[p.variant].k[mode][d], dim3(persist_ctas(p)), dim3(QT),
+                                     args, poly_plan_smem(p), s);
+}
+
 bool mix_poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const int diag = precond == 2 ? 1 : 0;
-  const int ctas = poly_ctas((const void*)kMixPolyKernels[0][diag], PT, PERSIST_SMEM_MAX);
-  if (!rows_plan(nx, ny, ctas, MROWS, mix_poly_plan_smem, out)) return false;
+  const int ctas = poly_ctas((const void*)kMixPolyKernels[0][diag], QT, PERSIST_SMEM_MAX);
+  if (!rows_plan(nx, ny, ctas, QT, MROWS, mix_poly_plan_smem, out)) return false;
   for (int mode = 0; mode < 2; ++mode)
-    if (poly_ctas((const void*)kMixPolyKernels[mode][diag], PT, mix_poly_plan_smem(*out)) < persist_ctas(*out))
+    if (poly_ctas((const void*)kMixPolyKernels[mode][diag], QT, mix_poly_plan_smem(*out)) < persist_ctas(*out))
       return false;
   return true;
 }
@@ -2317,7 +2611,7 @@ cudaError_t launch_persistent_mix_poly(const MixFields& m, const Layout& L, cons
   void* args[] = {&g};
   ++launch_counter();
   return cudaLaunchCooperativeKernel((const void*)kMixPolyKernels[ppcg ? 0 : 1][m.mi ? 1 : 0], dim3(persist_ctas(p)),
-                                     dim3(PT), args, mix_poly_plan_smem(p), s);
+                                     dim3(QT), args, mix_poly_plan_smem(p), s);
 }
 
 }  // namespace tl

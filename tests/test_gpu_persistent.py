@@ -68,7 +68,8 @@ def test_persistent_fp32_steps_match_the_sweeps(size, case, monkeypatch):
     assert np.max(np.abs(u1 - u0)) <= 8 * 2 * 8 * 2.0 ** -23 * np.max(np.abs(u0 - b))
 
 
-POLY_SIZES = [(9, 9), (22, 21), (1, 700), (700, 1), (97, 131), (301, 499), (600, 433), (777, 813), (1000, 1000)]
+POLY_SIZES = [(9, 9), (22, 21), (1, 700), (700, 1), (97, 131), (301, 499), (600, 433), (777, 813), (1000, 1000), (1003, 1201),
+              (1399, 1391)]
 
 
 @pytest.mark.parametrize("precond", ["none", "jac_diag"])
