@@ -123,7 +123,7 @@ void launch_flush_u(const LoopArgs& a, cudaStream_t s);
 // ry-th row of its tile
 struct PersistPlan {
   int gx, gy, tw, th, ry, variant, cs;
-  int rows;  // FP32 form: a thread owns this many consecutive rows
+  int rows;  // the forms with tensor memory: a thread owns this many consecutive rows at most
 };
 // the plan of a mesh on the current device; false if it does not fit on chip
 bool persist_prepare(int nx, int ny, int precond, PersistPlan* out);

@@ -1604,6 +1604,14 @@ bool persist_plan(int nx, int ny, const int (&clusters)[5], PersistPlan* out) {
 
 constexpr int WIDE = 100;  // PersistPlan::variant of k_persistent_cg_wide
 
+// Kernels that keep fields in tensor memory ask for more than half of an SM's shared memory, so that no two
+// of them share an SM: each waits in its allocation for all of tensor memory, and two grids that each hold
+// the other's SM would wait for ever.
+size_t tmem_smem(size_t cells, size_t cell_bytes) {
+  const size_t n = cells * cell_bytes;
+  return n > 118 * 1024 ? n : 118 * 1024;
+}
+
 namespace {
 // The tiling with the fewest cycles an iteration (16 a row of a warp, 3200 for each of the two
 // sums' exchange when there is more than one tile); tiles at least 32 columns wide, where
@@ -1646,7 +1654,7 @@ bool rows_plan(int nx, int ny, int ctas, int threads, int max_rows, F&& smem, Pe
 
 const PersistKernel kWideKernels[2] = {k_persistent_cg_wide<false>, k_persistent_cg_wide<true>};
 size_t wide_plan_smem(const PersistPlan& p) {
-  return ((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw) * sizeof(double);
+  return tmem_smem((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw, sizeof(double));
 }
 const void* cg_kernel(const PersistPlan& p, int precond) {
   const int diag = precond == 2 ? 1 : 0;
@@ -1685,7 +1693,7 @@ const MixPersistKernel kMixKernels[2][2] = {{k_persistent_mix<false, 2>, k_persi
 // Groups of 8 spill: 13.0 us at 200 x 300, 22.5 at 2048^2.
 const void* mix_kernel(const PersistPlan& p, bool diag) { return (const void*)kMixKernels[p.rows > 6][diag]; }
 size_t mix_plan_smem(const PersistPlan& p) {
-  return ((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw + 1) * sizeof(float);
+  return tmem_smem((size_t)(p.th + 2) * (p.tw + 2) + (size_t)p.th * p.tw + 1, sizeof(float));
 }
 
 }  // namespace
@@ -2554,10 +2562,10 @@ const PolyPersistKernel kPolyWideKernels[2][2] = {  // PPCG / Chebyshev, without
     {k_persistent_poly_wide<ON_PPCG, false>, k_persistent_poly_wide<ON_PPCG, true>},
     {k_persistent_poly_wide<ON_CHEBY, false>, k_persistent_poly_wide<ON_CHEBY, true>}};
 size_t poly_wide_plan_smem(const PersistPlan& p) {
-  return ((size_t)2 * (p.th + 2) * (p.tw + 2) + 1) * sizeof(double);
+  return tmem_smem((size_t)2 * (p.th + 2) * (p.tw + 2) + 1, sizeof(double));
 }
 size_t mix_poly_plan_smem(const PersistPlan& p) {
-  return ((size_t)2 * (p.th + 2) * (p.tw + 2) + 1) * sizeof(float);
+  return tmem_smem((size_t)2 * (p.th + 2) * (p.tw + 2) + 1, sizeof(float));
 }
 
 }  // namespace

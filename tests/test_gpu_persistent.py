@@ -174,3 +174,36 @@ def test_on_chip_fp32_polynomial_wait_is_bounded(solver, monkeypatch):
         c.reset_eigen()
         got = c.tea_leaf(o, d.initial_timestep)
         assert (got.n_exit, got.error) == (want.n_exit, want.error)
+
+
+def test_on_chip_solves_of_two_threads():
+    """Two threads, each with chunks of its own, solve at the same time in every on-chip form: the bits
+    are those of the same solves one after the other."""
+    import threading
+
+    from tealeaf_ref_gb300 import native
+
+    work = [(solver, precision, size) for size in ((200, 160), (420, 390))
+            for solver, precision in (("cg", "fp64"), ("cg", "mixed"), ("ppcg", "fp64"), ("ppcg", "mixed"),
+                                      ("chebyshev", "mixed"))]
+
+    def solve_all(order, out):
+        for k in order:
+            solver, precision, (nx, ny) = work[k]
+            d = small_deck(nx=nx, ny=ny, solver=solver, ch_cg_presteps=10, ch_cg_epslim=1e30, ppcg_inner_steps=6,
+                           max_iters=120, steps=1)
+            with native.Chunk.from_deck(d) as c:
+                c.tea_leaf(native.opts_from_deck(d, precision), d.initial_timestep)
+                out[k] = c.download("u")
+
+    want, got = {}, [{}, {}]
+    solve_all(range(len(work)), want)
+    orders = [range(len(work)), range(len(work) - 1, -1, -1)]
+    threads = [threading.Thread(target=solve_all, args=(o, g)) for o, g in zip(orders, got)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for g in got:
+        for k in range(len(work)):
+            assert k in g and np.array_equal(g[k], want[k]), work[k]
