@@ -1613,11 +1613,16 @@ size_t tmem_smem(size_t cells, size_t cell_bytes) {
 }
 
 namespace {
-// The tiling with the fewest cycles an iteration (16 a row of a warp, 3200 for each of the two
-// sums' exchange when there is more than one tile); tiles at least 32 columns wide, where
-// the mesh is, for the sake of the coefficients' loads.
+// The tiling with the fewest cycles an iteration (16 a row of a warp, 3200 for each of the two sums'
+// exchange when there is more than one tile); tiles at least 32 columns wide, where the mesh is, for the
+// sake of the coefficients' loads.
+// FP32, from 7 rows a thread on: the warps of the busiest of the SM's four schedulers count, so 12 or 16
+// warps rather than 13.  By their sum the FP32 CG step at 1400^2 with jac_diag took 18.8 us, so it takes 16.9;
+// Chebyshev solves there 35.3 and 31.9 ms, at 1999 x 1500 59.6 and 57.2.  Below, at 512^2, 10.0 and 10.1 us.
+// FP64: their sum, as a CTA's FP64 work sets the time: k_persistent_cg_wide at 1000^2 22.8 us, by the busiest
+// scheduler 24.3; k_persistent_poly_wide at 1200^2 with jac_diag 23.0 and 25.6 ms.
 template <typename F>
-bool rows_plan(int nx, int ny, int ctas, int threads, int max_rows, F&& smem, PersistPlan* out) {
+bool rows_plan(int nx, int ny, int ctas, int threads, int max_rows, bool fp32, F&& smem, PersistPlan* out) {
   double best = 0.0;
   bool found = false;
   if (ctas > PERSIST_MAX_CTAS) ctas = PERSIST_MAX_CTAS;
@@ -1639,8 +1644,9 @@ bool rows_plan(int nx, int ny, int ctas, int threads, int max_rows, F&& smem, Pe
       p.variant = 0;
       const int halo = 2 * (p.tw + p.th);
       if (p.rows > max_rows || halo > PH * threads || smem(p) > PERSIST_SMEM_MAX) continue;
-      const double cost =
-          (double)((p.ry * tw + 31) / 32) * p.rows * 16.0 + 0.5 * halo + (p.gx * p.gy > 1 ? 6400.0 : 0.0);
+      int warps = (p.ry * tw + 31) / 32;
+      if (fp32 && p.rows > 6) warps = (warps + 3) / 4 * 4;
+      const double cost = (double)warps * p.rows * 16.0 + 0.5 * halo + (p.gx * p.gy > 1 ? 6400.0 : 0.0);
       if (!found || cost < best) {
         best = cost;
         *out = p;
@@ -1668,7 +1674,7 @@ bool persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const void* k0 = (const void*)kVariants[0].k[precond == 2 ? 1 : 0];
   for (int i = 0; i < 5; ++i) clusters[i] = persist_clusters(k0, 1 << i, PERSIST_SMEM_MAX);
   if (!persist_plan(nx, ny, clusters, out)) {
-    if (!rows_plan(nx, ny, clusters[0], PT, WROWS, wide_plan_smem, out)) return false;
+    if (!rows_plan(nx, ny, clusters[0], PT, WROWS, false, wide_plan_smem, out)) return false;
     out->variant = WIDE;
   }
   return persist_clusters(cg_kernel(*out, precond), out->cs, cg_smem(*out)) * out->cs >= persist_ctas(*out);
@@ -1701,7 +1707,7 @@ size_t mix_plan_smem(const PersistPlan& p) {
 bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const bool diag = precond == 2;
   const int ctas = persist_clusters((const void*)kMixKernels[1][diag], 1, PERSIST_SMEM_MAX);
-  if (!rows_plan(nx, ny, ctas, PT, MROWS, mix_plan_smem, out)) return false;
+  if (!rows_plan(nx, ny, ctas, PT, MROWS, true, mix_plan_smem, out)) return false;
   return persist_clusters(mix_kernel(*out, diag), 1, mix_plan_smem(*out)) >= persist_ctas(*out);
 }
 
@@ -1992,9 +1998,9 @@ int poly_ctas(const void* k, int threads, size_t smem) {
 //
 // A Chebyshev cycle's step took about 7 us at 1999 x 1500 against 15 in the blocked sweeps (four steps a
 // pass over the fields), bound by the coefficients' way from L2.  Whole solves, CG presteps included,
-// against the blocked sweeps: Chebyshev 200 x 300 4.0 ms against 10.4, 512^2 7.2 / 20.6, 1000^2 19.6 /
-// 42.6, 1999 x 1500 59.3 / 94.8, 2040^2 84 / 118; PPCG with 10 inner steps 512^2 11.1 / 21.3, 1000^2 28.3 /
-// 43.6, 1999 x 1500 78.7 / 94.7 (5 inner steps 103 / 120), 2040^2 with 20 inner steps 91 / 105.  Every mesh
+// against the blocked sweeps: Chebyshev 200 x 300 4.0 ms against 10.4, 512^2 7.2 / 20.6, 1000^2 19.4 /
+// 42.6, 1999 x 1500 57.2 / 94.8, 2040^2 84 / 118; PPCG with 10 inner steps 512^2 11.1 / 21.3, 1000^2 28.0 /
+// 43.6, 1999 x 1500 77.4 / 94.7 (5 inner steps 103 / 120), 2040^2 with 20 inner steps 91 / 105.  Every mesh
 // that fits runs here.
 namespace {
 
@@ -2578,7 +2584,7 @@ bool poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
     fits = poly_ctas((const void*)kPolyVariants[out->variant].k[mode][diag], QT, poly_plan_smem(*out)) >= persist_ctas(*out);
   if (fits) return true;
   const int wide = poly_ctas((const void*)kPolyWideKernels[0][diag], QT, PERSIST_SMEM_MAX);
-  if (!rows_plan(nx, ny, wide, QT, WROWS, poly_wide_plan_smem, out)) return false;
+  if (!rows_plan(nx, ny, wide, QT, WROWS, false, poly_wide_plan_smem, out)) return false;
   out->variant = WIDE;
   for (int mode = 0; mode < 2; ++mode)
     if (poly_ctas((const void*)kPolyWideKernels[mode][diag], QT, poly_wide_plan_smem(*out)) < persist_ctas(*out))
@@ -2603,7 +2609,7 @@ cudaError_t launch_persistent_poly(const Fields& f, const Layout& L, const Persi
 bool mix_poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const int diag = precond == 2 ? 1 : 0;
   const int ctas = poly_ctas((const void*)kMixPolyKernels[0][diag], QT, PERSIST_SMEM_MAX);
-  if (!rows_plan(nx, ny, ctas, QT, MROWS, mix_poly_plan_smem, out)) return false;
+  if (!rows_plan(nx, ny, ctas, QT, MROWS, true, mix_poly_plan_smem, out)) return false;
   for (int mode = 0; mode < 2; ++mode)
     if (poly_ctas((const void*)kMixPolyKernels[mode][diag], QT, mix_poly_plan_smem(*out)) < persist_ctas(*out))
       return false;
