@@ -2,7 +2,8 @@
 // solvers: the PPCG inner Chebyshev steps (the preconditioner z = p(A) r) and the Chebyshev
 // iteration on a correction inside FP64 iterative refinement.  The FP64 outer parts (PPCG's
 // w = A p, u/r updates, dot products, p update; Chebyshev's residual u0 - A u and u += d) are
-// the FP64 kernels of tl_kernels.cu and tl_mixed.cu.
+// the FP64 kernels of tl_kernels.cu and tl_mixed.cu.  Meshes that fit on chip take
+// k_persistent_mix_poly (tl_persist.cu) instead, with the same bits.
 //
 // Fields (MixFields, FP32, the context layout): cx, cy, di are the FP32 operator (k_mix_prep);
 // PPCG uses r = rtemp, p / p2 = sd (ping-pong), w = utemp; Chebyshev uses r = its right-hand

@@ -1,7 +1,8 @@
-"""The persistent on-chip CG kernel against the batched sweeps (TL_CG_PERSISTENT=0) after a few
-iterations, field by field, at the sizes where its tilings change: one CTA, one cluster (its last
-CTAs without a tile), the whole grid; one to eleven cells a thread, and the form of larger tiles; meshes one cell wide or high; ragged last
-tiles; nearly the largest mesh that fits.
+"""The loops on chip against the sweeps in memory.  The CG kernels (TL_CG_PERSISTENT=0 forces the
+batched sweeps) after a few iterations, field by field, at the sizes where their tilings change: one
+CTA, one cluster (its last CTAs without a tile), the whole grid; one to eleven cells a thread, and
+the form of larger tiles; meshes one cell wide or high; ragged last tiles; nearly the largest mesh
+that fits.
 
 Both forms do the same arithmetic per cell and differ in the rounding of the sums p.w and r.z only:
 alpha and beta agree to a few units of 2^-53, so after N iterations a field differs by at most some
@@ -15,7 +16,8 @@ from helpers import small_deck
 pytestmark = pytest.mark.gpu
 
 SIZES = [(2, 2), (10, 10), (21, 22), (1, 900), (900, 1), (33, 31), (61, 60), (105, 104), (127, 129), (1, 20000),
-         (20000, 3), (256, 256), (301, 499), (512, 512), (700, 641), (777, 1013), (1000, 1000), (1099, 1097), (1391, 1399)]
+         (20000, 3), (256, 256), (301, 499), (512, 512), (700, 641), (777, 1013), (1000, 1000), (1099, 1097),
+         (1391, 1399)]
 
 
 @pytest.mark.parametrize("case", [dict(), dict(precond="jac_diag", reflective=True)], ids=["none", "diag-reflective"])
