@@ -119,10 +119,9 @@ void launch_fused_ppcg_rrn(const LoopArgs& a, bool copy_z, cudaStream_t s);
 // u += alpha p of the last CG iteration when it is still pending (end of a CG phase)
 void launch_flush_u(const LoopArgs& a, cudaStream_t s);
 // persistent cooperative CG on chip (no preconditioner or jac_diag; tl_persist.cu): the mesh in
-// tiles of tw x th cells, one per CTA, clusters of cs CTAs, a thread owning one column and every
-// ry-th row of its tile
+// tiles of tw x th cells, one per CTA, a thread owning one column and every ry-th row of its tile
 struct PersistPlan {
-  int gx, gy, tw, th, ry, variant, cs;
+  int gx, gy, tw, th, ry, variant;
   int rows;  // the forms with tensor memory: a thread owns this many consecutive rows at most
 };
 // the plan of a mesh on the current device; false if it does not fit on chip

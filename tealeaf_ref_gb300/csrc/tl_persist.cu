@@ -20,10 +20,8 @@
 //   partials have come (3300 cycles on 152 CTAs; 4400 when one warp polls five words a lane).  One
 //   table of partials that all CTAs poll takes 7000 cycles, since every store then waits behind the
 //   polls of its line; an arrival counter with a generation word is two dependent atomics and a
-//   second read.  Summing in clusters of 4 first (2600 cycles by itself) loses by its second
-//   conversion: the loop's scalar code runs on one warp, at the rate its instructions are fetched.
-//   A mesh of a few thousand cells takes one cluster of up to 16 CTAs, which exchange through
-//   shared memory (600 cycles), one of a few hundred a single CTA;
+//   second read.  A mesh of up to about a thousand cells takes a single CTA, which has nobody to wait
+//   for (4.4 us an iteration at 22^2, against 5.9 on the grid at 32^2);
 // - the rim goes the same way: its owner stores each value with the sum's number into the
 //   neighbour tile's box, and the neighbour's threads poll for it while the first warp waits for
 //   the sum.  Publishing it through the field needs a fence (1900 cycles) before the sum;
@@ -32,9 +30,9 @@
 //
 // Time per CG iteration, the solve's set-up included, against the form before it (up to 640K cells
 // one persistent kernel with the fields in memory and two barriers an iteration, above the batched
-// sweeps of tl_fused.cu in CUDA graphs): 64^2 3.8 against 12 us, 128^2 5.9 / 13.8, 256^2 7.2 / 14.5,
-// 512^2 10.2 / 27.6, 700^2 14.2 / 34.8, 777 x 1013 with jac_diag 22.3 / 43.9; larger meshes, to about
-// 1400^2, take k_persistent_cg_wide.  The FP64 pipe's share is 1.1 us at 256^2 and 8 us at 700^2.
+// sweeps of tl_fused.cu in CUDA graphs): 64^2 5.6 against 12 us, 128^2 5.5 / 13.8, 256^2 6.5 / 14.5,
+// 512^2 9.3 / 27.6, 700^2 13.3 / 34.8; meshes from about 800K cells, to about 1400^2, take
+// k_persistent_cg_wide.  The FP64 pipe's share is 1.1 us at 256^2 and 8 us at 700^2.
 #include "tl_mixed.cuh"
 
 namespace tl {
@@ -48,12 +46,9 @@ constexpr int PH = 2;          // halo cells per thread at most
 constexpr int POLLW = 5;       // warps that poll the inbox at most
 constexpr int SLOTS = 32 * POLLW;            // words of an inbox
 constexpr int PERSIST_MAX_CTAS = SLOTS - 1;  // one is left for the test of the bounded wait
-constexpr int MAX_CLUSTER = 16;                  // CTAs of a cluster
 constexpr size_t PERSIST_SMEM_MAX = 225 * 1024;
-// polls before a wait gives up (about a second: a poll takes an L2 round trip; one of shared
-// memory some 50 cycles)
+// polls before a wait gives up (about a second: a poll takes an L2 round trip)
 constexpr unsigned PERSIST_POLL_LIMIT = 1u << 21;
-constexpr unsigned PERSIST_POLL_LIMIT_SM = 1u << 25;
 
 struct PersistArgs {
   LoopArgs a;
@@ -125,26 +120,6 @@ __device__ __forceinline__ bool box_is(const ulonglong2& w, unsigned epoch) {
 __device__ __forceinline__ double box_value(const ulonglong2& w) {
   return emu::from_bits((w.x & 0xffffffff00000000ull) | (w.y >> 32));
 }
-// the same in the shared memory of a CTA of the cluster
-__device__ __forceinline__ void cbox_put(const ulonglong2* s, unsigned rank, double v, unsigned epoch) {
-  const unsigned long long b = emu::bits(v);
-  unsigned a;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(s)), "r"(rank));
-  asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(a),
-               "l"((b & 0xffffffff00000000ull) | epoch), "l"((b << 32) | epoch)
-               : "memory");
-}
-__device__ __forceinline__ ulonglong2 cbox_get(const ulonglong2* s) {
-  ulonglong2 w;
-  asm volatile("ld.relaxed.cluster.shared::cta.v2.u64 {%0, %1}, [%2];"
-               : "=l"(w.x), "=l"(w.y)
-               : "r"((unsigned)__cvta_generic_to_shared(s))
-               : "memory");
-  return w;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.aligned;\n barrier.cluster.wait.aligned;" ::: "memory");
-}
 __device__ __forceinline__ bool finite_bits(double v) { return expo(v) != 0x7ffu; }
 template <int ID, int N>
 __device__ __forceinline__ void bar_sync() {
@@ -170,21 +145,20 @@ __device__ __forceinline__ int fresh(int x) {
 struct Exchange {
   Fix part[PW];        // the owning warps' sums
   Fix inbox[POLLW];    // the polling warps' sums
-  ulonglong2 cbox[2][MAX_CLUSTER + 1];  // one cluster: its CTAs' partials, by parity of the sum's number
   int fail;            // a wait ran out
 };
 
 // First warp: the owning warps' sums added up over the grid; meanwhile() runs while the partials
 // are on their way.  in: the inboxes of this parity.  Not inlined, so that both sums of an
 // iteration run the same instructions.
-__device__ __noinline__ double exchange_sum(Exchange* x, ulonglong2* in, unsigned epoch, int ctas, int cs, int extra,
-                                            double rro, double* inv_rro) {
+__device__ __noinline__ double exchange_sum(Exchange* x, ulonglong2* in, unsigned epoch, int ctas, int extra, double rro,
+                                            double* inv_rro) {
   const int lane = threadIdx.x & 31;
   bar_sync<1, PTHREADS>();
   Fix p{0, 1u};
   if (lane < PW) p = x->part[lane];
   double total = fix_value(warp_fix(p));
-  if (ctas > cs) {
+  if (ctas > 1) {
 #pragma unroll
     for (int q = 0; q < POLLW; ++q)
       if (lane + 32 * q < ctas) box_put(in + (size_t)(lane + 32 * q) * SLOTS + blockIdx.x, total, epoch);
@@ -194,24 +168,8 @@ __device__ __noinline__ double exchange_sum(Exchange* x, ulonglong2* in, unsigne
     p = Fix{0, 1u};
     if (lane < nq) p = x->inbox[lane];
     total = fix_value(warp_fix(p));
-  } else {
-    const int mine = cs + extra;
-    if (mine > 1) {
-      const ulonglong2* box = x->cbox[epoch & 1u];
-      if (lane < cs) cbox_put(box + blockIdx.x, lane, total, epoch);
-      if (inv_rro) *inv_rro = 1.0 / rro;
-      ulonglong2 w = make_ulonglong2(0ull, 0ull);
-      bool here = lane >= mine;
-      for (unsigned tries = 0; !here && tries < PERSIST_POLL_LIMIT_SM; ++tries) {
-        w = cbox_get(box + lane);
-        here = box_is(w, epoch);
-      }
-      if (!here) x->fail = 1;
-      __syncwarp();
-      total = fix_value(warp_fix(lane < mine ? box_value(w) : 0.0));
-    } else if (inv_rro) {
-      *inv_rro = 1.0 / rro;
-    }
+  } else if (inv_rro) {
+    *inv_rro = 1.0 / rro;
   }
   return total;
 }
@@ -311,18 +269,14 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
   const bool owner = wid != 0;
   const int to = t - 32;  // number of the owner
-  const int cs = g.pl.cs, ctas = gridDim.x;
-  if (t < 2 * (MAX_CLUSTER + 1)) X.cbox[t / (MAX_CLUSTER + 1)][t % (MAX_CLUSTER + 1)] = make_ulonglong2(0ull, 0ull);
+  const int ctas = gridDim.x;
   if (t == 0) {
     S = *g.a.rd.st;
     sh_status = S.status;
     sh_beta = S.beta;
     X.fail = 0;
   }
-  if (cs > 1)
-    cluster_sync();  // every CTA's box is empty before a peer writes into it
-  else
-    __syncthreads();
+  __syncthreads();
   if (sh_status != RUN) {  // in every CTA
     if (blockIdx.x == 0 && t == 0) *g.st_host = S;
     return;
@@ -330,8 +284,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
 
   const int bx = blockIdx.x % g.pl.gx, by = blockIdx.x / g.pl.gx;
   const int j0 = bx * g.pl.tw, k0 = by * g.pl.th;  // first cell of the tile, from 0
-  const bool tile = owner && by < g.pl.gy;  // one cluster: the last CTAs may have no tile
-  const int tw = tile ? min(g.pl.tw, L.nx - j0) : 0, th = tile ? min(g.pl.th, L.ny - k0) : 0;
+  const int tw = min(g.pl.tw, L.nx - j0), th = min(g.pl.th, L.ny - k0);
   const int P = g.pl.tw + 2, ry = g.pl.ry;
   const int asz = (g.pl.th + 2) * P;
   double* const sp = psm;
@@ -341,7 +294,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
 
   // the thread's column and first row; cells i = 0 .. mine-1 at rows ty + i ry
   const int tx = owner ? to % g.pl.tw : 0, ty = owner ? to / g.pl.tw : 0;
-  const int mine = (tx < tw && ty < ry && ty < th) ? (th - 1 - ty) / ry + 1 : 0;
+  const int mine = (owner && tx < tw && ty < ry && ty < th) ? (th - 1 - ty) / ry + 1 : 0;
   const int o0 = (ty + 1) * P + tx + 1;
   const int c0 = (int)L.at(j0 + tx + 1, k0 + ty + 1);
   const int ostep = ry * P, cstep = ry * L.ld;
@@ -370,7 +323,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
     if (h >= g.pl.th) x = tw, y = h - g.pl.th, is = j0 + tw < L.nx && y < th;
     if (h >= 2 * g.pl.th) x = h - 2 * g.pl.th, y = -1, is = k0 > 0 && x < tw;
     if (h >= 2 * g.pl.th + g.pl.tw) x = h - 2 * g.pl.th - g.pl.tw, y = th, is = k0 + th < L.ny && x < tw;
-    if (is && tile && h < hbox) {
+    if (is && owner && h < hbox) {
       ho[q] = (y + 1) * P + x + 1;
       hh[q] = (int)blockIdx.x * hbox + h;
       const int c = (int)L.at(j0 + x + 1, k0 + y + 1);
@@ -421,7 +374,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
     if (lane == 0) X.part[wid - 1] = s;
     bar_arrive<1, PTHREADS>();
   };
-  const int nwait = ctas > cs ? ctas + g.extra : 0, nq = (nwait + 31) / 32;
+  const int nwait = ctas > 1 ? ctas + g.extra : 0, nq = (nwait + 31) / 32;
   auto poll = [&] {
     if (wid > nq) return;
     const int slot = (wid - 1) * 32 + lane;
@@ -494,7 +447,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       give(acc);
       poll();
     } else {
-      C.pw = exchange_sum(&X, inboxes(), epoch, ctas, cs, g.extra, C.rro, &C.inv_rro);
+      C.pw = exchange_sum(&X, inboxes(), epoch, ctas, g.extra, C.rro, &C.inv_rro);
       C.after_pw(&S, n, &sh_alpha, &sh_status, g.a.rd.hist_a);
     }
     ++epoch;
@@ -574,7 +527,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       }
       if (!got) X.fail = 1;
     } else {
-      C.rrn = exchange_sum(&X, inboxes(), epoch, ctas, cs, g.extra, C.rro, nullptr);
+      C.rrn = exchange_sum(&X, inboxes(), epoch, ctas, g.extra, C.rro, nullptr);
       C.after_rrn(&S, n, &sh_beta, &sh_status, g.a.rd.hist_b);
     }
     ++epoch;
@@ -587,7 +540,6 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       break;
     }
   }
-  if (cs > 1) cluster_sync();  // no CTA leaves while a peer may still write into its shared memory
   if (X.fail) {
     if (t == 0) g.a.rd.st->status = g.st_host->status = EXIT_TIMEOUT;
     return;
@@ -977,7 +929,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
       give(dot);
       poll();
     } else {
-      pw = exchange_sum(&X, inboxes(), epoch, ctas, 1, g.extra, rro, nullptr);
+      pw = exchange_sum(&X, inboxes(), epoch, ctas, g.extra, rro, nullptr);
       alpha_ = rro / pw;
       if (lane == 0) {
         sh_alpha = (float)alpha_;
@@ -1057,7 +1009,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
       }
       if (!got) X.fail = 1;
     } else {
-      rr_ = exchange_sum(&X, inboxes(), epoch, ctas, 1, g.extra, rro, nullptr);
+      rr_ = exchange_sum(&X, inboxes(), epoch, ctas, g.extra, rro, nullptr);
       beta_ = rr_ / rro;
       if (lane == 0) {
         sh_beta = (float)beta_;
@@ -1375,7 +1327,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg_wide(PersistArgs 
       give(dot);
       poll();
     } else {
-      C.pw = exchange_sum(&X, inboxes(), epoch, ctas, 1, g.extra, C.rro, &C.inv_rro);
+      C.pw = exchange_sum(&X, inboxes(), epoch, ctas, g.extra, C.rro, &C.inv_rro);
       C.after_pw(&S, n, &sh_alpha, &sh_status, g.a.rd.hist_a);
     }
     ++epoch;
@@ -1444,7 +1396,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg_wide(PersistArgs 
       }
       if (!got) X.fail = 1;
     } else {
-      C.rrn = exchange_sum(&X, inboxes(), epoch, ctas, 1, g.extra, C.rro, nullptr);
+      C.rrn = exchange_sum(&X, inboxes(), epoch, ctas, g.extra, C.rro, nullptr);
       C.after_rrn(&S, n, &sh_beta, &sh_status, g.a.rd.hist_b);
     }
     ++epoch;
@@ -1512,43 +1464,23 @@ const PersistVariant kVariants[] = {PERSIST_VARIANT(1), PERSIST_VARIANT(2), PERS
 // p, cx, cy and Di
 size_t plan_smem(const PersistPlan& p) { return (size_t)4 * (p.th + 2) * (p.tw + 2) * sizeof(double); }
 
-// A launch of a plan: cooperative (its CTAs wait for one another), in clusters.
-struct PersistLaunch {
-  cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at[2];
-  PersistLaunch(int ctas, int cs, size_t smem, cudaStream_t s) {
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(PTHREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cs;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeCooperative;
-    at[1].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
-  }
-};
-
-// Clusters of cs CTAs of kernel k that are co-resident (0: none).  Sets the attributes a launch
-// needs, the same for every plan: contexts share them.
-int persist_clusters(const void* k, int cs, size_t smem) {
-  int n = 0;
-  PersistLaunch l(cs, cs, smem, nullptr);
-  l.cfg.numAttrs = 1;
+// CTAs of `threads` threads of kernel k that are co-resident (0: none).  Sets the attribute a launch needs,
+// the same for every plan: contexts share it.
+int coresident_ctas(const void* k, int threads, size_t smem) {
+  int dev = 0, sms = 0, per_sm = 0;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM_MAX) != cudaSuccess ||
-      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, k, &l.cfg) != cudaSuccess) {
+      cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  return n;
+  return sms * per_sm;
 }
 
 }  // namespace
 
-int persist_ctas(const PersistPlan& p) { return (p.gx * p.gy + p.cs - 1) / p.cs * p.cs; }
+int persist_ctas(const PersistPlan& p) { return p.gx * p.gy; }
 
 // the inboxes of two sums and the halo boxes of two steps
 size_t persist_box_bytes(const PersistPlan& p) {
@@ -1557,24 +1489,16 @@ size_t persist_box_bytes(const PersistPlan& p) {
 
 // The tiling of an nx x ny mesh with the least cycles an iteration: FP64 instructions of a warp on
 // the busiest SM (10 an iteration and cell, 17 cycles of the SM's four pipes each), the halo, and
-// the two grid sums' exchange (700 more cycles each in one cluster, 3200 across the grid).
-// clusters[i]: co-resident clusters of 2^i CTAs.
-bool persist_plan(int nx, int ny, const int (&clusters)[5], PersistPlan* out) {
+// the two grid sums' exchange (3200 more cycles each across the grid).  all: co-resident CTAs.
+bool persist_plan(int nx, int ny, int all, PersistPlan* out) {
   double best = 0.0;
   bool found = false;
-  // one CTA, one cluster of 2 .. 16, all SMs
-  const int kinds[6][2] = {{1, 1}, {2, 1}, {4, 1}, {8, 1}, {16, 1}, {1, PERSIST_MAX_CTAS}};
-  for (const auto& kind : kinds) {
-    const int cs = kind[0];
-    int have = 0;
-    for (int i = 0; i < 5; ++i)
-      if (cs == 1 << i) have = clusters[i];
-    const int ctas = cs * (have < kind[1] ? have : kind[1]);
+  for (const int most : {1, PERSIST_MAX_CTAS}) {  // one CTA, all SMs
+    const int ctas = all < most ? all : most;
     for (int g0 = 1; g0 <= ctas && g0 <= nx; ++g0) {
       const int tw = (nx + g0 - 1) / g0;
       if (tw > PT) continue;
-      PersistPlan p;
-      p.cs = cs;
+      PersistPlan p{};
       p.tw = tw;
       p.gx = (nx + tw - 1) / tw;
       int gy = ctas / p.gx;
@@ -1590,7 +1514,7 @@ bool persist_plan(int nx, int ny, const int (&clusters)[5], PersistPlan* out) {
       const int halo = 2 * (p.tw + p.th);
       if (p.variant < 0 || halo > PH * PT || plan_smem(p) > PERSIST_SMEM_MAX) continue;
       const double slabs = (double)((p.ry * tw + 31) / 32) * m;
-      const double sums = kind[1] > 1 ? 3200.0 : (cs > 1 ? 700.0 : 0.0);
+      const double sums = most > 1 ? 3200.0 : 0.0;
       const double cost = slabs * 170.0 + 0.5 * halo + 8.0 * p.th + 2.0 * sums;
       if (!found || cost < best) {
         best = cost;
@@ -1629,8 +1553,7 @@ bool rows_plan(int nx, int ny, int ctas, int threads, int max_rows, bool fp32, F
   for (int g0 = 1; g0 <= ctas && g0 <= nx; ++g0) {
     const int tw = (nx + g0 - 1) / g0;
     if (tw > threads || (tw < 32 && g0 > 1)) continue;
-    PersistPlan p;
-    p.cs = 1;
+    PersistPlan p{};
     p.tw = tw;
     p.gx = (nx + tw - 1) / tw;
     for (int many = 0; many < 2; ++many) {
@@ -1670,23 +1593,20 @@ size_t cg_smem(const PersistPlan& p) { return p.variant == WIDE ? wide_plan_smem
 
 // Plans the mesh for the current device; false if it does not fit on chip.
 bool persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
-  int clusters[5];
-  const void* k0 = (const void*)kVariants[0].k[precond == 2 ? 1 : 0];
-  for (int i = 0; i < 5; ++i) clusters[i] = persist_clusters(k0, 1 << i, PERSIST_SMEM_MAX);
-  if (!persist_plan(nx, ny, clusters, out)) {
-    if (!rows_plan(nx, ny, clusters[0], PT, WROWS, false, wide_plan_smem, out)) return false;
+  const int ctas = coresident_ctas((const void*)kVariants[0].k[precond == 2 ? 1 : 0], PTHREADS, PERSIST_SMEM_MAX);
+  if (!persist_plan(nx, ny, ctas, out)) {
+    if (!rows_plan(nx, ny, ctas, PT, WROWS, false, wide_plan_smem, out)) return false;
     out->variant = WIDE;
   }
-  return persist_clusters(cg_kernel(*out, precond), out->cs, cg_smem(*out)) * out->cs >= persist_ctas(*out);
+  return coresident_ctas(cg_kernel(*out, precond), PTHREADS, cg_smem(*out)) >= persist_ctas(*out);
 }
 
 cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch, void* box,
                                  LoopState* st_host, cudaStream_t s, int extra) {
   PersistArgs g{a, p, max_run, epoch, static_cast<ulonglong2*>(box), st_host, extra};
   void* args[] = {&g};
-  PersistLaunch l(persist_ctas(p), p.cs, cg_smem(p), s);
   ++launch_counter();
-  return cudaLaunchKernelExC(&l.cfg, cg_kernel(p, a.precond), args);
+  return cudaLaunchCooperativeKernel(cg_kernel(p, a.precond), dim3(persist_ctas(p)), dim3(PTHREADS), args, cg_smem(p), s);
 }
 
 namespace {
@@ -1706,18 +1626,18 @@ size_t mix_plan_smem(const PersistPlan& p) {
 
 bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const bool diag = precond == 2;
-  const int ctas = persist_clusters((const void*)kMixKernels[1][diag], 1, PERSIST_SMEM_MAX);
+  const int ctas = coresident_ctas((const void*)kMixKernels[1][diag], PTHREADS, PERSIST_SMEM_MAX);
   if (!rows_plan(nx, ny, ctas, PT, MROWS, true, mix_plan_smem, out)) return false;
-  return persist_clusters(mix_kernel(*out, diag), 1, mix_plan_smem(*out)) >= persist_ctas(*out);
+  return coresident_ctas(mix_kernel(*out, diag), PTHREADS, mix_plan_smem(*out)) >= persist_ctas(*out);
 }
 
 cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState* ms, const PersistPlan& p, int max_run,
                                   unsigned epoch, void* box, cudaStream_t s, int extra) {
   MixPersistArgs g{m, L, ms, p, max_run, epoch, static_cast<ulonglong2*>(box), extra};
   void* args[] = {&g};
-  PersistLaunch l(persist_ctas(p), p.cs, mix_plan_smem(p), s);
   ++launch_counter();
-  return cudaLaunchKernelExC(&l.cfg, mix_kernel(p, m.mi != nullptr), args);
+  return cudaLaunchCooperativeKernel(mix_kernel(p, m.mi != nullptr), dim3(persist_ctas(p)), dim3(PTHREADS), args,
+                                     mix_plan_smem(p), s);
 }
 
 
@@ -1944,7 +1864,6 @@ bool poly_plan(int nx, int ny, int ctas, PersistPlan* out) {
     const int tw = (nx + g0 - 1) / g0;
     if (tw > QT) continue;
     PersistPlan p{};
-    p.cs = 1;
     p.tw = tw;
     p.gx = (nx + tw - 1) / tw;
     for (int many = 0; many < 2; ++many) {
@@ -1970,19 +1889,6 @@ bool poly_plan(int nx, int ny, int ctas, PersistPlan* out) {
     }
   }
   return found;
-}
-
-// threads of one CTA differ between the kernels
-int poly_ctas(const void* k, int threads, size_t smem) {
-  int dev = 0, sms = 0, per_sm = 0;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PERSIST_SMEM_MAX) != cudaSuccess ||
-      cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return sms * per_sm;
 }
 
 }  // namespace
@@ -2578,16 +2484,16 @@ size_t mix_poly_plan_smem(const PersistPlan& p) {
 
 bool poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const int diag = precond == 2 ? 1 : 0;
-  const int ctas = poly_ctas((const void*)kPolyVariants[0].k[0][diag], QT, PERSIST_SMEM_MAX);
+  const int ctas = coresident_ctas((const void*)kPolyVariants[0].k[0][diag], QT, PERSIST_SMEM_MAX);
   bool fits = poly_plan(nx, ny, ctas, out);
   for (int mode = 0; mode < 2 && fits; ++mode)
-    fits = poly_ctas((const void*)kPolyVariants[out->variant].k[mode][diag], QT, poly_plan_smem(*out)) >= persist_ctas(*out);
+    fits = coresident_ctas((const void*)kPolyVariants[out->variant].k[mode][diag], QT, poly_plan_smem(*out)) >= persist_ctas(*out);
   if (fits) return true;
-  const int wide = poly_ctas((const void*)kPolyWideKernels[0][diag], QT, PERSIST_SMEM_MAX);
+  const int wide = coresident_ctas((const void*)kPolyWideKernels[0][diag], QT, PERSIST_SMEM_MAX);
   if (!rows_plan(nx, ny, wide, QT, WROWS, false, poly_wide_plan_smem, out)) return false;
   out->variant = WIDE;
   for (int mode = 0; mode < 2; ++mode)
-    if (poly_ctas((const void*)kPolyWideKernels[mode][diag], QT, poly_wide_plan_smem(*out)) < persist_ctas(*out))
+    if (coresident_ctas((const void*)kPolyWideKernels[mode][diag], QT, poly_wide_plan_smem(*out)) < persist_ctas(*out))
       return false;
   return true;
 }
@@ -2608,10 +2514,10 @@ cudaError_t launch_persistent_poly(const Fields& f, const Layout& L, const Persi
 
 bool mix_poly_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
   const int diag = precond == 2 ? 1 : 0;
-  const int ctas = poly_ctas((const void*)kMixPolyKernels[0][diag], QT, PERSIST_SMEM_MAX);
+  const int ctas = coresident_ctas((const void*)kMixPolyKernels[0][diag], QT, PERSIST_SMEM_MAX);
   if (!rows_plan(nx, ny, ctas, QT, MROWS, true, mix_poly_plan_smem, out)) return false;
   for (int mode = 0; mode < 2; ++mode)
-    if (poly_ctas((const void*)kMixPolyKernels[mode][diag], QT, mix_poly_plan_smem(*out)) < persist_ctas(*out))
+    if (coresident_ctas((const void*)kMixPolyKernels[mode][diag], QT, mix_poly_plan_smem(*out)) < persist_ctas(*out))
       return false;
   return true;
 }
