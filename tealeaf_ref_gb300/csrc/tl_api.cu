@@ -403,7 +403,9 @@ bool use_persistent_poly(tl_ctx* c) {
   return !c->g.reflective && !(e && e[0] == '0') && use_persistent(c, c->ppoly, poly_persist_prepare);
 }
 
-// steps first .. first + steps - 1 (from 1) of the coefficients on the device
+// steps first .. first + steps - 1 (from 1) of the coefficients on the device, two at least: a tile reads
+// its neighbours' cells from the field it overwrites at the end, and only the first step's rims make it
+// wait for them
 int run_persistent_poly(tl_ctx* c, bool ppcg, const double* u_in, int first, int steps) {
   unsigned epoch;
   int rc = next_epoch(c, c->ppoly, &epoch, steps);
@@ -1633,7 +1635,7 @@ struct Solver {
     if (!fused) launch_ppcg_init_sd(c->f, c->L, c->g, c->theta, c->stream);
     const int h = c->halo_depth;
     int rc;
-    if (inner_steps > 0 && use_ppcg_inner_sweep() && use_persistent_poly(c)) {
+    if (inner_steps > 1 && use_ppcg_inner_sweep() && use_persistent_poly(c)) {
       poly_used = true;
       if ((rc = run_persistent_poly(c, true, nullptr, 1, inner_steps))) return rc;
       if (!fused) launch_copy_interior(c->f.z, c->f.utemp, c->L, c->stream);
@@ -2073,31 +2075,30 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
           const double gamm = (std::sqrt(c->cn) - 1.0) / (std::sqrt(c->cn) + 1.0);
           est_itc = (int)std::lround(std::log(it_alpha) / std::log(gamm));
           cheby_calc_steps = 1;
-        } else if (use_cheby_sweep() && use_persistent_poly(c)) {
-          // on chip, the iterations up to the next whose residual is checked, or at which the loop
-          // ends: in between the error is the last one's repeated square root (tea_solve.f90:273,402)
-          int run = 0;
-          while (true) {
-            const int at = n + run;
-            ++run;
-            if ((at >= est_itc && at % 10 == 0) || at >= max_iters || run >= PERSIST_RUN) break;
-            const double next = std::sqrt(std::fabs(error));
-            if (next < o->eps * initial_residual) break;
-            error = next;
-          }
-          S.poly_used = true;
-          if ((rc = run_persistent_poly(c, false, u_alt ? c->f.u1 : c->f.u, cheby_calc_steps, run))) return rc;
-          u_alt = wr_stale = false;
-          cheby_calc_steps += run - 1;
-          n += run - 1;
-          if (n >= est_itc && n % 10 == 0) {
-            if ((rc = S.norm(c->f.r, &error))) return rc;
-          }
         } else {
-          if ((rc = prof_begin(c))) return rc;
-          cheby_iterate(S.ch_a[cheby_calc_steps], S.ch_b[cheby_calc_steps],
-                        (n >= est_itc && n % 10 == 0) || n >= max_iters);
-          if ((rc = prof_end(c, TL_KERNEL_CHEBY_ITERATE, 1))) return rc;
+          // on chip, the iterations up to the next whose residual is checked, or at which the loop
+          // ends: in between the error is the last one's repeated square root (tea_solve.f90:273,402).
+          // A single one runs as a sweep (run_persistent_poly)
+          int run = 1;
+          if (use_cheby_sweep() && use_persistent_poly(c)) {
+            for (int at = n; !((at >= est_itc && at % 10 == 0) || at >= max_iters || run >= PERSIST_RUN); ++at, ++run) {
+              const double next = std::sqrt(std::fabs(error));
+              if (next < o->eps * initial_residual) break;
+              error = next;
+            }
+          }
+          if (run > 1) {
+            S.poly_used = true;
+            if ((rc = run_persistent_poly(c, false, u_alt ? c->f.u1 : c->f.u, cheby_calc_steps, run))) return rc;
+            u_alt = wr_stale = false;
+            cheby_calc_steps += run - 1;
+            n += run - 1;
+          } else {
+            if ((rc = prof_begin(c))) return rc;
+            cheby_iterate(S.ch_a[cheby_calc_steps], S.ch_b[cheby_calc_steps],
+                          (n >= est_itc && n % 10 == 0) || n >= max_iters);
+            if ((rc = prof_end(c, TL_KERNEL_CHEBY_ITERATE, 1))) return rc;
+          }
           if (n >= est_itc && n % 10 == 0) {
             if ((rc = S.norm(c->f.r, &error))) return rc;
           }

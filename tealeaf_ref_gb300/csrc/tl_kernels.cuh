@@ -132,7 +132,7 @@ size_t persist_box_bytes(const PersistPlan& p);  // its grid sums' inboxes and t
 // a.rd.st and in st_host (mapped host memory)
 cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch,
                                  void* box, LoopState* st_host, cudaStream_t s, int extra = 0);
-// the FP64 polynomial steps on chip (no reflective boundaries; no preconditioner or jac_diag): `steps`
+// the FP64 polynomial steps on chip (no reflective boundaries; no preconditioner or jac_diag): `steps`, two at least,
 // PPCG inner steps on sd, rtemp, utemp, or Chebyshev iterations from u_in and p into u and p (w and r,
 // and z with jac_diag, of the last one), with the coefficients ch_a[0..steps), ch_b[0..steps) in device
 // memory.  The boxes are persist_box_bytes, zeroed once; epoch .. epoch + steps - 1 as above.
