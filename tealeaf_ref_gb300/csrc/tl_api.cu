@@ -58,6 +58,7 @@ struct tl_ctx {
   unsigned* counter = nullptr;
   LoopState* st = nullptr;
   LoopState* st_host = nullptr;  // pinned mirror
+  unsigned* wait_err = nullptr;  // pinned: set by a CTA of an on-chip CG loop whose wait ran out
   double* hist_a = nullptr;
   double* hist_b = nullptr;
   int hist_cap = 0;
@@ -385,15 +386,27 @@ int next_epoch(tl_ctx* c, tl_ctx::Persist& p, unsigned* epoch, unsigned sums = 2
   return TL_OK;
 }
 
+// Tests of the bounded waits: TL_CG_BARRIER_EXTRA=1, the grid sums of the on-chip CG loops wait for one
+// partial that never comes, so every wait runs out; 3, one of their tiles gives its
+// rims up at once; 2, one tile of the polynomial steps sends no rims, so its neighbours' waits run out
+int wait_fault() {
+  const char* ex = getenv("TL_CG_BARRIER_EXTRA");
+  return ex && ex[0] >= '1' && ex[0] <= '3' ? ex[0] - '0' : 0;
+}
+
+// after a launch of an on-chip CG loop has ended
+int check_wait_err(tl_ctx* c) {
+  if (!*c->wait_err) return TL_OK;
+  *c->wait_err = 0;
+  return fail(TL_ERR_TIMEOUT, "tl_tea_leaf: a wait of the on-chip CG loop ran out");
+}
+
 int run_persistent(tl_ctx* c, const LoopArgs& la) {
   unsigned epoch;
   int rc = next_epoch(c, c->pcg, &epoch);
   if (rc) return rc;
-  // TL_CG_BARRIER_EXTRA=1: the grid sums wait for one partial that never comes, so every wait runs
-  // out (about a second) and the solve reports TL_ERR_TIMEOUT -- the test of the bounded wait
-  const char* ex = getenv("TL_CG_BARRIER_EXTRA");
-  CK(launch_persistent_cg(la, c->pcg.plan, PERSIST_RUN, epoch, c->pcg.box, c->st_host, c->stream,
-                          ex && ex[0] == '1' ? 1 : 0));
+  CK(launch_persistent_cg(la, c->pcg.plan, PERSIST_RUN, epoch, c->pcg.box, c->st_host, c->wait_err, wait_fault(),
+                          c->stream));
   return TL_OK;
 }
 
@@ -410,10 +423,9 @@ int run_persistent_poly(tl_ctx* c, bool ppcg, const double* u_in, int first, int
   unsigned epoch;
   int rc = next_epoch(c, c->ppoly, &epoch, steps);
   if (rc) return rc;
-  const char* ex = getenv("TL_CG_BARRIER_EXTRA");  // 2: one tile sends no rims, so its neighbours' waits run out
   CK(launch_persistent_poly(c->f, c->L, c->ppoly.plan, ppcg, c->g.precond == TL_PREC_JAC_DIAG, u_in, c->ch_a + first,
                             c->ch_b + first, steps, epoch, c->ppoly.box, c->counter + MIX_ERR_WORD,
-                            ex && ex[0] == '2', c->stream));
+                            wait_fault() == 2, c->stream));
   return TL_OK;
 }
 
@@ -432,9 +444,8 @@ int run_persistent_mix_poly(tl_ctx* c, bool ppcg, int steps) {
   unsigned epoch;
   int rc = next_epoch(c, c->pmpoly, &epoch, steps);
   if (rc) return rc;
-  const char* ex = getenv("TL_CG_BARRIER_EXTRA");  // 2: as for run_persistent_poly
   CK(launch_persistent_mix_poly(c->mix, c->L, c->pmpoly.plan, ppcg, c->f.r, c->f.z, c->theta, c->ch_a + 1, c->ch_b + 1,
-                                steps, epoch, c->pmpoly.box, c->counter + MIX_ERR_WORD, ex && ex[0] == '2', c->stream));
+                                steps, epoch, c->pmpoly.box, c->counter + MIX_ERR_WORD, wait_fault() == 2, c->stream));
   return TL_OK;
 }
 
@@ -442,7 +453,8 @@ int run_persistent_mix(tl_ctx* c) {
   unsigned epoch;
   int rc = next_epoch(c, c->pmix, &epoch);
   if (rc) return rc;
-  CK(launch_persistent_mix(c->mix, c->L, c->mst, c->pmix.plan, PERSIST_RUN, epoch, c->pmix.box, c->stream));
+  CK(launch_persistent_mix(c->mix, c->L, c->mst, c->pmix.plan, PERSIST_RUN, epoch, c->pmix.box, c->wait_err,
+                           wait_fault(), c->stream));
   return TL_OK;
 }
 
@@ -654,6 +666,7 @@ int tl_create(int x_cells, int y_cells, int halo_depth, int coefficient, int pre
   if (e == cudaSuccess) e = cudaMalloc(&c->st, sizeof(LoopState));
   if (e == cudaSuccess) e = cudaMemsetAsync(c->st, 0, sizeof(LoopState), c->stream);
   if (e == cudaSuccess) e = cudaMallocHost(&c->st_host, sizeof(LoopState));
+  if (e == cudaSuccess) e = cudaMallocHost(&c->wait_err, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc(&c->halo_list, sizeof(double*) * 16);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
@@ -672,6 +685,7 @@ int tl_create(int x_cells, int y_cells, int halo_depth, int coefficient, int pre
     return rc;
   }
   memset(c->st_host, 0, sizeof(LoopState));
+  *c->wait_err = 0;
   Fields& f = c->f;
   f.density = c->slot(S_DENSITY);
   f.energy1 = c->slot(S_ENERGY1);
@@ -710,6 +724,7 @@ int tl_destroy(tl_ctx* c) {
   cudaFree(c->counter);
   cudaFree(c->st);
   if (c->st_host) cudaFreeHost(c->st_host);
+  if (c->wait_err) cudaFreeHost(c->wait_err);
   cudaFree(c->hist_a);
   cudaFree(c->hist_b);
   cudaFree(c->ch_a);
@@ -1420,6 +1435,7 @@ int mixed_cg(tl_ctx* c, const tl_solve_opts* o, tl_solve_info* info, long long l
       }
       if ((rc = check_launch("mixed batch"))) return rc;
       if ((rc = sync_mix(c))) return rc;
+      if ((rc = check_wait_err(c))) return rc;
       if (c->prof) {
         const int ran = std::min(std::max(H.n - n_before, 0), batch);
         for (int i = 0; i < ran; ++i) {
@@ -1434,8 +1450,6 @@ int mixed_cg(tl_ctx* c, const tl_solve_opts* o, tl_solve_info* info, long long l
       }
     }
     if (H.status == EXIT_BREAKDOWN) return fail(TL_ERR_BREAKDOWN, "tl_tea_leaf: non-finite FP32 CG scalar");
-    if (H.status == EXIT_TIMEOUT)
-      return fail(TL_ERR_TIMEOUT, "tl_tea_leaf: a wait of the persistent FP32 CG kernel expired");
     const bool switching = pre && H.status == STOP_SWITCH;
     const bool capped = H.n > H.max_n;
     // trial replacement: true FP64 residual of u + d, u itself untouched
@@ -1898,6 +1912,7 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
         CK(cudaStreamSynchronize(c->stream));  // the kernel wrote the state into the mirror too
       else if ((rc = sync_state(c)))
         return rc;
+      if ((rc = check_wait_err(c))) return rc;
       initial_residual = H.initial_residual;
       if (c->prof) {
         // iterations of this batch that did work (the rest returned on the status word); the
@@ -1918,8 +1933,6 @@ int solve(tl_ctx* c, const tl_solve_opts* o, double dt, tl_solve_info* info, con
       }
       cg_calc_steps = H.cg_calc_steps;
       if (H.status == EXIT_BREAKDOWN) return fail(TL_ERR_BREAKDOWN, "tl_tea_leaf: non-finite CG scalar");
-      if (H.status == EXIT_TIMEOUT)
-        return fail(TL_ERR_TIMEOUT, "tl_tea_leaf: a grid-barrier wait of the persistent CG kernel expired");
       if (H.status != RUN) {
         // the CG phase stops here: apply the deferred u += alpha p of its last iteration -- in
         // the finalise sweep when nothing reads u before it (a CG solve without check_result)

@@ -129,9 +129,11 @@ bool persist_prepare(int nx, int ny, int precond, PersistPlan* out);
 size_t persist_box_bytes(const PersistPlan& p);  // its grid sums' inboxes and the tiles' halo boxes
 // up to max_run iterations in one launch; epoch .. epoch + 2 max_run - 1 number its grid sums, and
 // no earlier launch on these boxes (zeroed once) has used them or higher ones.  The state is left in
-// a.rd.st and in st_host (mapped host memory)
+// a.rd.st and in st_host (mapped host memory); *err (mapped host memory too, zero before) is set if a
+// wait ran out in any CTA, and then nothing else counts.  fault: 0, or for the tests 1 (the sums wait
+// for one partial that never comes) or 3 (the second tile gives its rims up at once)
 cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch,
-                                 void* box, LoopState* st_host, cudaStream_t s, int extra = 0);
+                                 void* box, LoopState* st_host, unsigned* err, int fault, cudaStream_t s);
 // the FP64 polynomial steps on chip (no reflective boundaries; no preconditioner or jac_diag): `steps`, two at least,
 // PPCG inner steps on sd, rtemp, utemp, or Chebyshev iterations from u_in and p into u and p (w and r,
 // and z with jac_diag, of the last one), with the coefficients ch_a[0..steps), ch_b[0..steps) in device
@@ -198,10 +200,10 @@ void launch_mix_iteration(const MixFields& m, const Layout& L, const Reduce& rd,
 void launch_mix_apply(const Fields& f, const MixFields& m, const Layout& L, cudaStream_t s);
 
 // The FP32 steps on chip (tl_persist.cu), for meshes that fit: up to max_run steps of the loop in
-// one launch, as launch_mix_iteration would run them
+// one launch, as launch_mix_iteration would run them; err and fault as for launch_persistent_cg
 bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out);
 cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState* ms, const PersistPlan& p, int max_run,
-                                  unsigned epoch, void* box, cudaStream_t s, int extra = 0);
+                                  unsigned epoch, void* box, unsigned* err, int fault, cudaStream_t s);
 
 // ---- FP32 polynomial sweeps of the precision form of Chebyshev / PPCG (tl_mixed_poly.cu) ----
 // PPCG inner loop in FP32 from the FP64 r: inner_steps Chebyshev steps with ch_a/ch_b[1..],

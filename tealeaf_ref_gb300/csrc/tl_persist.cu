@@ -47,7 +47,7 @@ constexpr int POLLW = 5;       // warps that poll the inbox at most
 constexpr int SLOTS = 32 * POLLW;            // words of an inbox
 constexpr int PERSIST_MAX_CTAS = SLOTS - 1;  // one is left for the test of the bounded wait
 constexpr size_t PERSIST_SMEM_MAX = 225 * 1024;
-// polls before a wait gives up (about a second: a poll takes an L2 round trip)
+// polls before a wait gives up (some tenths of a second: a poll takes an L2 round trip)
 constexpr unsigned PERSIST_POLL_LIMIT = 1u << 21;
 
 struct PersistArgs {
@@ -57,7 +57,9 @@ struct PersistArgs {
   unsigned epoch;   // number of the launch's first grid sum
   ulonglong2* box;  // by parity of the sum's number, an inbox per CTA; then the tiles' halo boxes
   LoopState* st_host;
-  int extra;        // partials waited for beyond the grid's (the test of the bounded wait)
+  unsigned* err;    // set when a wait ran out in any CTA: the results are void
+  int extra;        // partials waited for beyond the grid's (test of the bounded wait)
+  int lame;         // this CTA gives its rims up at once (test of the report; -1: none)
 };
 
 // Sums across lanes: a value as an integer multiple of 2^(e - 1075 - FSH), e the largest biased
@@ -515,7 +517,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
         c += MG * cstep;
       }
       bool got = false;
-      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+      const unsigned limit = g.lame == (int)blockIdx.x ? 0u : PERSIST_POLL_LIMIT;
+      for (unsigned tries = 0; !got && tries < limit; ++tries) {
         got = true;
 #pragma unroll
         for (int q = 0; q < PH; ++q)
@@ -540,8 +543,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
       break;
     }
   }
-  if (X.fail) {
-    if (t == 0) g.a.rd.st->status = g.st_host->status = EXIT_TIMEOUT;
+  if (X.fail) {  // in a word of its own: CTA 0 may have ended its loop and store its state after this
+    if (t == 0) *g.err = 1u;
     return;
   }
   // ---- the fields and the state as the loop's kernels leave them (w = A p_n formed again) ----
@@ -596,7 +599,9 @@ struct MixPersistArgs {
   int max_run;
   unsigned epoch;
   ulonglong2* box;
-  int extra;
+  unsigned* err;  // set when a wait ran out in any CTA: the results are void
+  int extra;      // as in PersistArgs
+  int lame;
 };
 
 // a float beside the sum's number
@@ -997,7 +1002,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
       load_coefs(0, ka);  // of the next phase A
       poll();
       bool got = false;
-      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+      const unsigned limit = g.lame == (int)blockIdx.x ? 0u : PERSIST_POLL_LIMIT;
+      for (unsigned tries = 0; !got && tries < limit; ++tries) {
         got = true;
 #pragma unroll
         for (int q = 0; q < PH; ++q)
@@ -1057,7 +1063,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
   __syncthreads();  // every warp is done with tensor memory
   if (wid == 0) tmem_free(sh_tmem);
   if (failed) {
-    if (t == 0) g.ms->status = EXIT_TIMEOUT;
+    if (t == 0) *g.err = 1u;
     return;
   }
   if (blockIdx.x == 0 && t == 0) {
@@ -1384,7 +1390,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg_wide(PersistArgs 
         tmem_put_done();
       }
       bool got = false;
-      for (unsigned tries = 0; !got && tries < PERSIST_POLL_LIMIT; ++tries) {
+      const unsigned limit = g.lame == (int)blockIdx.x ? 0u : PERSIST_POLL_LIMIT;
+      for (unsigned tries = 0; !got && tries < limit; ++tries) {
         got = true;
 #pragma unroll
         for (int q = 0; q < PH; ++q)
@@ -1442,7 +1449,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg_wide(PersistArgs 
   __syncthreads();  // every warp is done with tensor memory
   if (wid == 0) tmem_free(sh_tmem);
   if (failed) {
-    if (t == 0) g.a.rd.st->status = g.st_host->status = EXIT_TIMEOUT;
+    if (t == 0) *g.err = 1u;
     return;
   }
   if (blockIdx.x == 0 && t == 0) {
@@ -1602,8 +1609,8 @@ bool persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
 }
 
 cudaError_t launch_persistent_cg(const LoopArgs& a, const PersistPlan& p, int max_run, unsigned epoch, void* box,
-                                 LoopState* st_host, cudaStream_t s, int extra) {
-  PersistArgs g{a, p, max_run, epoch, static_cast<ulonglong2*>(box), st_host, extra};
+                                 LoopState* st_host, unsigned* err, int fault, cudaStream_t s) {
+  PersistArgs g{a, p, max_run, epoch, static_cast<ulonglong2*>(box), st_host, err, fault == 1 ? 1 : 0, fault == 3 ? 1 : -1};
   void* args[] = {&g};
   ++launch_counter();
   return cudaLaunchCooperativeKernel(cg_kernel(p, a.precond), dim3(persist_ctas(p)), dim3(PTHREADS), args, cg_smem(p), s);
@@ -1632,8 +1639,8 @@ bool mix_persist_prepare(int nx, int ny, int precond, PersistPlan* out) {
 }
 
 cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState* ms, const PersistPlan& p, int max_run,
-                                  unsigned epoch, void* box, cudaStream_t s, int extra) {
-  MixPersistArgs g{m, L, ms, p, max_run, epoch, static_cast<ulonglong2*>(box), extra};
+                                  unsigned epoch, void* box, unsigned* err, int fault, cudaStream_t s) {
+  MixPersistArgs g{m, L, ms, p, max_run, epoch, static_cast<ulonglong2*>(box), err, fault == 1 ? 1 : 0, fault == 3 ? 1 : -1};
   void* args[] = {&g};
   ++launch_counter();
   return cudaLaunchCooperativeKernel(mix_kernel(p, m.mi != nullptr), dim3(persist_ctas(p)), dim3(PTHREADS), args,
