@@ -24,6 +24,7 @@
 // against the FPU's multiply.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -65,6 +66,19 @@ TL_EMU_FN double from_bits(uint64_t u) {
   std::memcpy(&x, &u, 8);
   return x;
 #endif
+}
+
+TL_EMU_FN unsigned expo(double v) { return (unsigned)(bits(v) >> 52) & 0x7ffu; }
+
+// a / b from y, the reciprocal of b rounded to nearest: with an exact remainder one correction gives the
+// correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34(1), 1990).  The remainder is a multiple of
+// the product of two units in the last place, so it is exact while a, b and the quotient are far from the
+// subnormal range; elsewhere (a below 2^-1000, say, where it would be off in the last place) the division.
+TL_EMU_FN double quotient(double a, double b, double y) {
+  double q = a * y;
+  q = fma(fma(-q, b, a), y, q);
+  const auto plain = [](double v) { return expo(v) - 300u <= 1400u; };
+  return plain(a) && plain(b) && plain(q) ? q : a / b;
 }
 
 TL_EMU_FN int clz64(uint64_t v) {

@@ -71,7 +71,7 @@ struct Fix {
   long long q;
   unsigned e;  // 0x7ff: an infinity or NaN among the values
 };
-__device__ __forceinline__ unsigned expo(double v) { return (unsigned)(emu::bits(v) >> 52) & 0x7ffu; }
+using emu::expo;
 // the sum over the warp of q (|q| < 2^58), as limbs of 21 bits through redux.sync
 __device__ __forceinline__ long long warp_add(long long q) {
   const int l0 = __reduce_add_sync(0xffffffffu, (int)(q & 0x1fffff));
@@ -211,13 +211,7 @@ struct CgScalars {
   }
   // rrn is known: beta, the error, the loop's tests
   __device__ __forceinline__ void after_rrn(LoopState* S, int n, double* sh_beta, int* sh_status, double* hist) {
-    // rrn / rro from the reciprocal of rro: one correction gives the correctly rounded quotient
-    // in the normal range (P. Markstein, IBM J. Res. Dev. 34(1), 1990); else the division
-    double b = rrn * inv_rro;
-    b = fma(fma(-b, rro, rrn), inv_rro, b);
-    const unsigned eb = expo(b), eo = expo(rro);
-    if (eb < 300u || eb > 1700u || eo < 300u || eo > 1700u) b = rrn / rro;
-    beta = b;
+    const double b = beta = emu::quotient(rrn, rro, inv_rro);
     // without the square root when the outcome is plain: the error is far enough above the goal
     // (goal2: its square with a margin; non-negative doubles order as their bits) and nothing
     // else can stop the loop.  The error itself is then left to the launch's end.
