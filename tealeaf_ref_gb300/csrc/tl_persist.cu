@@ -69,7 +69,7 @@ struct PersistArgs {
 constexpr int FSH = 1;  // 53 + FSH bits for the largest value: 512 of them fit 63 bits
 struct Fix {
   long long q;
-  unsigned e;  // 0x7ff: an infinity or NaN among the values
+  unsigned e;  // 0x7ff: an infinity or NaN among the values; q is then the infinity's sign, 0 for NaN
 };
 using emu::expo;
 // the sum over the warp of q (|q| < 2^58), as limbs of 21 bits through redux.sync
@@ -79,10 +79,19 @@ __device__ __forceinline__ long long warp_add(long long q) {
   const int l2 = __reduce_add_sync(0xffffffffu, (int)(q >> 42));
   return (long long)l0 + ((long long)l1 << 21) + ((long long)l2 << 42);
 }
+// the sum when a lane holds an infinity or NaN, as IEEE addition gives it
+__device__ __noinline__ Fix warp_nonfinite(int sign, bool nan) {
+  const bool p = __any_sync(0xffffffffu, sign > 0), m = __any_sync(0xffffffffu, sign < 0);
+  return Fix{__any_sync(0xffffffffu, nan) || p == m ? 0ll : (p ? 1ll : -1ll), 0x7ffu};
+}
 __device__ __forceinline__ Fix warp_fix(double v) {
   const uint64_t b = emu::bits(v);
   const unsigned ev = max((unsigned)(b >> 52) & 0x7ffu, 1u);
   const unsigned e = __reduce_max_sync(0xffffffffu, ev);
+  if (e == 0x7ffu) {
+    const bool nan = (b & ~emu::SIGN) > emu::INF, inf = (b & ~emu::SIGN) == emu::INF;
+    return warp_nonfinite(inf ? ((b & emu::SIGN) ? -1 : 1) : 0, nan);
+  }
   const uint64_t m = (b & emu::FRAC) | ((b << 1 >> 53) ? emu::HIDDEN : 0ull);
   const long long i = (long long)((((m << (FSH + 1)) >> min(e - ev, 63u)) + 1ull) >> 1);
   return Fix{warp_add((b & emu::SIGN) ? -i : i), e};
@@ -90,12 +99,16 @@ __device__ __forceinline__ Fix warp_fix(double v) {
 // the sum over the warp of sums, one a lane, of at most 16 lanes or of single values
 __device__ __forceinline__ Fix warp_fix(const Fix& f) {
   const unsigned e = __reduce_max_sync(0xffffffffu, f.e);
+  if (e == 0x7ffu) {
+    const bool odd = f.e == 0x7ffu;
+    return warp_nonfinite(odd ? (f.q > 0) - (f.q < 0) : 0, odd && f.q == 0);
+  }
   const unsigned d = min(e - f.e, 63u);
   return Fix{warp_add((f.q + (d ? 1ll << (d - 1) : 0ll)) >> d), e};
 }
 __device__ __noinline__ double scale_slowly(double t, int k) { return ldexp(t, k); }
 __device__ __forceinline__ double fix_value(const Fix& f) {
-  if (f.e == 0x7ffu) return emu::from_bits(emu::QNAN);
+  if (f.e == 0x7ffu) return emu::from_bits(f.q ? (f.q < 0 ? emu::SIGN : 0ull) | emu::INF : emu::QNAN);
   const double t = (double)f.q;
   const int k = (int)f.e - 1075 - FSH, et = (int)expo(t);
   if (et == 0) return t;  // zero
@@ -622,8 +635,9 @@ __device__ __forceinline__ Fix warp_fix(const Dot2& d) {
     return (b >> 31) ? -i : i;
   };
   const unsigned es = ex(bs), ec = ex(bc);
-  const unsigned e = __reduce_max_sync(0xffffffffu, max(es, ec)) ;
-  return Fix{warp_add((fix(bs, es, e) >> 1) + (fix(bc, ec, e) >> 1)), e == 0x7ffu ? e : e + 1u};
+  const unsigned e = __reduce_max_sync(0xffffffffu, max(es, ec));
+  if (e == 0x7ffu) return Fix{0, e};  // beside an infinite sum the error terms are NaN
+  return Fix{warp_add((fix(bs, es, e) >> 1) + (fix(bc, ec, e) >> 1)), e + 1u};
 }
 
 // Tensor memory as the threads' own storage: 512 columns of 128 lanes, of which a warp reaches the
