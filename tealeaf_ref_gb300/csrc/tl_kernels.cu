@@ -739,8 +739,7 @@ void launch_init_faces(const Fields& f, const Layout& L, const Geometry& g, cuda
   // marches as long as they leave 8 CTAs an SM (a row each on small meshes), 32 rows at most
   const int strips = (L.nx + 1 + TB - 1) / TB;
   const long long want = (long long)strips * (L.ny + 1) / (8 * sm_count());
-  int rows = want < 1 ? 1 : want > 32 ? 32 : (int)want;
-  if (rows == 1 && L.ny + 1 > 65535) rows = 2;
+  const int rows = want < 1 ? 1 : want > 32 ? 32 : (int)want;
   { ++launch_counter(); k_init_faces<<<dim3(strips, (L.ny + rows) / rows), TB, 0, s>>>(f, L, g, rows); }
 }
 void launch_init_cells(const Fields& f, const Layout& L, const Geometry& g, bool with_residual, cudaStream_t s) {
