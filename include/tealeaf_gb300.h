@@ -335,7 +335,9 @@ int tl_adjoint_end(tl_ctx* ctx);
 /* Enable (1) or disable (0) CUDA-event timing of every launch of the solver-loop kernels
  * (TL_KERNEL_*) on the context's stream; enabling also clears the accumulated totals.  The
  * host-driven loops (Chebyshev, PPCG, Jacobi) wait for each timed launch, which adds launch
- * gaps to the solve time while timing is on. */
+ * gaps to the solve time while timing is on.  The timers are of the kernels that work in memory:
+ * while timing is on these run on every mesh, also where the solve otherwise takes its on-chip
+ * loop (FP64 to about 1400^2 cells, the FP32 steps of the precision form to about 2050^2). */
 int tl_profile(tl_ctx* ctx, int enable);
 /* Accumulated device time (ms) and launch count of one TL_KERNEL_* since tl_profile(ctx,1). */
 int tl_profile_read(tl_ctx* ctx, int kernel_id, double* total_ms, long long* launches);

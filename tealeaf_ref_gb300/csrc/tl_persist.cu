@@ -64,15 +64,17 @@ struct PersistArgs {
 
 // Sums across lanes: a value as an integer multiple of 2^(e - 1075 - FSH), e the largest biased
 // exponent among the values, rounded to nearest; the integers are added exactly, so the result does
-// not depend on an order.  A value's rounding error is at most 2^-55 of the largest, where an FP64
-// tree makes one of 2^-53 at each level.
-constexpr int FSH = 1;  // 53 + FSH bits for the largest value: 512 of them fit 63 bits
+// not depend on an order.  A value's rounding error is at most 2^-54 of the warp's largest, and those of
+// its 32 values add up; an FP64 tree rounds by 2^-53 of the partial sum at each of its levels.  Against
+// sums in 64 bits a 256^2 run's error is 2.3e-15 (2.2e-15 with the tree), 777 x 1013's 1.4e-14 (1.3e-14).
+constexpr int FSH = 1;  // 53 + FSH bits for the largest value: a CTA's 480 fit 63 bits
 struct Fix {
   long long q;
   unsigned e;  // 0x7ff: an infinity or NaN among the values; q is then the infinity's sign, 0 for NaN
 };
 using emu::expo;
-// the sum over the warp of q (|q| < 2^58), as limbs of 21 bits through redux.sync
+// the sum over the warp of q, as limbs of 21 bits through redux.sync: of single values (|q| <= 2^54), or of
+// at most 16 lanes' sums of a warp (|q| <= 2^59, together below 2^63)
 __device__ __forceinline__ long long warp_add(long long q) {
   const int l0 = __reduce_add_sync(0xffffffffu, (int)(q & 0x1fffff));
   const int l1 = __reduce_add_sync(0xffffffffu, (int)((q >> 21) & 0x1fffff));
@@ -591,8 +593,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_cg(PersistArgs g) {
 // compiler cannot tell the arrays of shared memory apart, and a load behind a store waits for it), and the
 // coefficients of the next group are in flight while one is used.  d is updated before the wait for beta's
 // partials, in the time they take; the rim's columns are sent by whole warps.  Time per iteration, the
-// replacements included, against the sweeps' two launches: 512^2 10.0 against 25.0 us, 1000^2 12.3 / 34.0,
-// 1500 x 1999 17.7 / 48.0, 2048^2 21.3 / 50.4, with jac_diag 25.4 / 55.5.  Row by row, with a test of
+// replacements included, against the sweeps' two launches: 512^2 9.7 against 25.0 us, 1000^2 11.5 / 34.0,
+// 1500 x 1999 17.1 / 48.0, 2048^2 20.4 / 50.4, with jac_diag 24.2 / 55.5.  Row by row, with a test of
 // the row, a test of the mesh's walls and a store to the neighbour's box in each, 2048^2 took 32.4 us and
 // 1000^2 13.2: the walls are mirrored by the neighbours' offsets, and what has no row works on a cell of
 // zeros.  The sums' exchange, 6 us, bounds it up to about 1000^2, the coefficients' way from L2 (13 bytes
@@ -1094,11 +1096,12 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persistent_mix(MixPersistArgs g
 // k_persistent_cg's loop laid out as k_persistent_mix: p with its halo and r in shared memory, w and u in
 // tensor memory, the coefficients (and Mi) streamed from the fields through L2, a group of rows ahead.
 // 16 bytes a cell in shared memory take meshes of up to 2.1 million cells.  It runs where k_persistent_cg's
-// tiles do not fit (11 cells a thread, about 800K cells): at 700^2 it takes 14.5 us an iteration against
-// 14.2, at 777 x 1013 and 1000^2 it is even with larger tiles there (22.3 and 22.9 us), which spilled from
-// 14 cells a thread on (26.2 us at 1024^2 against 24.1).  Against the batched sweeps: 1000^2 22.9 us an
-// iteration against 42.1, 1024^2 24.1 / 42.4, 1100^2 with jac_diag 31.2 / 50.4, 1200^2 28.9 / 48.1, 1300 x
-// 1400 37.1 / 61.7.  The FP64 pipe's share is 17 us at 1000^2, 31 at 1300 x 1400.
+// tiles do not fit (11 cells a thread, about 800K cells; 777 x 1013 runs here): at 700^2 it takes 14.5 us
+// an iteration against 14.2; larger tiles there spilled from 14 cells a thread on (26.2 us at 1024^2 against
+// 24.1).  Its two groups of four rows' coefficients fill the registers (68 to 72 bytes spilled).  Against
+// the batched sweeps: 1000^2 22.3 us an iteration against 42.1, 1024^2 24.1 / 42.4, 1100^2 with jac_diag
+// 31.2 / 50.4, 1200^2 28.4 / 48.1, 1300 x 1400 36.7 / 61.7.  The FP64 pipe's share is 17 us at 1000^2, 31 at
+// 1300 x 1400.
 constexpr int WROWS = 32;  // rows a thread may own
 constexpr int WC = 4;      // rows handled together
 __device__ __forceinline__ void tmem_put(unsigned a, const double (&v)[4]) {
@@ -1473,6 +1476,8 @@ struct PersistVariant {
   PersistKernel k[2];  // without / with jac_diag
 };
 #define PERSIST_VARIANT(M) {M, {k_persistent_cg<M, false>, k_persistent_cg<M, true>}}
+// A tile's rows are rounded up to the next of these: up to 4 p stays in registers, up to 6 u and Mi; at 11
+// the registers are full (56 bytes spilled), and more cells go to k_persistent_cg_wide.
 const PersistVariant kVariants[] = {PERSIST_VARIANT(1), PERSIST_VARIANT(2), PERSIST_VARIANT(4),
                                     PERSIST_VARIANT(6), PERSIST_VARIANT(8), PERSIST_VARIANT(11)};
 
@@ -1666,7 +1671,7 @@ cudaError_t launch_persistent_mix(const MixFields& m, const Layout& L, MixState*
 // the residual run on the integer pipes, as in the staged sweeps of tl_fused.cu.  Same bits.
 //
 // A PPCG solve of 124 inner steps an outer iteration took, per inner step, 2.2 us at 60^2 against 13.6
-// with a launch a step, 2.7 / 14.9 at 256^2, 6.0 / 15.0 at 512^2, 11.8 / 19.3 at 777 x 813 and 17.3 /
+// with a launch a step, 2.7 / 14.9 at 256^2, 5.8 / 15.0 at 512^2, 11.5 / 19.3 at 777 x 813 and 16.9 /
 // 21.7 at 1000^2, where the FP64 pipe's share is 11; 332 Chebyshev iterations with their presteps 3.8
 // against 14.4 us each at 128^2 and 21.9 against 24.7 at 1000^2.
 namespace {
@@ -1866,6 +1871,8 @@ struct PolyPersistVariant {
   {M,                                                                                        \
    {{k_persistent_poly<M, ON_PPCG, false>, k_persistent_poly<M, ON_PPCG, true>},             \
     {k_persistent_poly<M, ON_CHEBY, false>, k_persistent_poly<M, ON_CHEBY, true>}}}
+// 14 cells of 512 threads are what the four arrays of shared memory hold (36 to 48 bytes spilled); the steps
+// between keep the rows a tile is rounded up by below half of its own.
 const PolyPersistVariant kPolyVariants[] = {POLY_VARIANT(1), POLY_VARIANT(2), POLY_VARIANT(4),
                                             POLY_VARIANT(7), POLY_VARIANT(10), POLY_VARIANT(14)};
 size_t poly_plan_smem(const PersistPlan& p) { return (size_t)4 * (p.th + 2) * (p.tw + 2) * sizeof(double); }
@@ -1919,8 +1926,8 @@ bool poly_plan(int nx, int ny, int ctas, PersistPlan* out) {
 //
 // A Chebyshev cycle's step took about 7 us at 1999 x 1500 against 15 in the blocked sweeps (four steps a
 // pass over the fields), bound by the coefficients' way from L2.  Whole solves, CG presteps included,
-// against the blocked sweeps: Chebyshev 200 x 300 4.0 ms against 10.4, 512^2 7.2 / 20.6, 1000^2 19.4 /
-// 42.6, 1999 x 1500 57.2 / 94.8, 2040^2 84 / 118; PPCG with 10 inner steps 512^2 11.1 / 21.3, 1000^2 28.0 /
+// against the blocked sweeps: Chebyshev 200 x 300 3.8 ms against 10.4, 512^2 7.2 / 20.6, 1000^2 19.0 /
+// 42.6, 1999 x 1500 56.6 / 94.8, 2040^2 82 / 118; PPCG with 10 inner steps 512^2 11.1 / 21.3, 1000^2 28.0 /
 // 43.6, 1999 x 1500 77.4 / 94.7 (5 inner steps 103 / 120), 2040^2 with 20 inner steps 91 / 105.  Every mesh
 // that fits runs here.
 namespace {
